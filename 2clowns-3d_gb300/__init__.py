@@ -397,7 +397,7 @@ def tuned_shape(sizes, precision=0):
         return {"mode": "graph", "block": 256 if bal else b.value, "fused_sweeps": bool(f.value & 1),
                 "reduce_block": 64 if f.value & 2 else (256 if bal else b.value), "balanced_rows": bal,
                 "staged_axsub": bool(f.value & 16)}
-    return {"mode": {0: "persistent", 3: "wave"}.get(mo.value, str(mo.value)), "block": b.value,
+    return {"mode": {0: "persistent", 3: "wave", 4: "resident"}.get(mo.value, str(mo.value)), "block": b.value,
             "grid": g.value, "registers": r.value}
 
 

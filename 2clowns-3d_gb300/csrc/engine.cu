@@ -17,6 +17,7 @@
 
 #include "engine.cuh"
 #include "engine_api.h"
+#include "resident.cuh"
 #include "trace.h"
 
 namespace clowns {
@@ -200,9 +201,14 @@ __global__ void __launch_bounds__(kEngBlock) k_mx_update(Eng<T> E) {
     }
 }
 
-// ctrl[2] accumulates the loop bodies of earlier sweeps.
+// ctrl[2] accumulates the loop bodies of earlier sweeps; the resident loop's epochs go on.
 __global__ void k_mx_reset_ctrl(int* ctrl, int inner_max) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) { ctrl[2] += ctrl[0]; ctrl[0] = 0; ctrl[1] = inner_max; }
+    if (threadIdx.x == 0 && blockIdx.x == 0) {
+        ctrl[2] += ctrl[0];
+        ctrl[0] = 0;
+        ctrl[1] = inner_max;
+        ctrl[6] = ctrl[7];
+    }
 }
 
 template <typename T>
@@ -224,7 +230,7 @@ __global__ void k_mixed_init_scalars(MemberScalars* S, int M, double eps, int oi
         z.mode = 1;
         S[m] = z;
     }
-    if (threadIdx.x == 0) { ctrl[0] = 0; ctrl[1] = 0; ctrl[2] = 0; }
+    if (threadIdx.x == 0) { ctrl[0] = 0; ctrl[1] = 0; ctrl[2] = 0; ctrl[6] = 0; ctrl[7] = 0; }
 }
 
 // Export of the scaled/sorted matrix (test hook), member 0 only.
@@ -250,6 +256,13 @@ static inline int member_groups(int n) {
     return (nc + kGroupChunks - 1) / kGroupChunks;
 }
 
+// Single systems up to this many rows run the resident loop, without tuning.
+// Measured against the tuned graph (ms per solve, graph / resident): FP64 2.7 /
+// 0.9 at 4 k rows, 6.8 / 2.7 at 74 k, 10.7 / 7.2 at 239 k, 13.6 / 13.9 at 413 k;
+// mixed 3.8 / 1.7, 5.9 / 2.7, 9.2 / 5.3, 10.7 / 8.2, and 17.2 / 18.5 at 660 k.
+constexpr int kResMaxRowsFp64 = 300000;
+constexpr int kResMaxRowsMixed = 500000;
+
 struct EngLayout {
     long NV = 0;
     int M = 0, nblk = 0, ngrp = 0, mixed = 0, tsize = 8, wave = 0, nchunk = 0, n1 = 0;
@@ -257,6 +270,8 @@ struct EngLayout {
     size_t o_mem_grp0, o_mem_ngrp, o_gticket, o_gpartials;
     size_t o_in, o_S, o_partials, o_bar, o_al, o_ll, o_d, o_vec[8], o_W, o_x64, o_r64, o_s64, o_t64;
     size_t o_wave, o_wbuf[kWaveBufs];
+    int res = 0;           // the resident loop's words and composed coefficients are laid out
+    size_t o_rword[4], o_rpart, o_ra, o_rc;
     size_t o_baltab = 0;   // ensembles: block tables of the balanced kernels
     size_t o_balg = 0;     // ensembles: blocks of each table's launch
     size_t total = 0;
@@ -317,6 +332,13 @@ static EngLayout eng_layout(int M, const int* n, int mixed, int wave = -1) {
     } else {
         L.o_wave = 0;
         for (int k = 0; k < kWaveBufs; k++) L.o_wbuf[k] = 0;
+    }
+    L.res = wave < 0 && M == 1 && n[0] <= (mixed ? kResMaxRowsMixed : kResMaxRowsFp64);
+    if (L.res) {
+        for (int k = 0; k < 4; k++) L.o_rword[k] = take(2 * (size_t)L.tsize * NV);
+        L.o_rpart = take(sizeof(TagWord<double>) * 6 * (size_t)(NV / kChunk));
+        L.o_ra = take((size_t)L.tsize * kResCoef<6> * NV);
+        L.o_rc = take(sizeof(int) * kResIdx<6> * (size_t)NV);
     }
     if (M > 1) {
         L.o_baltab = take(sizeof(BalBlock) * 16 * (size_t)kBalTabMax);
@@ -399,6 +421,21 @@ static Eng<T> eng_bind(void* work, const EngLayout& L) {
     E.pf = l2_prefetch_rows();
     E.balg = L.o_balg ? (const int*)(b + L.o_balg) : nullptr;
     return E;
+}
+
+template <typename T>
+static ResBufs<T> res_bind(void* work, const EngLayout& L) {
+    ResBufs<T> R = {};
+    if (!L.res) return R;
+    char* b = (char*)work;
+    R.p = (TagWord<T>*)(b + L.o_rword[0]);
+    R.e = (TagWord<T>*)(b + L.o_rword[1]);
+    R.t0 = (TagWord<T>*)(b + L.o_rword[2]);
+    R.t3 = (TagWord<T>*)(b + L.o_rword[3]);
+    R.part = (TagWord<double>*)(b + L.o_rpart);
+    R.a = (T*)(b + L.o_ra);
+    R.c = (int*)(b + L.o_rc);
+    return R;
 }
 
 // Reduction groups: member m's groups are mem_grp0[m] .. mem_grp0[m] +
@@ -507,8 +544,9 @@ static void launch_ldusub64(const Eng<T>& E, const Shape& sh, double inner_tol, 
 }
 
 // ---------------------------------------------------------------------------
-// The iteration loop, executed one of three ways (the autotuner times them on
-// the actual row space and keeps the fastest):
+// The iteration loop.  Single systems of small and medium size run it resident
+// (one kernel, resident.cuh; by rule, see kResMaxRowsFp64); for the others the
+// autotuner times three executions on the actual row space and keeps the fastest:
 //   graph:      a CUDA graph whose WHILE node repeats the iteration's kernels,
 //               chained by programmatic dependent launch (dynamic scheduling,
 //               full occupancy, launch latency overlapped with the previous
@@ -523,7 +561,7 @@ struct LoopShape {
     int block = kStepBlock;
     int grid = 0;
     int minb = 8;     // register budget of the loop kernel: 8 -> 32, 4 -> 64 registers
-    int graph = 0;    // 1: CUDA graph; 2: host-launched kernels; 3: wavefront kernel
+    int graph = 0;    // 1: CUDA graph; 2: host-launched kernels; 3: wavefront kernel; 4: resident kernel
     int wk = 1;       // wavefront: tiles per item
     int wslack = 3;   // wavefront: slack rounds
     int fuse = 1;     // graph / host launches: fused sweep pairs
@@ -532,7 +570,7 @@ struct LoopShape {
     int stg = 0;      // with bal = 4, FP32 single systems: the staged AXSUB (k_bal_axsub_stg)
 };
 
-// CLOWNS_LOOP_MODE=graph|persistent|launch|wave forces one execution of the loop
+// CLOWNS_LOOP_MODE=graph|persistent|launch|wave|resident forces one execution of the loop
 // (with graph and launch, CLOWNS_SWEEP_FUSE=0 selects the four single sweeps and,
 // for single systems, CLOWNS_BALANCED_ROWS=4|8 the balanced one-wave kernels)
 // ("launch": the iteration's kernels launched from the host, eight iterations
@@ -545,6 +583,7 @@ static int forced_loop_mode() {
     if (!strcmp(v, "graph")) return 1;
     if (!strcmp(v, "launch")) return 2;
     if (!strcmp(v, "wave")) return 3;
+    if (!strcmp(v, "resident")) return 4;
     return -1;
 }
 
@@ -556,6 +595,33 @@ static const void* loop_fn(int minb) {
 template <typename T>
 static const void* wave_fn(int minb) {
     return minb == 12 ? (const void*)k_eng_wave<T, 12> : (const void*)k_eng_wave<T, 8>;
+}
+
+static int device_sms() {
+    static const int sms = [] {
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1) {
+            cudaGetLastError();
+            v = kNumSMs;
+        }
+        return v;
+    }();
+    return sms;
+}
+
+// Launch shape of the resident loop for a single system: at most one block per
+// SM, each with the warps its 32-row quarters of chunks fill, or the fewest
+// rounds of at most kResWarps that cover them.
+static LoopShape res_shape(int n) {
+    const int nc = (n + kChunk - 1) / kChunk;
+    LoopShape sh;
+    sh.graph = 4;
+    sh.grid = std::min(nc, device_sms());
+    const int per = (nc + sh.grid - 1) / sh.grid, most = kResWarps / kChunkRows;
+    const int rounds = (per + most - 1) / most;
+    sh.block = kChunk * ((per + rounds - 1) / rounds);
+    return sh;
 }
 
 static std::mutex g_loop_mu;
@@ -934,9 +1000,21 @@ static void wait_params(bool take, long* limit, int* absent) {
 // take_fault: this run is a solve's (not a tuning trial's), so an armed wait
 // fault applies to it.
 template <typename T>
-static int run_loop(Eng<T> E, const void* work, GridBar* gb, int prec, const LoopShape& sh, cudaStream_t s,
-                    bool take_fault = false) {
+static int run_loop(Eng<T> E, const ResBufs<T>& R, const void* work, GridBar* gb, int prec, const LoopShape& sh,
+                    cudaStream_t s, bool take_fault = false) {
     TraceRange trace_range_("iteration loop");
+    if (sh.graph == 4) {
+        CLOWNS_CUDA_TRY(cudaMemsetAsync(gb, 0, sizeof(GridBar), s));
+        ResBufs<T> r = R;
+        long lim;
+        int absent;
+        wait_params(take_fault, &lim, &absent);
+        void* args[] = {(void*)&E, (void*)&r, (void*)&lim, (void*)&absent};
+        const void* fn = E.nl == 4 ? (const void*)k_res_loop<T, 4> : (const void*)k_res_loop<T, 6>;
+        CLOWNS_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(sh.grid), dim3(sh.block), args, 0, s));
+        t_launches += 1;
+        return CLOWNS_OK;
+    }
     if (sh.bal && E.M > 1 && E.baltab && (sh.graph == 1 || sh.graph == 2)) {
         // ensembles on the balanced kernels: block tables over the members that iterate
         k_bal_rebuild<<<1, kBalScanThreads, 0, s>>>(E.S, E.M, E.mem_n, (BalBlock*)E.baltab, E.balg, E.ctrl + 4);
@@ -1008,6 +1086,12 @@ static int run_loop(Eng<T> E, const void* work, GridBar* gb, int prec, const Loo
     return CLOWNS_OK;
 }
 
+template <typename T>
+static void res_compose(const Eng<T>& E, const ResBufs<T>& R, int grid, cudaStream_t s) {
+    if (E.nl == 4) k_res_compose<T, 4><<<grid, kEngBlock, 0, s>>>(E, R);
+    else k_res_compose<T, 6><<<grid, kEngBlock, 0, s>>>(E, R);
+}
+
 static int check_abort(GridBar* gb, cudaStream_t s) {
     int abort = 0;
     CLOWNS_CUDA_TRY(cudaMemcpyAsync(&abort, &gb->abort, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1028,8 +1112,8 @@ static int check_abort(GridBar* gb, cudaStream_t s) {
 // `prime` re-creates the state the loop starts from.
 constexpr int kTuneIters = 24;
 template <typename T, typename Prime>
-static int tune_loop(Eng<T> E, const void* work, GridBar* gb, long key_nv, int key_prec, Prime prime,
-                     cudaStream_t s, LoopShape* out) {
+static int tune_loop(Eng<T> E, const ResBufs<T>& R, const void* work, GridBar* gb, long key_nv, int key_prec,
+                     Prime prime, cudaStream_t s, LoopShape* out) {
     TraceRange trace_range_("loop autotuner");
     const int forced = forced_loop_mode();
     const bool wave_ok = E.wave != nullptr && E.M == 1;
@@ -1057,6 +1141,12 @@ static int tune_loop(Eng<T> E, const void* work, GridBar* gb, long key_nv, int k
         std::lock_guard<std::mutex> lk(g_loop_mu);
         auto it = g_loop_shapes.find(key);
         if (it != g_loop_shapes.end()) { *out = it->second; return CLOWNS_OK; }
+    }
+    if (R.p && (forced == 4 || forced < 0)) {
+        *out = res_shape(E.n1);
+        std::lock_guard<std::mutex> lk(g_loop_mu);
+        g_loop_shapes[key] = *out;
+        return CLOWNS_OK;
     }
     std::vector<LoopShape> cands;
     // Automatic tuning keeps one shape each of the wavefront and persistent
@@ -1110,7 +1200,7 @@ static int tune_loop(Eng<T> E, const void* work, GridBar* gb, long key_nv, int k
             cands.push_back(sh);
         }
     }
-    if (forced < 0 || (forced == 3 && !wave_ok)) {     // forced wave: ensembles keep the graph
+    if (forced < 0 || (forced == 3 && !wave_ok) || forced == 4) {     // forced wave or resident: systems they do not serve keep the graph
         // FP64 dot-product kernels may run 64 threads per tile (8 rows per
         // thread before the warp sums: half the FP64 additions per row); the
         // FP32 ones have FP32 warp sums and keep 128
@@ -1158,7 +1248,7 @@ static int tune_loop(Eng<T> E, const void* work, GridBar* gb, long key_nv, int k
             if (failed[c]) continue;
             prime(s);
             CLOWNS_CUDA_TRY(cudaEventRecord(e0, s));
-            if (run_loop(E, work, gb, key_prec, cands[c], s)) {
+            if (run_loop(E, R, work, gb, key_prec, cands[c], s)) {
                 cudaGetLastError();
                 failed[c] = 1;
                 continue;
@@ -1312,6 +1402,7 @@ int engine_solve_plain(int M, const MemberIn* ins, double eps, double parm, int 
     if (rc) return rc;
     Eng<double> E = eng_bind<double>(work, L);
     E.nl = nl;
+    const ResBufs<double> R = res_bind<double>(work, L);
     bool bal_ok = false;
     rc = upload_bal_tables<double>(work, L, s, &bal_ok);
     if (rc) return rc;
@@ -1323,6 +1414,7 @@ int engine_solve_plain(int M, const MemberIn* ins, double eps, double parm, int 
         k_eng_init_scalars<<<1, 256, 0, cs>>>(E.S, M, e, it, mode, E.ctrl);
         if (nl == 6) k_eng_setup<double, 6><<<gs, kEngBlock, 0, cs>>>(E, P1, P2, 0);
         else k_eng_setup<double, 4><<<gs, kEngBlock, 0, cs>>>(E, P1, P2, 0);
+        if (R.p) res_compose(E, R, gs, cs);
     };
     // PCGPME's start (b^ = PM W b, q = PM A x0, residuals) as plain launches
     const Shape ksh;
@@ -1333,14 +1425,14 @@ int engine_solve_plain(int M, const MemberIn* ins, double eps, double parm, int 
     };
     LoopShape sh;
     // tuning runs: kTuneIters iterations from the real start (not counted as the solve's launches)
-    rc = tune_loop(E, work, gb, L.NV, 0, [&](cudaStream_t cs) { prime(cs, 1e-300, kTuneIters); start(cs); }, s, &sh);
+    rc = tune_loop(E, R, work, gb, L.NV, 0, [&](cudaStream_t cs) { prime(cs, 1e-300, kTuneIters); start(cs); }, s, &sh);
     if (rc) return rc;
     t_launches = 0;
     prime(s, eps_r, iter_r);
     start(s);
     t_launches += 2 + 8;
     CLOWNS_CUDA_TRY(cudaGetLastError());
-    rc = run_loop(E, work, gb, 0, sh, s, true);
+    rc = run_loop(E, R, work, gb, 0, sh, s, true);
     if (rc) return rc;
     k_eng_copy_out<double><<<gs, kEngBlock, 0, s>>>(E);
     t_launches += 1;
@@ -1382,6 +1474,7 @@ int engine_solve_mixed(int M, const MemberIn* ins, double eps, double parm, doub
     if (rc) return rc;
     Eng<float> E = eng_bind<float>(work, L);
     E.nl = nl;
+    const ResBufs<float> R = res_bind<float>(work, L);
     bool bal_ok = false;
     rc = upload_bal_tables<float>(work, L, s, &bal_ok);
     if (rc) return rc;
@@ -1395,6 +1488,7 @@ int engine_solve_mixed(int M, const MemberIn* ins, double eps, double parm, doub
         k_mixed_init_scalars<<<1, 256, 0, cs>>>(E.S, M, eps_r, max_outer, E.ctrl);
         if (nl == 6) k_eng_setup<float, 6><<<gs, kEngBlock, 0, cs>>>(E, P1, P2, 1);
         else k_eng_setup<float, 4><<<gs, kEngBlock, 0, cs>>>(E, P1, P2, 1);
+        if (R.p) res_compose(E, R, gs, cs);
         launch_ldusub64<float, 0>(E, ksh, inner_tol, inner_max, cs);   // BN64 = ||PM W b||^2
     };
     // one refinement sweep up to the inner loop: residual, PM r, ERR test, inner RHS
@@ -1405,7 +1499,7 @@ int engine_solve_mixed(int M, const MemberIn* ins, double eps, double parm, doub
         k_mx_normalize<float><<<kg, ksh.block, 0, cs>>>(E);
     };
     LoopShape sh;
-    rc = tune_loop(E, work, gb, L.NV, 1, [&](cudaStream_t cs) { setup(cs); sweep_head(cs, 1e-30, kTuneIters); },
+    rc = tune_loop(E, R, work, gb, L.NV, 1, [&](cudaStream_t cs) { setup(cs); sweep_head(cs, 1e-30, kTuneIters); },
                    s, &sh);
     if (rc) return rc;
     t_launches = 0;
@@ -1422,7 +1516,7 @@ int engine_solve_mixed(int M, const MemberIn* ins, double eps, double parm, doub
         bool all = true;
         for (int m = 0; m < M; m++) all = all && h[m].odone;
         if (all) break;
-        rc = run_loop(E, work, gb, 1, sh, s);
+        rc = run_loop(E, R, work, gb, 1, sh, s);
         if (rc) return rc;
         k_mx_update<float><<<kg, ksh.block, 0, s>>>(E);
         t_launches += 1;

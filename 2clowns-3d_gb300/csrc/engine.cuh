@@ -130,7 +130,8 @@ struct Eng {
     MemberScalars* S;
     double* partials;         // 2 per chunk of the row space (chunk totals)
     unsigned* ticket;         // groups summed, one per member
-    int* ctrl;                // [0] loop-body count, [1] max ITER over members, [2] bodies of earlier sweeps
+    int* ctrl;                // [0] loop-body count, [1] max ITER over members, [2] bodies of earlier sweeps,
+                              // [6] first epoch of the next resident loop, [7] epochs used so far
     const BalBlock* baltab;   // ensembles: 16 block tables of the balanced kernels (nullptr: none)
     const int* balg;          // ensembles: the blocks of each table's launch (16)
     int nl;                   // columns the members' matrices fill: 6 (3D) or 4 (2DV, and the 2DH
@@ -527,7 +528,7 @@ static __global__ void k_eng_init_scalars(MemberScalars* S, int M, double eps, i
         z.mode = mode;
         S[m] = z;
     }
-    if (threadIdx.x == 0) { ctrl[0] = 0; ctrl[1] = iter; ctrl[2] = 0; }
+    if (threadIdx.x == 0) { ctrl[0] = 0; ctrl[1] = iter; ctrl[2] = 0; ctrl[6] = 0; ctrl[7] = 0; }
 }
 
 // ---------------------------------------------------------------------------

@@ -171,8 +171,10 @@ int clowns_pcgpme_batched_dev(int m, const clowns_member* members, int precision
  * systems of sizes n[], precision as above).  mode: CLOWNS_LOOP_PERSISTENT
  * (one cooperative kernel, phases separated by grid barriers),
  * CLOWNS_LOOP_GRAPH (a CUDA graph of per-phase kernels chained by programmatic
- * dependent launch) or CLOWNS_LOOP_WAVE (one cooperative kernel running
- * (stage, tile) items in wavefront order; single systems only).  block:
+ * dependent launch), CLOWNS_LOOP_WAVE (one cooperative kernel running
+ * (stage, tile) items in wavefront order; single systems only) or
+ * CLOWNS_LOOP_RESIDENT (one cooperative kernel whose blocks exchange rows as
+ * {value, epoch} words; small and medium single systems, by rule).  block:
  * threads per block; grid: blocks of the cooperative kernels (0 for the graph);
  * regs: their register budget per thread (0 for the graph); fused (graph): bit 0
  * set when LDUSUB's sweeps 1-2 and 3-4 run as fused pairs, bit 1 set when the
@@ -185,6 +187,7 @@ int clowns_pcgpme_batched_dev(int m, const clowns_member* members, int precision
 #define CLOWNS_LOOP_PERSISTENT 0
 #define CLOWNS_LOOP_GRAPH 1
 #define CLOWNS_LOOP_WAVE 3
+#define CLOWNS_LOOP_RESIDENT 4
 int clowns_tuned_shape(int m, const int* n, int precision, int* mode, int* block, int* grid, int* regs,
                        int* fused);
 

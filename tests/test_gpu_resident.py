@@ -1,0 +1,99 @@
+"""The resident iteration loop (one kernel, rows exchanged as {value, epoch} words)
+against the graph of balanced kernels on the same system: the summation tree and
+the per-row arithmetic are the same, so iterations, ERR and pressure must agree
+bit for bit, in FP64 and mixed precision, on matrices with six and four columns,
+with neighbours near by (band) and anywhere (random: self references, repeated
+columns and empty slots among them).  Sizes sit at the edges of its mapping: a
+lane, a 32-row group, a 128-row chunk, a reduction group of 64 chunks, one chunk
+per SM and one round of a block's warps.  A wait that runs out is reported and
+leaves the context usable."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [1, 31, 33, 127, 128, 129, 4097, 8192, 8193, 19456, 19457, 116736, 116737]
+
+
+def _system(n, nl, kind):
+    import torch
+    rng = np.random.default_rng(n * 10 + nl)
+    ll = np.zeros((nl, n), np.int32)
+    if kind == "random":
+        ll[:] = rng.integers(0, n + 1, (nl, n))
+    else:
+        w = max(1, int(n ** 0.5))
+        for k, o in enumerate([-1, 1, -w, w, -3 * w, 3 * w][:nl]):
+            j = np.arange(n) + o
+            ll[k] = np.where((j >= 0) & (j < n), j + 1, 0)
+    al = -rng.uniform(0.05, 1.0, (nl, n)) * (ll > 0)
+    d = 1.02 * np.abs(al).sum(0) + 0.01
+    b = rng.standard_normal(n)
+    return [torch.from_numpy(np.ascontiguousarray(v)).cuda() for v in (al, ll, d, b)]
+
+
+def _solve(gpu, system, mixed, eps):
+    import torch
+    al, ll, d, b = system
+    n = b.numel()
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    s = (gpu.MixedSolver if mixed else gpu.Solver)(n, al.shape[0])
+    info = s.solve(al, ll, d, b, x, eps=eps)
+    return x, info.as_dict()
+
+
+def _force(monkeypatch, mode):
+    monkeypatch.setenv("CLOWNS_LOOP_MODE", mode)
+    monkeypatch.setenv("CLOWNS_SWEEP_FUSE", "1")
+    monkeypatch.setenv("CLOWNS_BALANCED_ROWS", "4")
+
+
+@pytest.mark.parametrize("kind", ["band", "random"])
+@pytest.mark.parametrize("nl", [6, 4])
+@pytest.mark.parametrize("n", SIZES)
+def test_resident_equals_graph(gpu, monkeypatch, n, nl, kind):
+    import torch
+    system = _system(n, nl, kind)
+    for mixed in (False, True):
+        _force(monkeypatch, "graph")
+        xg, ig = _solve(gpu, system, mixed, 1e-10)
+        _force(monkeypatch, "resident")
+        xr, ir = _solve(gpu, system, mixed, 1e-10)
+        assert ir == ig, (mixed, ir, ig)
+        assert torch.equal(xr, xg), mixed
+
+
+def test_resident_nan_and_cap(gpu, monkeypatch):
+    """A NaN right-hand side and an exhausted iteration cap end as in the graph."""
+    import torch
+    al, ll, d, b = _system(4097, 6, "band")
+    bad = b.clone()
+    bad[77] = float("nan")
+    n = b.numel()
+    for rhs, kw in ((bad, {}), (b, {"itmax": 5})):
+        got = []
+        for mode in ("graph", "resident"):
+            _force(monkeypatch, mode)
+            x = torch.zeros(n, dtype=torch.float64, device="cuda")
+            info = gpu.Solver(n).solve(al, ll, d, rhs, x, eps=1e-10, **kw)
+            got.append((x.cpu().numpy(), info.iter, info.ier, info.reason))
+        assert got[0][1:] == got[1][1:]
+        assert np.array_equal(got[0][0], got[1][0], equal_nan=True)
+        assert got[0][2] != 0
+
+
+def test_resident_wait_runs_out_and_context_recovers(gpu, monkeypatch):
+    import torch
+    al, ll, d, b = _system(19457, 6, "band")
+    n = b.numel()
+    _force(monkeypatch, "resident")
+    x_ok, ok = _solve(gpu, (al, ll, d, b), False, 1e-10)
+    assert gpu.lib().clowns_test_arm_wait_timeout(C.c_long(10000), 0) == 0
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    with pytest.raises(gpu.ClownsError) as err:
+        gpu.Solver(n).solve(al, ll, d, b, x, eps=1e-10)
+    assert "(-4)" in str(err.value), str(err.value)
+    x, info = _solve(gpu, (al, ll, d, b), False, 1e-10)
+    assert info == ok and torch.equal(x, x_ok)
