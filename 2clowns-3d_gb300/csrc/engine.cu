@@ -258,10 +258,11 @@ static inline int member_groups(int n) {
 
 // Single systems up to this many rows run the resident loop, without tuning.
 // Measured against the tuned graph (ms per solve, graph / resident): FP64 2.7 /
-// 0.9 at 4 k rows, 6.8 / 2.7 at 74 k, 10.7 / 7.2 at 239 k, 13.6 / 13.9 at 413 k;
-// mixed 3.8 / 1.7, 5.9 / 2.7, 9.2 / 5.3, 10.7 / 8.2, and 17.2 / 18.5 at 660 k.
-constexpr int kResMaxRowsFp64 = 300000;
-constexpr int kResMaxRowsMixed = 500000;
+// 0.9 at 4 k rows, 6.8 / 2.4 at 74 k, 10.6 / 5.8 at 239 k, 12.2 / 9.9 at 413 k,
+// 23.6 / 25.5 at 660 k; mixed 3.9 / 1.7, 5.9 / 2.6, 9.1 / 4.5, 11.0 / 7.5, 17.2 /
+// 15.5 and 20.0 / 28.0 at 960 k (its words and matrix no longer fit L2).
+constexpr int kResMaxRowsFp64 = 500000;
+constexpr int kResMaxRowsMixed = 700000;
 
 struct EngLayout {
     long NV = 0;
@@ -271,7 +272,7 @@ struct EngLayout {
     size_t o_in, o_S, o_partials, o_bar, o_al, o_ll, o_d, o_vec[8], o_W, o_x64, o_r64, o_s64, o_t64;
     size_t o_wave, o_wbuf[kWaveBufs];
     int res = 0;           // the resident loop's words and composed coefficients are laid out
-    size_t o_rword[4], o_rpart, o_ra, o_rc;
+    size_t o_rword[2 + kResSteps], o_rpart, o_rgpart, o_ra, o_rc;
     size_t o_baltab = 0;   // ensembles: block tables of the balanced kernels
     size_t o_balg = 0;     // ensembles: blocks of each table's launch
     size_t total = 0;
@@ -335,8 +336,9 @@ static EngLayout eng_layout(int M, const int* n, int mixed, int wave = -1) {
     }
     L.res = wave < 0 && M == 1 && n[0] <= (mixed ? kResMaxRowsMixed : kResMaxRowsFp64);
     if (L.res) {
-        for (int k = 0; k < 4; k++) L.o_rword[k] = take(2 * (size_t)L.tsize * NV);
+        for (int k = 0; k < 2 + kResSteps; k++) L.o_rword[k] = take(2 * (size_t)L.tsize * NV);
         L.o_rpart = take(sizeof(TagWord<double>) * 6 * (size_t)(NV / kChunk));
+        L.o_rgpart = take(sizeof(TagWord<double>) * 6 * (size_t)ngrp);
         L.o_ra = take((size_t)L.tsize * kResCoef<6> * NV);
         L.o_rc = take(sizeof(int) * kResIdx<6> * (size_t)NV);
     }
@@ -430,9 +432,10 @@ static ResBufs<T> res_bind(void* work, const EngLayout& L) {
     char* b = (char*)work;
     R.p = (TagWord<T>*)(b + L.o_rword[0]);
     R.e = (TagWord<T>*)(b + L.o_rword[1]);
-    R.t0 = (TagWord<T>*)(b + L.o_rword[2]);
-    R.t3 = (TagWord<T>*)(b + L.o_rword[3]);
+    for (int k = 0; k < kResSteps; k++) R.t[k] = (TagWord<T>*)(b + L.o_rword[2 + k]);
     R.part = (TagWord<double>*)(b + L.o_rpart);
+    R.gpart = (TagWord<double>*)(b + L.o_rgpart);
+    R.ngrp = L.ngrp;
     R.a = (T*)(b + L.o_ra);
     R.c = (int*)(b + L.o_rc);
     return R;
@@ -620,8 +623,14 @@ static LoopShape res_shape(int n) {
     sh.grid = std::min(nc, device_sms());
     const int per = (nc + sh.grid - 1) / sh.grid, most = kResWarps / kChunkRows;
     const int rounds = (per + most - 1) / most;
-    sh.block = kChunk * ((per + rounds - 1) / rounds);
+    sh.block = kChunk * ((per + rounds - 1) / rounds) + 32;     // and the scalar warp
     return sh;
+}
+
+template <typename T>
+static void res_compose(const Eng<T>& E, const ResBufs<T>& R, int grid, cudaStream_t s) {
+    if (E.nl == 4) k_res_compose<T, 4><<<grid, kEngBlock, 0, s>>>(E, R);
+    else k_res_compose<T, 6><<<grid, kEngBlock, 0, s>>>(E, R);
 }
 
 static std::mutex g_loop_mu;
@@ -1086,12 +1095,6 @@ static int run_loop(Eng<T> E, const ResBufs<T>& R, const void* work, GridBar* gb
     return CLOWNS_OK;
 }
 
-template <typename T>
-static void res_compose(const Eng<T>& E, const ResBufs<T>& R, int grid, cudaStream_t s) {
-    if (E.nl == 4) k_res_compose<T, 4><<<grid, kEngBlock, 0, s>>>(E, R);
-    else k_res_compose<T, 6><<<grid, kEngBlock, 0, s>>>(E, R);
-}
-
 static int check_abort(GridBar* gb, cudaStream_t s) {
     int abort = 0;
     CLOWNS_CUDA_TRY(cudaMemcpyAsync(&abort, &gb->abort, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1132,6 +1135,12 @@ static int tune_loop(Eng<T> E, const ResBufs<T>& R, const void* work, GridBar* g
         return CLOWNS_OK;
     }
     const auto key = std::make_tuple(key_nv, key_prec, (int)wave_ok, forced);
+    if (R.p && (forced == 4 || forced < 0)) {             // by rule: nothing to time
+        *out = res_shape(E.n1);
+        std::lock_guard<std::mutex> lk(g_loop_mu);
+        g_loop_shapes[key] = *out;                        // for clowns_tuned_shape only
+        return CLOWNS_OK;
+    }
     // CLOWNS_WAVE_PARAMS="K,slack,minb,frac" pins the wavefront candidate (tuning sweeps; read on every call)
     const char* wp = getenv("CLOWNS_WAVE_PARAMS");
     int pk = 0, ps = 0, pm = 0, pf = 0;
@@ -1141,12 +1150,6 @@ static int tune_loop(Eng<T> E, const ResBufs<T>& R, const void* work, GridBar* g
         std::lock_guard<std::mutex> lk(g_loop_mu);
         auto it = g_loop_shapes.find(key);
         if (it != g_loop_shapes.end()) { *out = it->second; return CLOWNS_OK; }
-    }
-    if (R.p && (forced == 4 || forced < 0)) {
-        *out = res_shape(E.n1);
-        std::lock_guard<std::mutex> lk(g_loop_mu);
-        g_loop_shapes[key] = *out;
-        return CLOWNS_OK;
     }
     std::vector<LoopShape> cands;
     // Automatic tuning keeps one shape each of the wavefront and persistent

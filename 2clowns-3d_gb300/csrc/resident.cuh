@@ -16,16 +16,28 @@
 //   - chunk totals of the dot products travel the same way, and every block sums
 //     them itself along the canonical tree (engine.cuh), so every block holds
 //     the same scalars and takes the same stop decisions;
-//   - LDUSUB's sweeps run in two steps instead of five: 1-2-3 and 4-5-6 (four
-//     columns: 1-2 and 3-4).  A row re-evaluates the one or two levels of its
-//     neighbours' sweeps it needs from coefficients composed once per solve
+//   - LDUSUB's sweeps run in pairs (1-2 | 3-4 | 5-6, with four columns 1-2 | 3-4;
+//     5 and 6 are one sweep).  A row re-evaluates the one neighbour value its
+//     pair's second sweep needs from coefficients composed once per solve
 //     (k_res_compose), with the same fused multiply-adds, so the bits are those of
-//     separate sweeps.  That costs 12 more operations per row and iteration and
-//     saves six trips.
+//     separate sweeps.  That costs 4 more operations per row and iteration and
+//     saves four trips.  (us per iteration with pairs / threes, 1-2-3 | 4-5-6, 12
+//     more operations and one trip less each way / single sweeps: FP64 16.6 / 16.7 /
+//     18.5 at 27 k rows, 39.8 / 43.5 / 40.7 at 239 k, 67.0 / 72.6 / 70.4 at 413 k.)
+// What bounds it: a trip takes 0.3-0.5 us; a warp's FP64 operation holds its SM
+// sub-partition for 64 cycles whatever its active lanes (76 with all four busy),
+// so small systems are bound by the chain of dependent FP64 operations and large
+// ones by their number.  Hence: rows are dealt out in groups of 32, one row per
+// lane, so that a chunk's four groups use four sub-partitions; the two totals of
+// a dot-product pair are folded by different warps; an extra warp per block
+// finalises the scalars, and takes the square root and the stop tests of an
+// iteration while the others already run the next one's first steps (after a stop
+// those have only written scratch vectors); x is updated and p - AMU q formed
+// while the totals travel.
 // A word is overwritten only after a reduction of the same iteration that every
 // reader's own contribution had to precede, so no reader can miss its epoch:
-// the operator's intermediates are rewritten once per reduction RQ / AMU, p and
-// e once per iteration, and each of the three reductions has its own totals.
+// the operator's intermediates (a vector of its own for each step) are rewritten
+// once per reduction RQ / AMU, p and e once per iteration, and each of the three reductions has its own totals.
 // Every poll is bounded: a warp that runs out raises the abort flag, polls of
 // the other warps and blocks then give up too, and the block leaves at the next
 // reduction; the host reports the failure.
@@ -37,20 +49,18 @@
 
 namespace clowns {
 
-constexpr int kResThreads = 768;                 // 24 warps: 80 registers per thread
-constexpr int kResWarps = kResThreads / 32;
-constexpr int kResMaxGroups = 512;               // reduction groups of one member (4.2 M rows)
+constexpr int kResWarps = 28;                    // row warps of a block at most
+constexpr int kResThreads = 32 * kResWarps + 32; // and the scalar warp: 64 registers per thread
+constexpr int kResSteps = 3;                     // vectors between the operator's steps (NL / 2 of them used)
 
 // Coefficients and indices of one 32-row group in the resident loop's layout:
 // group-major, each a run of 32 lanes, so that one address and constant offsets
 // reach all of a row's.  With c1..c6 the row's columns in sweep order:
-//   slots 0..5 AL(1..6) / LL(1..6);
-//   six columns   6: sweep 2 at c3   7: sweep 1 at c3   8: sweep 1 at c2
-//                 9: sweep 1 at c2(c3)   10: sweep 4 at c5   11: sweep 4 at c6
-//   four columns  4: sweep 1 at c2   5: sweep 3 at c4
+//   slots 0..NL-1   AL(1..NL) / LL(1..NL)
+//   slots NL, NL+1  sweep 1's coefficient and index at row c2, sweep 3's at c4
 //   last coefficient: D
 template <int NL>
-constexpr int kResIdx = NL == 6 ? 12 : 6;
+constexpr int kResIdx = NL + 2;
 template <int NL>
 constexpr int kResCoef = kResIdx<NL> + 1;
 
@@ -96,10 +106,12 @@ __device__ __forceinline__ unsigned tag_get(const TagWord<float>* p, float& v) {
 // Words and composed coefficients of the resident loop (pointers into the workspace).
 template <typename T>
 struct ResBufs {
-    TagWord<T> *p, *e, *t0, *t3;     // NV words each
+    TagWord<T> *p, *e, *t[kResSteps];   // NV words each
     TagWord<double>* part;           // 3 reductions x 2 values x (NV / kChunk) chunk totals
-    T* a;                            // kResCoef x 32 per 32-row group
-    int* c;                          // kResIdx x 32 per 32-row group
+    TagWord<double>* gpart;          // 3 reductions x 2 values x ngrp group totals
+    int ngrp;                        // groups of all members
+    T* a;                            // coefficients, kResCoef x 32 per 32-row group
+    int* c;                          // indices, kResIdx x 32 per 32-row group
     const BalBlock* tab;             // one entry per block (nullptr: a single system)
 };
 
@@ -109,36 +121,27 @@ template <typename T, int NL>
 __global__ void __launch_bounds__(kEngBlock) k_res_compose(Eng<T> E, ResBufs<T> R) {
     const long NV = E.NV;
     const long stride = (long)gridDim.x * blockDim.x, t0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int NI = kResIdx<NL>;
     for (long i = t0; i < 6 * (NV / kChunk); i += stride) R.part[i].tag = 0;
+    for (long i = t0; i < 6 * R.ngrp; i += stride) R.gpart[i].tag = 0;
     for (long i = t0; i < NV; i += stride) {
         const int m = E.blk_member[i / kTile];
         if (m < 0) continue;
         R.p[i].tag = 0;
         R.e[i].tag = 0;
-        R.t0[i].tag = 0;
-        R.t3[i].tag = 0;
-        T* a = R.a + (i >> 5) * (32 * kResCoef<NL>) + (i & 31);
-        int* c = R.c + (i >> 5) * (32 * kResIdx<NL>) + (i & 31);
-        auto put = [&](int slot, int k, long j) {
-            a[32 * slot] = E.al[k * NV + j];
-            c[32 * slot] = E.ll[k * NV + j];
+#pragma unroll
+        for (int k = 0; k < NL / 2; k++) R.t[k][i].tag = 0;
+        T* a = R.a + (i >> 5) * (32 * (NI + 1)) + (i & 31);
+        int* c = R.c + (i >> 5) * (32 * NI) + (i & 31);
+        auto put = [&](int slot, int sweep, long j) {
+            a[32 * slot] = E.al[(sweep - 1) * NV + j];
+            c[32 * slot] = E.ll[(sweep - 1) * NV + j];
         };
 #pragma unroll
-        for (int k = 0; k < NL; k++) put(k, k, i);
-        a[32 * kResIdx<NL>] = E.d[i];
-        const int c2 = E.ll[1 * NV + i];
-        if (NL == 6) {
-            const int c3 = E.ll[2 * NV + i];
-            put(6, 1, c3);
-            put(7, 0, c3);
-            put(8, 0, c2);
-            put(9, 0, E.ll[1 * NV + c3]);
-            put(10, 3, E.ll[4 * NV + i]);
-            put(11, 3, E.ll[5 * NV + i]);
-        } else {
-            put(4, 0, c2);
-            put(5, 2, E.ll[3 * NV + i]);
-        }
+        for (int k = 0; k < NL; k++) put(k, k + 1, i);
+        a[32 * NI] = E.d[i];
+        put(NL, 1, E.ll[1 * NV + i]);
+        put(NL + 1, 3, E.ll[3 * NV + i]);
     }
 }
 
@@ -184,13 +187,66 @@ __device__ __forceinline__ void res_gather(const TagWord<T>* __restrict__ buf, c
     }
 }
 
-// The reductions' finalisations out of line: one thread runs them, and inlined
-// their divisions and square roots would raise the loop's register count.
-__device__ __noinline__ void res_finish(int red, MemberScalars* S, double t0, double t1) {
-    const double tot[2] = {t0, t1};
-    if (red == 0) finish_sweep56<1, true>(S, tot, S);
-    else if (red == 1) finish_sweep56<2, true>(S, tot, S);
-    else finish_xrupdate<true>(S, tot, S);
+// Integer forms of the scalar tests: an FP64 comparison costs as much as an addition.
+__device__ __forceinline__ bool f64_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+__device__ __forceinline__ bool f64_finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+
+// finish_xrupdate's stop tests (pcgpme_para.F90:215-254) by one thread, BETA
+// already formed.  ERR = sqrt(RN / BN) takes a division and a square root, some 2000
+// cycles in which the next reduction would wait; but with q = RN (1 / BN), within a
+// few roundings of ERR^2, two inequalities rule both tests out in nearly every
+// iteration: q above EPS^2, and |q - q_prev| above 2e-6 q (|ERR - ERRP| <= 1e-6 ERR
+// gives at most that).  Otherwise ERR and ERRP are formed and compared exactly as
+// finish_xrupdate does; at the loop's end ERR is formed from RN in any case.
+struct ResStop {
+    double invbn, eps2, q, rn_prev;
+};
+__device__ __noinline__ void res_stop_exact(MemberScalars* S, double RN, double rn_prev) {
+    const double ERR = sqrt(RN / S->BN);                         // 215
+    const double ERRP = S->K > 1 ? sqrt(rn_prev / S->BN) : S->ERRP;
+    S->ERR = ERR;
+    if (S->K >= 10 && fabs(ERR - ERRP) <= ERR * 1.0e-6) {        // 228
+        stop_member(S, CLOWNS_STOP_STAGNATION, 0);
+        S->ERRP = ERRP;
+    } else if (ERR <= S->EPS) {                                  // 232
+        stop_member(S, CLOWNS_STOP_TOL, 0);
+        S->ERRP = ERRP;
+    }
+}
+__device__ __forceinline__ void res_stop_tests(MemberScalars* S, ResStop& st, double RN, double C1, double BETA) {
+    const double q = RN * st.invbn, dq = fabs(q - st.q);
+    const int K = S->K + 1;
+    S->RN = RN;
+    S->C1 = C1;
+    S->K = K;
+    S->total_iter += 1;
+    if (!f64_finite(RN) || !f64_finite(C1)) {
+        S->ERR = sqrt(RN / S->BN);
+        stop_member(S, CLOWNS_STOP_NONFINITE, S->mode != 1 ? CLOWNS_IER_NONFINITE : 0);
+        return;
+    }
+    // q in (1e-290, 1e290) by its exponent; a NaN fails the comparisons
+    const int ex = (__double2hiint(q) >> 20) & 0x7ff;
+    const bool clear = ex > 60 && ex < 1986 && q > st.eps2 && dq > 2.1e-6 * q;
+    if (!clear) res_stop_exact(S, RN, st.rn_prev);
+    st.q = q;
+    st.rn_prev = RN;
+    if (S->done) return;
+    if (f64_zero(S->AMU)) {                                      // 234
+        stop_member(S, CLOWNS_STOP_AMU_ZERO, 0);
+    } else if (f64_zero(C1)) {                                   // 240
+        stop_member(S, CLOWNS_STOP_C1_ZERO, 0);
+    } else {
+        S->BETA = BETA;
+        if (K >= S->ITER) {                                      // 250-254
+            if (S->mode != 1) {
+                stop_member(S, CLOWNS_STOP_MAXITER, CLOWNS_IER_MAXITER);
+                S->K = S->ITER + 1;
+            } else {
+                stop_member(S, CLOWNS_STOP_MAXITER, 0);
+            }
+        }
+    }
 }
 
 // Shared state of one block of the resident loop.
@@ -198,76 +254,91 @@ template <typename T>
 struct ResShared {
     MemberScalars s;
     T y[kResWarps][32], u[kResWarps][32];
-    double g[2 * kResMaxGroups];
+    double beta;         // of the iteration that starts (its stop tests may still run)
+    ResStop st;
     int fail;            // a poll ran out
-    int stop;            // thread 0's verdict at the last reduction: leave the loop
+    int stop;            // the scalar warp's verdict at the last reduction: leave the loop
 };
 
-// Totals of the member's chunk totals (reduction `red`, epoch tag), summed by
-// this block along the canonical tree; fin(tot) runs in thread 0, and every
-// thread leaves after a block barrier.
-template <int NVAL, typename T>
-__device__ __forceinline__ void res_totals(const TagWord<double>* part, int nc, unsigned tag, ResShared<T>& sh,
-                                           const ResWait& wt, int red) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int ng = (nc + kGroupChunks - 1) / kGroupChunks;
+// The sum of up to 64 tagged pairs by one warp, along the canonical tree of a
+// group: lane l adds words l and l + 32, then the butterfly.  NVAL = 2: value k in
+// lanes 16 k .. 16 k + 15.
+template <int NVAL>
+__device__ __forceinline__ double res_group(const TagWord<double>* p, int cnt, unsigned tag, const ResWait& wt) {
+    const int lane = threadIdx.x & 31;
+    double a[2][NVAL];
+    long spins = 0;
 #pragma unroll 1
-    for (int g = w; g < ng; g += nw) {
-        const int cg = min(kGroupChunks, nc - g * kGroupChunks);
-        const TagWord<double>* p = part + 2L * g * kGroupChunks;
-        double a[2][NVAL];
-        long spins = 0;
-#pragma unroll 1
-        for (;;) {
-            unsigned bad = 0;
+    for (;;) {
+        unsigned bad = 0;
 #pragma unroll
-            for (int h = 0; h < 2; h++)
+        for (int h = 0; h < 2; h++)
 #pragma unroll
-                for (int k = 0; k < NVAL; k++) {
-                    a[h][k] = 0.0;
-                    if (lane + 32 * h < cg) bad |= tag_get(p + 2 * (lane + 32 * h) + k, a[h][k]) ^ tag;
-                }
-            if (__all_sync(0xffffffffu, bad == 0)) break;
-            if (!__all_sync(0xffffffffu, wt.more(spins))) break;
-        }
-        if (lane + 32 < cg)
+            for (int k = 0; k < NVAL; k++) {
+                a[h][k] = 0.0;
+                if (lane + 32 * h < cnt) bad |= tag_get(p + 2 * (lane + 32 * h) + k, a[h][k]) ^ tag;
+            }
+        if (__all_sync(0xffffffffu, bad == 0)) break;
+        if (!__all_sync(0xffffffffu, wt.more(spins))) break;
+    }
+    if (cnt > 32) {
+        if (lane + 32 < cnt)
 #pragma unroll
             for (int k = 0; k < NVAL; k++) a[0][k] += a[1][k];
-        if (NVAL == 1) {
-            const double s = warp_sum(a[0][0]);
-            if (lane == 0) sh.g[2 * g] = s;
-        } else {
-            const double s = warp_pair_sum(a[0][0], a[0][NVAL - 1]);
-            if ((lane & 15) == 0) sh.g[2 * g + (lane >> 4)] = s;
-        }
-    }
-    if (ng > 1) __syncthreads();
-    if (w == 0) {
         __syncwarp();
-        double a = 0.0, b = 0.0, tot[2];
-        for (int j = lane; j < ng; j += 32) {
-            a += sh.g[2 * j];
-            if (NVAL == 2) b += sh.g[2 * j + 1];
-        }
-        if (ng > 1) {
-            if (NVAL == 1) {
-                tot[0] = warp_sum(a);
-                tot[1] = 0.0;
-            } else {
-                const double s = warp_pair_sum(a, b);
-                tot[0] = __shfl_sync(0xffffffffu, s, 0);
-                tot[1] = __shfl_sync(0xffffffffu, s, 16);
-            }
-        } else {                          // one group: the butterfly adds zeros only
-            tot[0] = a;
-            tot[1] = b;
-        }
-        if (lane == 0) {
-            res_finish(red, &sh.s, tot[0], tot[1]);
-            sh.stop = sh.s.done || *(volatile int*)&sh.fail;
-        }
     }
-    __syncthreads();
+    return NVAL == 1 ? warp_sum(a[0][0]) : warp_pair_sum(a[0][0], a[0][NVAL - 1]);
+}
+
+// Member totals of one reduction (epoch tag), by the scalar warp of every block.
+// Up to 64 chunks (one group) each block sums the chunk totals itself; otherwise
+// a group is summed by one block -- the one that holds its first chunk -- and its
+// total published, and every block sums the groups: 152 blocks polling every
+// chunk total held up the stores they waited for (3-6 us per reduction at 27 k -
+// 74 k rows).  Totals in every lane.
+template <int NVAL>
+__device__ __forceinline__ void res_totals(const TagWord<double>* part, TagWord<double>* gpart, int nc, int c0, int c1,
+                                           unsigned tag, const ResWait& wt, double (&tot)[2]) {
+    const int lane = threadIdx.x & 31;
+    const int ng = (nc + kGroupChunks - 1) / kGroupChunks;
+    double s;
+    if (ng == 1) {
+        s = res_group<NVAL>(part, nc, tag, wt);
+        s += 0.0;                             // the member sum starts from 0
+    } else {
+#pragma unroll 1
+        for (int g = (c0 + kGroupChunks - 1) / kGroupChunks; g * kGroupChunks < c1; g++) {
+            const double t = res_group<NVAL>(part + 2L * g * kGroupChunks, min(kGroupChunks, nc - g * kGroupChunks),
+                                             tag, wt);
+            if ((lane & (32 / NVAL - 1)) == 0) tag_put(gpart + 2 * g + lane / (32 / NVAL), t, tag);
+        }
+        double a[NVAL];
+#pragma unroll
+        for (int k = 0; k < NVAL; k++) a[k] = 0.0;
+        long spins = 0;
+#pragma unroll 1
+        for (int j = lane; j < ((ng + 31) & ~31); j += 32) {      // lane l: groups l, l + 32, ... in order
+            double v[NVAL];
+#pragma unroll 1
+            for (;;) {
+                unsigned bad = 0;
+#pragma unroll
+                for (int k = 0; k < NVAL; k++) {
+                    v[k] = 0.0;
+                    if (j < ng) bad |= tag_get(gpart + 2 * j + k, v[k]) ^ tag;
+                }
+                if (__all_sync(0xffffffffu, bad == 0)) break;
+                if (!__all_sync(0xffffffffu, wt.more(spins))) break;
+            }
+            if (j < ng)
+#pragma unroll
+                for (int k = 0; k < NVAL; k++) a[k] += v[k];
+        }
+        __syncwarp();
+        s = NVAL == 1 ? warp_sum(a[0]) : warp_pair_sum(a[0], a[NVAL - 1]);
+    }
+    tot[0] = __shfl_sync(0xffffffffu, s, 0);
+    tot[1] = __shfl_sync(0xffffffffu, s, 16);
 }
 
 // One block's walk over its rows: 32-row groups of its chunks, one row per
@@ -283,7 +354,8 @@ template <typename T, int NL>
 __global__ void __launch_bounds__(kResThreads, 1) k_res_loop(Eng<T> E, ResBufs<T> R, long limit, int absent) {
     if ((int)blockIdx.x == absent) return;
     __shared__ ResShared<T> sh;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int nw = (blockDim.x >> 5) - 1, ws = nw;      // row warps; the scalar warp
     BalBlock bb;
     long off;
     int n, c0, c1;
@@ -294,12 +366,20 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_loop(Eng<T> E, ResBufs<T
     const unsigned ep = (unsigned)sld(E.ctrl + 6);
     const ResWait wt{limit, E.abort, &sh.fail};
     __syncthreads();
-    constexpr int NC = kResCoef<NL>, NI = kResIdx<NL>;
-    const int nc = (n + kChunk - 1) / kChunk, nq = 4 * (c1 - c0), pad = (int)off + n;
-    const int nround = (nq + nw - 1) / nw;
+    if (w == ws && lane == 0) {
+        // EPS^2 with a margin far above the roundings of q (an EPS whose square underflows
+        // gives 0: then q decides, and q = 0 goes to the exact tests)
+        sh.st = ResStop{1.0 / sh.s.BN, sh.s.EPS * sh.s.EPS * (1.0 + 1e-9), 0.0, 0.0};
+    }
+    constexpr int NI = kResIdx<NL>, NC = NI + 1;
+    const int nc = (n + kChunk - 1) / kChunk, pad = (int)off + n;
+    const int nq = w == ws ? 0 : 4 * (c1 - c0);         // the scalar warp has no rows
+    const int nround = (4 * (c1 - c0) + nw - 1) / nw;
     const unsigned row0 = (unsigned)(off + (long)c0 * kChunk) + lane;
     TagWord<double>* part = R.part + 2 * (off / kChunk);
     const long pstride = 2 * (E.NV / kChunk);
+    TagWord<double>* gpart = R.gpart + 2 * E.mem_grp0[bb.m];
+    const int gstride = 2 * R.ngrp;
     auto row = [&](int q) {
         unsigned i = row0 + 32u * q;
         asm volatile("" : "+r"(i));          // addresses are formed in each phase, not carried through all of them
@@ -307,7 +387,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_loop(Eng<T> E, ResBufs<T
     };
     auto coef = [&](const ResRow& rw) { return R.a + (size_t)(rw.i >> 5) * (32 * NC) + lane; };
     auto idx = [&](const ResRow& rw) { return R.c + (size_t)(rw.i >> 5) * (32 * NI) + lane; };
-    // t0 = D in + sum_k AL_k in[LL_k] (as k_bal_axsub)
+    auto self = [&](const ResRow& rw) { return rw.ok ? (int)rw.i : pad; };
+    // t[0] = D in + sum_k AL_k in[LL_k] (as k_bal_axsub)
     auto axsub = [&](const TagWord<T>* in, const T* own, unsigned tag) {
 #pragma unroll 1
         for (int q = w; q < nq; q += nw) {
@@ -322,85 +403,70 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_loop(Eng<T> E, ResBufs<T
             res_gather<T, NL>(in, c, pad, tag, g, wt);
 #pragma unroll
             for (int k = 0; k < NL; k++) s = fma_rn(a[32 * k], g[k], s);
-            if (rw.ok) tag_put(R.t0 + rw.i, s, tag);
+            if (rw.ok) tag_put(R.t[0] + rw.i, s, tag);
         }
     };
-    // sweeps 1-2-3 (1-2 of four columns): t3 from t0
-    auto sweeps_a = [&](unsigned tag) {
+    // Sweeps S, S + 1 of LDUSUB at a row, from the words `in`; X: the slot of sweep S at
+    // column S + 1.
+    auto pair = [&](const ResRow& rw, const TagWord<T>* in, unsigned tag, auto S, auto X) {
+        constexpr int s = decltype(S)::value - 1, x = decltype(X)::value;
+        const T* a = coef(rw);
+        const int* cp = idx(rw);
+        const int c[4] = {self(rw), cp[32 * s], cp[32 * (s + 1)], cp[32 * x]};
+        T g[4];
+        res_gather<T, 4>(in, c, pad, tag, g, wt);
+        const T o = fnma(a[32 * s], g[1], g[0]);
+        return fnma(a[32 * (s + 1)], fnma(a[32 * x], g[3], g[2]), o);
+    };
+    using std::integral_constant;
+#define RES_K(k) integral_constant<int, k>()
+    // every step of LDUSUB but the last, from t[0]
+    auto step = [&](int k, unsigned tag, auto S, auto X) {
 #pragma unroll 1
         for (int q = w; q < nq; q += nw) {
             const ResRow rw = row(q);
+            const T o = pair(rw, R.t[k], tag, S, X);
+            if (rw.ok) tag_put(R.t[k + 1] + rw.i, o, tag);
+        }
+    };
+    auto sweeps = [&](unsigned tag) {
+        step(0, tag, RES_K(1), RES_K(NL));
+        if constexpr (NL == 6) step(1, tag, RES_K(3), RES_K(NL + 1));
+    };
+    // the last step at one row
+    auto last = [&](const ResRow& rw, unsigned tag) {
+        if constexpr (NL == 4) {
+            return pair(rw, R.t[1], tag, RES_K(3), RES_K(NL + 1));
+        } else {
             const T* a = coef(rw);
             const int* cp = idx(rw);
-            T o;
-            if constexpr (NL == 6) {
-                const int c[8] = {rw.ok ? (int)rw.i : pad, cp[0], cp[32], cp[64], cp[32 * 6], cp[32 * 7], cp[32 * 8],
-                                  cp[32 * 9]};
-                T g[8];
-                res_gather<T, 8>(R.t0, c, pad, tag, g, wt);
-                const T o1c3 = fnma(a[32 * 7], g[5], g[3]);         // sweep 1 at c3
-                const T o1x = fnma(a[32 * 9], g[7], g[4]);          // at c2(c3)
-                const T o2c3 = fnma(a[32 * 6], o1x, o1c3);          // sweep 2 at c3
-                const T o1c2 = fnma(a[32 * 8], g[6], g[2]);         // sweep 1 at c2
-                const T o2 = fnma(a[32], o1c2, fnma(a[0], g[1], g[0]));
-                o = fnma(a[64], o2c3, o2);
-            } else {
-                const int c[4] = {rw.ok ? (int)rw.i : pad, cp[0], cp[32], cp[32 * 4]};
-                T g[4];
-                res_gather<T, 4>(R.t0, c, pad, tag, g, wt);
-                const T o1c2 = fnma(a[32 * 4], g[3], g[2]);
-                o = fnma(a[32], o1c2, fnma(a[0], g[1], g[0]));
-            }
-            if (rw.ok) tag_put(R.t3 + rw.i, o, tag);
+            const int c[3] = {self(rw), cp[32 * 4], cp[32 * 5]};
+            T g[3];
+            res_gather<T, 3>(R.t[2], c, pad, tag, g, wt);
+            return fnma(a[32 * 5], g[2], fnma(a[32 * 4], g[1], g[0]));
         }
     };
-    // sweeps 4-5-6 (3-4 of four columns) at row rw
-    auto sweeps_b = [&](const ResRow& rw, unsigned tag) {
-        const T* a = coef(rw);
-        const int* cp = idx(rw);
-        if constexpr (NL == 6) {
-            const int c[6] = {rw.ok ? (int)rw.i : pad, cp[32 * 3], cp[32 * 4], cp[32 * 5], cp[32 * 10], cp[32 * 11]};
-            T g[6];
-            res_gather<T, 6>(R.t3, c, pad, tag, g, wt);
-            const T o45 = fnma(a[32 * 10], g[4], g[2]);
-            const T o46 = fnma(a[32 * 11], g[5], g[3]);
-            const T o4 = fnma(a[32 * 3], g[1], g[0]);
-            return fnma(a[32 * 5], o46, fnma(a[32 * 4], o45, o4));
-        } else {
-            const int c[4] = {rw.ok ? (int)rw.i : pad, cp[32 * 2], cp[32 * 3], cp[32 * 5]};
-            T g[4];
-            res_gather<T, 4>(R.t3, c, pad, tag, g, wt);
-            const T o3c4 = fnma(a[32 * 5], g[3], g[2]);
-            return fnma(a[32 * 3], o3c4, fnma(a[32 * 2], g[1], g[0]));
-        }
-    };
-    // The chunk totals of one round (nw / 4 chunks): lane l of a chunk's warp folds
-    // its rows 32 u + l in order, then the butterfly.  MODE 0: (u, y); 1: (u, y)
-    // and (y, y); 2: (y, y) and (y, u).
+    // The chunk totals of one round (nw / 4 chunks, their rows' y and u in shared
+    // memory): lane l of a chunk's warp folds its rows 32 u + l in order, then the
+    // butterfly.  MODE 0: (u, y); 1: (u, y) and (y, y); 2: (y, y) and (y, u), each
+    // total by a warp of its own.
     auto fold = [&](int rd, int red, unsigned tag, auto mode) {
         constexpr int MODE = decltype(mode)::value;
         constexpr int NVAL = MODE == 0 ? 1 : 2;
         __syncthreads();
-        const int cc = c0 + rd * (nw / 4) + w;
-        if (w < nw / 4 && cc < c1) {
-            T v[NVAL];
-#pragma unroll
-            for (int k = 0; k < NVAL; k++) v[k] = T(0);
+        const int cw = w / NVAL, k = w % NVAL, cc = c0 + rd * (nw / 4) + cw;
+        if (cw < nw / 4 && cc < c1) {
+            const bool square = MODE == 1 ? k == 1 : MODE == 2 ? k == 0 : false;
+            T v = T(0);
 #pragma unroll
             for (int u = 0; u < kChunkRows; u++) {
                 if ((long)cc * kChunk + 32 * u + lane >= n) continue;
-                const T y = sh.y[4 * w + u][lane], b = sh.u[4 * w + u][lane];
-                if (MODE == 2) {
-                    v[0] = fma_rn(y, y, v[0]);
-                    v[NVAL - 1] = fma_rn(y, b, v[NVAL - 1]);
-                } else {
-                    v[0] = fma_rn(b, y, v[0]);
-                    if (MODE == 1) v[NVAL - 1] = fma_rn(y, y, v[NVAL - 1]);
-                }
+                const T y = sh.y[4 * cw + u][lane], b = square ? y : sh.u[4 * cw + u][lane];
+                v = fma_rn(b, y, v);
             }
-            int idx;
-            const T s = warp_tsum<T, NVAL>(v, idx);
-            if ((lane & (32 / NVAL - 1)) == 0) tag_put(part + red * pstride + 2 * cc + idx, (double)s, tag);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) tag_put(part + red * pstride + 2 * cc + k, (double)v, tag);
         }
         if (rd + 1 < nround) __syncthreads();
     };
@@ -408,35 +474,43 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_loop(Eng<T> E, ResBufs<T
 #pragma unroll 1
     for (;; it++) {
         const unsigned ta = 2 * (ep + it) + 1, tb = ta + 1;
+        double tot[2];
         {                                                   // p = r + BETA (p - AMU q), published
-            const T BETA = T(sh.s.BETA), AMU = T(sh.s.AMU);
+            const T BETA = T(sh.beta);
 #pragma unroll 1
             for (int q = w; q < nq; q += nw) {
                 const ResRow rw = row(q);
-                T p = E.p[rw.i];
+                T p = E.p[rw.i];                            // p - AMU q after the first iteration
                 if (it > 0) {
-                    p = fma_rn(BETA, fnma(AMU, E.q[rw.i], p), E.r[rw.i]);
+                    p = fma_rn(BETA, p, E.r[rw.i]);
                     if (rw.ok) E.p[rw.i] = p;
                 }
                 if (rw.ok) tag_put(R.p + rw.i, p, ta);
             }
         }
         axsub(R.p, E.p, ta);                                // q = PM A p ; RQ -> ALP
-        sweeps_a(ta);
+        sweeps(ta);
 #pragma unroll 1
         for (int rd = 0; rd < nround; rd++) {
-            const int q = rd * nw + w;
+            const int q = rd * nw + w;                      // past nq in the scalar warp
             if (q < nq) {
                 const ResRow rw = row(q);
                 const T r0 = E.r0[rw.i];
-                const T y = sweeps_b(rw, ta);
+                const T y = last(rw, ta);
                 if (rw.ok) E.q[rw.i] = y;
                 sh.y[w][lane] = y;
                 sh.u[w][lane] = r0;
             }
-            fold(rd, 0, ta, std::integral_constant<int, 0>());
+            fold(rd, 0, ta, RES_K(0));
         }
-        res_totals<1>(part, nc, ta, sh, wt, 0);
+        if (w == ws) {
+            res_totals<1>(part, gpart, nc, c0, c1, ta, wt, tot);
+            if (lane == 0) {
+                if (!sh.s.done) finish_sweep56<1, true>(&sh.s, tot, &sh.s);   // done: by the last iteration's stop tests
+                sh.stop = sh.s.done || *(volatile int*)&sh.fail;
+            }
+        }
+        __syncthreads();
         if (sh.stop) break;
         {                                                   // e = r - ALP q, published
             const T ALP = T(sh.s.ALP);
@@ -451,46 +525,73 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_loop(Eng<T> E, ResBufs<T
             }
         }
         axsub(R.e, E.e, tb);                                // v = PM A e ; AMU
-        sweeps_a(tb);
+        sweeps(tb);
 #pragma unroll 1
         for (int rd = 0; rd < nround; rd++) {
-            const int q = rd * nw + w;
+            const int q = rd * nw + w;                      // past nq in the scalar warp
             if (q < nq) {
                 const ResRow rw = row(q);
                 const T e = E.e[rw.i];
-                const T y = sweeps_b(rw, tb);
+                const T y = last(rw, tb);
                 if (rw.ok) E.v[rw.i] = y;
                 sh.y[w][lane] = y;
                 sh.u[w][lane] = e;
             }
-            fold(rd, 1, tb, std::integral_constant<int, 1>());
+            fold(rd, 1, tb, RES_K(1));
         }
-        res_totals<2>(part + pstride, nc, tb, sh, wt, 1);
-        if (sh.stop) break;
-        {                                                   // x, r ; RN, C1 ; stop tests
-            const T ALP = T(sh.s.ALP), AMU = T(sh.s.AMU);
-#pragma unroll 1
-            for (int rd = 0; rd < nround; rd++) {
-                const int q = rd * nw + w;
-                if (q < nq) {
-                    const ResRow rw = row(q);
-                    const long i = rw.i;
-                    const T ev = E.e[i], r0 = E.r0[i];
-                    const T xn = fma_rn(AMU, ev, fma_rn(ALP, E.p[i], E.xi[i]));
-                    const T rn = fnma(AMU, E.v[i], ev);
-                    if (rw.ok) {
-                        E.xi[i] = xn;
-                        E.r[i] = rn;
-                    }
-                    sh.y[w][lane] = rn;
-                    sh.u[w][lane] = r0;
-                }
-                fold(rd, 2, ta, std::integral_constant<int, 2>());
+        if (w == ws) {
+            res_totals<2>(part + pstride, gpart + gstride, nc, c0, c1, tb, wt, tot);
+            if (lane == 0) {
+                finish_sweep56<2, true>(&sh.s, tot, &sh.s);
+                sh.stop = sh.s.done || *(volatile int*)&sh.fail;
             }
         }
-        res_totals<2>(part + 2 * pstride, nc, ta, sh, wt, 2);
+        __syncthreads();
         if (sh.stop) break;
+        const T ALP = T(sh.s.ALP), AMU = T(sh.s.AMU);       // x, r ; RN, C1 ; stop tests
+#pragma unroll 1
+        for (int rd = 0; rd < nround; rd++) {
+            const int q = rd * nw + w;                      // past nq in the scalar warp
+            if (q < nq) {
+                const ResRow rw = row(q);
+                const T r0 = E.r0[rw.i];
+                const T rn = fnma(AMU, E.v[rw.i], E.e[rw.i]);
+                if (rw.ok) E.r[rw.i] = rn;
+                sh.y[w][lane] = rn;
+                sh.u[w][lane] = r0;
+            }
+            fold(rd, 2, ta, RES_K(2));
+        }
+#pragma unroll 1
+        for (int q = w; q < nq; q += nw) {                  // while the totals travel
+            const ResRow rw = row(q);
+            if (rw.ok) {
+                const T p = E.p[rw.i];
+                E.xi[rw.i] = fma_rn(AMU, E.e[rw.i], fma_rn(ALP, p, E.xi[rw.i]));
+                E.p[rw.i] = fnma(AMU, E.q[rw.i], p);
+            }
+        }
+        double beta = 0.0;
+        if (w == ws) {
+            res_totals<2>(part + 2 * pstride, gpart + 2 * gstride, nc, c0, c1, ta, wt, tot);
+            if (lane == 0) {                                // 241 (pcgpme_para.F90); pcgpme_2DH.f90:255
+                beta = sh.s.mode == 2 ? tot[1] / (sh.s.AMU * sh.s.RQ) : tot[1] / sh.s.AMU / sh.s.RQ;
+                sh.beta = beta;
+            }
+        }
+        __syncthreads();
+        // the stop tests, while the row warps start the next iteration; the verdict counts
+        // at its first reduction
+        if (w == ws && lane == 0) res_stop_tests(&sh.s, sh.st, tot[0], tot[1], beta);
     }
+#undef RES_K
+    if (bb.j == 0 && w == ws && lane == 0 && sh.s.K > 0 && f64_finite(sh.s.RN)) {
+        // ERR of the last iteration, and ERRP where no stop test kept the older one
+        sh.s.ERR = sqrt(sh.s.RN / sh.s.BN);
+        if (!(sh.s.done && (sh.s.reason == CLOWNS_STOP_STAGNATION || sh.s.reason == CLOWNS_STOP_TOL)))
+            sh.s.ERRP = sh.s.ERR;
+    }
+    __syncthreads();
     if (bb.j == 0) {                                        // the member's scalars, for the host and later kernels
         constexpr int W = (int)(sizeof(MemberScalars) / 4);
         if (threadIdx.x < W) ((int*)(E.S + bb.m))[threadIdx.x] = ((const int*)&sh.s)[threadIdx.x];

@@ -14,7 +14,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 31, 33, 127, 128, 129, 4097, 8192, 8193, 19456, 19457, 116736, 116737]
+SIZES = [1, 31, 33, 127, 128, 129, 4097, 8192, 8193, 19456, 19457, 136192, 136193]
 
 
 def _system(n, nl, kind):
@@ -82,6 +82,23 @@ def test_resident_nan_and_cap(gpu, monkeypatch):
         assert got[0][1:] == got[1][1:]
         assert np.array_equal(got[0][0], got[1][0], equal_nan=True)
         assert got[0][2] != 0
+
+
+@pytest.mark.parametrize("eps", [1e-6, 1.1e-15])
+@pytest.mark.parametrize("n", [129, 8193])
+def test_resident_stop_tests(gpu, monkeypatch, n, eps):
+    """The stop decisions, ERR and the last residual state at a loose and at an
+    unreachable tolerance (stagnation, or a residual that ends in zeros)."""
+    import torch
+    al, ll, d, b = _system(n, 6, "band")
+    got = []
+    for mode in ("graph", "resident"):
+        _force(monkeypatch, mode)
+        x = torch.zeros(n, dtype=torch.float64, device="cuda")
+        info = gpu.Solver(n).solve(al, ll, d, b, x, eps=eps, itmax=400)
+        got.append((x.cpu().numpy(), info.as_dict()))
+    assert str(got[0][1]) == str(got[1][1])
+    assert np.array_equal(got[0][0], got[1][0], equal_nan=True)
 
 
 def test_resident_wait_runs_out_and_context_recovers(gpu, monkeypatch):
