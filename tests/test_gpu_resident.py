@@ -8,6 +8,7 @@ lane, a 32-row group, a 128-row chunk, a reduction group of 64 chunks, one chunk
 per SM and one round of a block's warps.  A wait that runs out is reported and
 leaves the context usable."""
 import ctypes as C
+import itertools
 
 import numpy as np
 import pytest
@@ -84,21 +85,34 @@ def test_resident_nan_and_cap(gpu, monkeypatch):
         assert got[0][2] != 0
 
 
-@pytest.mark.parametrize("eps", [1e-6, 1.1e-15])
-@pytest.mark.parametrize("n", [129, 8193])
-def test_resident_stop_tests(gpu, monkeypatch, n, eps):
-    """The stop decisions, ERR and the last residual state at a loose and at an
-    unreachable tolerance (stagnation, or a residual that ends in zeros)."""
+def test_resident_stop_tests(gpu, monkeypatch):
+    """Every stop decision, with the iteration count, ERR and x it leaves: indefinite
+    and skew systems end by the tolerance, by stagnation, by a vanishing C1 and at the
+    cap (the reference's stop tests, pcgpme_para.F90:215-254), at a loose and at an
+    unreachable tolerance."""
     import torch
-    al, ll, d, b = _system(n, 6, "band")
-    got = []
-    for mode in ("graph", "resident"):
-        _force(monkeypatch, mode)
-        x = torch.zeros(n, dtype=torch.float64, device="cuda")
-        info = gpu.Solver(n).solve(al, ll, d, b, x, eps=eps, itmax=400)
-        got.append((x.cpu().numpy(), info.as_dict()))
-    assert str(got[0][1]) == str(got[1][1])
-    assert np.array_equal(got[0][0], got[1][0], equal_nan=True)
+    reasons = set()
+    for n, skew, diag in itertools.product((40, 129, 500), (False, True), (0.0, 1e-6, 0.1, 1.0)):
+        rng = np.random.default_rng(0)
+        ll = np.zeros((6, n), np.int32)
+        al = np.zeros((6, n))
+        for k, o in enumerate([-1, 1, -5, 5]):
+            j = np.arange(n) + o
+            ok = (j >= 0) & (j < n)
+            ll[k] = np.where(ok, j + 1, 0)
+            al[k] = np.where(ok, (np.sign(o) if skew else 1.0) * rng.uniform(0.5, 1.0), 0.0)
+        t = [torch.from_numpy(v).cuda() for v in (al, ll, np.full(n, diag), rng.standard_normal(n))]
+        for eps in (1e-3, 1.1e-15):
+            got = []
+            for mode in ("graph", "resident"):
+                _force(monkeypatch, mode)
+                x = torch.zeros(n, dtype=torch.float64, device="cuda")
+                info = gpu.Solver(n).solve(*t, x, eps=eps, itmax=1500)
+                got.append((x.cpu().numpy(), str(info.as_dict())))
+            assert got[0][1] == got[1][1]
+            assert np.array_equal(got[0][0], got[1][0], equal_nan=True)
+            reasons.add(info.as_dict()["reason"])
+    assert {"tolerance", "stagnation", "c1_zero"} <= reasons, reasons
 
 
 def test_resident_wait_runs_out_and_context_recovers(gpu, monkeypatch):
