@@ -79,11 +79,7 @@ __global__ void __launch_bounds__(kEngBlock) k_mx_sweep(Eng<T> E, int k, const d
 // Last sweep on FP64 vectors with the squared norm of the result per member
 // (the canonical reduction: warp w takes the tile's chunks w, w + nw, ...).
 //   PHASE 0: BN64 = ||PM W b||^2
-//   PHASE 1: ERR64 = sqrt(||PM r||^2 / BN64); stop the member at the outer
-//            tolerance or sweep cap, else arm its inner solve (mode 1) with
-//            the relative reduction the outer tolerance still needs, halved
-//            for margin, but no tighter than inner_tol: the last sweep then
-//            stops near EPS64 instead of overshooting by up to inner_tol.
+//   PHASE 1: ERR64 and the outer test (mx_outer_test).
 template <typename T, int PHASE>
 __global__ void __launch_bounds__(kEngBlock) k_mx_sweep56(Eng<T> E, const double* __restrict__ in,
                                                          double* __restrict__ out, double inner_tol,
@@ -122,27 +118,7 @@ __global__ void __launch_bounds__(kEngBlock) k_mx_sweep56(Eng<T> E, const double
         if (PHASE == 0) {
             S->BN64 = tot[0];
         } else {
-            const double err = sqrt(tot[0] / S->BN64);
-            S->ERR64 = err;
-            if (!isfinite(err)) {
-                S->odone = 1;
-                stop_member(S, CLOWNS_STOP_NONFINITE, CLOWNS_IER_NONFINITE);
-            } else if (err <= S->EPS64) {
-                S->odone = 1;
-                stop_member(S, CLOWNS_STOP_TOL, 0);
-            } else if (S->outer >= S->OITER) {
-                S->odone = 1;
-                stop_member(S, CLOWNS_STOP_MAXITER, CLOWNS_IER_MAXITER);
-            } else {
-                S->outer += 1;
-                S->SIGMA = sqrt(tot[0]);
-                S->K = 0;
-                S->ERRP = 0.0;
-                S->done = 0;
-                S->mode = 1;
-                S->EPS = fmax(inner_tol, 0.5 * S->EPS64 / err);
-                S->ITER = inner_max;
-            }
+            mx_outer_test(S, tot[0], inner_tol, inner_max);
         }
         __threadfence();
     }
@@ -201,14 +177,9 @@ __global__ void __launch_bounds__(kEngBlock) k_mx_update(Eng<T> E) {
     }
 }
 
-// ctrl[2] accumulates the loop bodies of earlier sweeps; the resident loop's epochs go on.
+// ctrl[2] accumulates the loop bodies of earlier sweeps.
 __global__ void k_mx_reset_ctrl(int* ctrl, int inner_max) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        ctrl[2] += ctrl[0];
-        ctrl[0] = 0;
-        ctrl[1] = inner_max;
-        ctrl[6] = ctrl[7];
-    }
+    if (threadIdx.x == 0 && blockIdx.x == 0) { ctrl[2] += ctrl[0]; ctrl[0] = 0; ctrl[1] = inner_max; }
 }
 
 template <typename T>
@@ -230,7 +201,7 @@ __global__ void k_mixed_init_scalars(MemberScalars* S, int M, double eps, int oi
         z.mode = 1;
         S[m] = z;
     }
-    if (threadIdx.x == 0) { ctrl[0] = 0; ctrl[1] = 0; ctrl[2] = 0; ctrl[6] = 0; ctrl[7] = 0; }
+    if (threadIdx.x == 0) { ctrl[0] = 0; ctrl[1] = 0; ctrl[2] = 0; }
 }
 
 // Export of the scaled/sorted matrix (test hook), member 0 only.
@@ -256,13 +227,22 @@ static inline int member_groups(int n) {
     return (nc + kGroupChunks - 1) / kGroupChunks;
 }
 
-// Single systems up to this many rows run the resident loop, without tuning.
-// Measured against the tuned graph (ms per solve, graph / resident): FP64 2.7 /
-// 0.9 at 4 k rows, 6.8 / 2.4 at 74 k, 10.6 / 5.8 at 239 k, 12.2 / 9.9 at 413 k,
-// 23.6 / 25.5 at 660 k; mixed 3.9 / 1.7, 5.9 / 2.6, 9.1 / 4.5, 11.0 / 7.5, 17.2 /
-// 15.5 and 20.0 / 28.0 at 960 k (its words and matrix no longer fit L2).
+// Systems and ensembles of up to this many rows in all are solved resident, without
+// tuning.  Measured (ms per solve, the tuned graph / resident): single systems FP64
+// 2.7 / 0.8 at 4 k rows, 6.8 / 2.3 at 74 k, 10.6 / 5.6 at 239 k, 12.1 / 9.5 at 413 k,
+// 23.5 / 23.5-31 at 660 k; mixed 3.7 / 1.1, 5.8 / 2.0, 9.1 / 4.0, 11.0 / 7.4, 17.1 / 13.1;
+// ensembles FP64 5.5 / 2.6 at 16 members of 214 k rows, 9.2 / 5.8 at 12 of 407 k, 8.8 /
+// 7.9 at 70 of 552 k, 13.1 / 15.9 at 40 of 1.01 M; mixed 5.7 / 2.1, 7.1 / 4.4, 7.5 / 5.5,
+// 10.7 / 11.8.  Beyond, words, matrix and vectors no longer fit L2.
 constexpr int kResMaxRowsFp64 = 500000;
-constexpr int kResMaxRowsMixed = 700000;
+constexpr int kResMaxRowsMixed = 750000;
+constexpr int kResMaxBlocks = kNumSMs;
+
+static bool res_serves(int M, const int* n, int mixed) {
+    long rows = 0;
+    for (int m = 0; m < M; m++) rows += n[m];
+    return 2 * M <= kResMaxBlocks && rows <= (mixed ? kResMaxRowsMixed : kResMaxRowsFp64);
+}
 
 struct EngLayout {
     long NV = 0;
@@ -272,7 +252,7 @@ struct EngLayout {
     size_t o_in, o_S, o_partials, o_bar, o_al, o_ll, o_d, o_vec[8], o_W, o_x64, o_r64, o_s64, o_t64;
     size_t o_wave, o_wbuf[kWaveBufs];
     int res = 0;           // the resident loop's words and composed coefficients are laid out
-    size_t o_rword[2 + kResSteps], o_rpart, o_rgpart, o_ra, o_rc;
+    size_t o_restab, o_tables, o_rword[1 + kResSteps], o_rword64[1 + kResSteps], o_rpart, o_rgpart, o_ra, o_rc;
     size_t o_baltab = 0;   // ensembles: block tables of the balanced kernels
     size_t o_balg = 0;     // ensembles: blocks of each table's launch
     size_t total = 0;
@@ -307,12 +287,14 @@ static EngLayout eng_layout(int M, const int* n, int mixed, int wave = -1) {
     L.o_mem_grp0 = take(sizeof(int) * M);
     L.o_mem_ngrp = take(sizeof(int) * M);
     L.o_gticket = take(sizeof(unsigned) * ngrp);
-    L.o_gpartials = take(sizeof(double) * 2 * ngrp);
-    L.o_ctrl = take(sizeof(int) * 8);
     L.o_in = take(sizeof(MemberIn) * M);
+    L.o_ctrl = take(sizeof(int) * 8);          // results: read back in one copy
     L.o_S = take(sizeof(MemberScalars) * M);
-    L.o_partials = take(sizeof(double) * 2 * (NV / kChunk));
     L.o_bar = take(sizeof(GridBar));
+    L.o_restab = take(sizeof(BalBlock) * (M > 1 ? kResMaxBlocks : 0));
+    L.o_tables = o;                            // uploaded up to here (the resident path) or up to o_ctrl
+    L.o_gpartials = take(sizeof(double) * 2 * ngrp);
+    L.o_partials = take(sizeof(double) * 2 * (NV / kChunk));
     L.o_al = take((size_t)L.tsize * 6 * NV);
     L.o_ll = take(sizeof(int) * 6 * NV);
     L.o_d = take((size_t)L.tsize * NV);
@@ -334,11 +316,13 @@ static EngLayout eng_layout(int M, const int* n, int mixed, int wave = -1) {
         L.o_wave = 0;
         for (int k = 0; k < kWaveBufs; k++) L.o_wbuf[k] = 0;
     }
-    L.res = wave < 0 && M == 1 && n[0] <= (mixed ? kResMaxRowsMixed : kResMaxRowsFp64);
+    L.res = wave < 0 && res_serves(M, n, mixed);
     if (L.res) {
-        for (int k = 0; k < 2 + kResSteps; k++) L.o_rword[k] = take(2 * (size_t)L.tsize * NV);
-        L.o_rpart = take(sizeof(TagWord<double>) * 6 * (size_t)(NV / kChunk));
-        L.o_rgpart = take(sizeof(TagWord<double>) * 6 * (size_t)ngrp);
+        for (int k = 0; k < 1 + kResSteps; k++) L.o_rword[k] = take(2 * (size_t)L.tsize * NV);
+        if (mixed)
+            for (int k = 0; k < 1 + kResSteps; k++) L.o_rword64[k] = take(sizeof(TagWord<double>) * (size_t)NV);
+        L.o_rpart = take(sizeof(TagWord<double>) * 2 * kResReds * (size_t)(NV / kChunk));
+        L.o_rgpart = take(sizeof(TagWord<double>) * 2 * kResReds * (size_t)ngrp);
         L.o_ra = take((size_t)L.tsize * kResCoef<6> * NV);
         L.o_rc = take(sizeof(int) * kResIdx<6> * (size_t)NV);
     }
@@ -430,9 +414,13 @@ static ResBufs<T> res_bind(void* work, const EngLayout& L) {
     ResBufs<T> R = {};
     if (!L.res) return R;
     char* b = (char*)work;
-    R.p = (TagWord<T>*)(b + L.o_rword[0]);
-    R.e = (TagWord<T>*)(b + L.o_rword[1]);
-    for (int k = 0; k < kResSteps; k++) R.t[k] = (TagWord<T>*)(b + L.o_rword[2 + k]);
+    R.in = (TagWord<T>*)(b + L.o_rword[0]);
+    for (int k = 0; k < kResSteps; k++) R.t[k] = (TagWord<T>*)(b + L.o_rword[1 + k]);
+    if (L.mixed) {
+        R.x64 = (TagWord<double>*)(b + L.o_rword64[0]);
+        for (int k = 0; k < kResSteps; k++) R.t64[k] = (TagWord<double>*)(b + L.o_rword64[1 + k]);
+    }
+    R.tab = L.M > 1 ? (const BalBlock*)(b + L.o_restab) : nullptr;
     R.part = (TagWord<double>*)(b + L.o_rpart);
     R.gpart = (TagWord<double>*)(b + L.o_rgpart);
     R.ngrp = L.ngrp;
@@ -452,40 +440,36 @@ static void fill_groups(int M, const int* n, int* mem_grp0, int* mem_ngrp) {
     }
 }
 
-// Upload the member tables (static for a given layout) and the input table.
-static int eng_upload_tables(void* work, const EngLayout& L, const int* n, const MemberIn* ins,
-                             cudaStream_t s) {
+// The member tables (static for a given layout) and the input table, as they lie at
+// the workspace's start.
+static std::vector<char> eng_tables(const EngLayout& L, const int* n, const MemberIn* ins) {
     const int M = L.M;
-    std::vector<int> blk_member(L.nblk, -1), blk_rows(L.nblk, 0), off(M), nn(M), nblk(M), blk0(M);
+    std::vector<char> t(L.o_tables, 0);
+    auto at = [&](size_t o) { return (int*)(t.data() + o); };
+    int *blk_member = at(L.o_blk_member), *blk_rows = at(L.o_blk_rows);
+    std::fill(blk_member, blk_member + L.nblk, -1);
     long o = 0;
     for (int m = 0; m < M; m++) {
-        off[m] = (int)o;
-        nn[m] = n[m];
-        blk0[m] = (int)(o / kTile);
-        nblk[m] = (n[m] + kTile - 1) / kTile;
+        at(L.o_mem_off)[m] = (int)o;
+        at(L.o_mem_n)[m] = n[m];
+        at(L.o_mem_blk0)[m] = (int)(o / kTile);
+        at(L.o_mem_nblk)[m] = (n[m] + kTile - 1) / kTile;
         const long R = (long)align_up((size_t)n[m] + 1, kTile);
         for (long b = o / kTile; b < (o + R) / kTile; b++) {
             blk_member[b] = m;
-            long rows = n[m] - (b * kTile - o);
-            blk_rows[b] = (int)std::max(0L, std::min((long)kTile, rows));
+            blk_rows[b] = (int)std::max(0L, std::min((long)kTile, n[m] - (b * kTile - o)));
         }
         o += R;
     }
-    std::vector<int> mem_grp0(M), mem_ngrp(M);
-    fill_groups(M, n, mem_grp0.data(), mem_ngrp.data());
-    std::vector<unsigned> zeros(std::max(M, L.ngrp), 0u);
-    char* b = (char*)work;
-    CLOWNS_CUDA_TRY(cudaMemcpyAsync(b + L.o_blk_member, blk_member.data(), sizeof(int) * L.nblk, cudaMemcpyHostToDevice, s));
-    CLOWNS_CUDA_TRY(cudaMemcpyAsync(b + L.o_blk_rows, blk_rows.data(), sizeof(int) * L.nblk, cudaMemcpyHostToDevice, s));
-    CLOWNS_CUDA_TRY(cudaMemcpyAsync(b + L.o_mem_off, off.data(), sizeof(int) * M, cudaMemcpyHostToDevice, s));
-    CLOWNS_CUDA_TRY(cudaMemcpyAsync(b + L.o_mem_n, nn.data(), sizeof(int) * M, cudaMemcpyHostToDevice, s));
-    CLOWNS_CUDA_TRY(cudaMemcpyAsync(b + L.o_mem_nblk, nblk.data(), sizeof(int) * M, cudaMemcpyHostToDevice, s));
-    CLOWNS_CUDA_TRY(cudaMemcpyAsync(b + L.o_mem_blk0, blk0.data(), sizeof(int) * M, cudaMemcpyHostToDevice, s));
-    CLOWNS_CUDA_TRY(cudaMemcpyAsync(b + L.o_ticket, zeros.data(), sizeof(unsigned) * M, cudaMemcpyHostToDevice, s));
-    CLOWNS_CUDA_TRY(cudaMemcpyAsync(b + L.o_mem_grp0, mem_grp0.data(), sizeof(int) * M, cudaMemcpyHostToDevice, s));
-    CLOWNS_CUDA_TRY(cudaMemcpyAsync(b + L.o_mem_ngrp, mem_ngrp.data(), sizeof(int) * M, cudaMemcpyHostToDevice, s));
-    CLOWNS_CUDA_TRY(cudaMemcpyAsync(b + L.o_gticket, zeros.data(), sizeof(unsigned) * L.ngrp, cudaMemcpyHostToDevice, s));
-    CLOWNS_CUDA_TRY(cudaMemcpyAsync(b + L.o_in, ins, sizeof(MemberIn) * M, cudaMemcpyHostToDevice, s));
+    fill_groups(M, n, at(L.o_mem_grp0), at(L.o_mem_ngrp));
+    memcpy(t.data() + L.o_in, ins, sizeof(MemberIn) * M);
+    return t;
+}
+
+static int eng_upload_tables(void* work, const EngLayout& L, const int* n, const MemberIn* ins,
+                             cudaStream_t s) {
+    const std::vector<char> t = eng_tables(L, n, ins);
+    CLOWNS_CUDA_TRY(cudaMemcpyAsync(work, t.data(), L.o_ctrl, cudaMemcpyHostToDevice, s));
     CLOWNS_CUDA_TRY(cudaStreamSynchronize(s));
     return CLOWNS_OK;
 }
@@ -547,7 +531,7 @@ static void launch_ldusub64(const Eng<T>& E, const Shape& sh, double inner_tol, 
 }
 
 // ---------------------------------------------------------------------------
-// The iteration loop.  Single systems of small and medium size run it resident
+// The iteration loop.  Systems and ensembles of small and medium size are solved resident
 // (one kernel, resident.cuh; by rule, see kResMaxRowsFp64); for the others the
 // autotuner times three executions on the actual row space and keeps the fastest:
 //   graph:      a CUDA graph whose WHILE node repeats the iteration's kernels,
@@ -613,24 +597,42 @@ static int device_sms() {
     return sms;
 }
 
-// Launch shape of the resident loop for a single system: at most one block per
-// SM, each with the warps its 32-row quarters of chunks fill, or the fewest
-// rounds of at most kResWarps that cover them.
-static LoopShape res_shape(int n) {
-    const int nc = (n + kChunk - 1) / kChunk;
+// Launch shape of the resident solve: at most one block per SM, dealt to the members
+// in proportion to their chunks (each block takes its member's next even share), with
+// the warps that a block's 32-row groups fill, or the fewest rounds of at most
+// kResWarps that cover them, and the scalar warp.
+static LoopShape res_shape(int M, const int* n, BalBlock* tab) {
+    std::vector<int> nc(M), g(M);
+    long total = 0;
+    for (int m = 0; m < M; m++) total += nc[m] = (n[m] + kChunk - 1) / kChunk;
+    const int G = (int)std::min<long>(total, std::min(device_sms(), kResMaxBlocks));
+    int used = 0;
+    for (int m = 0; m < M; m++) used += g[m] = (int)std::max<long>(1, std::min<long>(nc[m], (long)G * nc[m] / total));
+    // the largest share per block gets the next block; a surplus comes from the smallest
+    for (; used < G; used++) {
+        int best = -1;
+        for (int m = 0; m < M; m++)
+            if (g[m] < nc[m] && (best < 0 || (long)nc[m] * g[best] > (long)nc[best] * g[m])) best = m;
+        if (best < 0) break;
+        g[best]++;
+    }
+    for (; used > G; used--) {
+        int best = -1;
+        for (int m = 0; m < M; m++)
+            if (g[m] > 1 && (best < 0 || (long)nc[m] * g[best] < (long)nc[best] * g[m])) best = m;
+        g[best]--;
+    }
     LoopShape sh;
     sh.graph = 4;
-    sh.grid = std::min(nc, device_sms());
-    const int per = (nc + sh.grid - 1) / sh.grid, most = kResWarps / kChunkRows;
-    const int rounds = (per + most - 1) / most;
-    sh.block = kChunk * ((per + rounds - 1) / rounds) + 32;     // and the scalar warp
+    sh.grid = used;
+    int per = 0, b = 0;
+    for (int m = 0; m < M; m++) {
+        per = std::max(per, (nc[m] + g[m] - 1) / g[m]);
+        for (int j = 0; tab && j < g[m]; j++, b++) tab[b] = BalBlock{m, j, g[m], b - j};
+    }
+    const int most = kResWarps / kChunkRows, rounds = (per + most - 1) / most;
+    sh.block = kChunk * ((per + rounds - 1) / rounds) + 32;
     return sh;
-}
-
-template <typename T>
-static void res_compose(const Eng<T>& E, const ResBufs<T>& R, int grid, cudaStream_t s) {
-    if (E.nl == 4) k_res_compose<T, 4><<<grid, kEngBlock, 0, s>>>(E, R);
-    else k_res_compose<T, 6><<<grid, kEngBlock, 0, s>>>(E, R);
 }
 
 static std::mutex g_loop_mu;
@@ -1009,21 +1011,9 @@ static void wait_params(bool take, long* limit, int* absent) {
 // take_fault: this run is a solve's (not a tuning trial's), so an armed wait
 // fault applies to it.
 template <typename T>
-static int run_loop(Eng<T> E, const ResBufs<T>& R, const void* work, GridBar* gb, int prec, const LoopShape& sh,
-                    cudaStream_t s, bool take_fault = false) {
+static int run_loop(Eng<T> E, const void* work, GridBar* gb, int prec, const LoopShape& sh, cudaStream_t s,
+                    bool take_fault = false) {
     TraceRange trace_range_("iteration loop");
-    if (sh.graph == 4) {
-        CLOWNS_CUDA_TRY(cudaMemsetAsync(gb, 0, sizeof(GridBar), s));
-        ResBufs<T> r = R;
-        long lim;
-        int absent;
-        wait_params(take_fault, &lim, &absent);
-        void* args[] = {(void*)&E, (void*)&r, (void*)&lim, (void*)&absent};
-        const void* fn = E.nl == 4 ? (const void*)k_res_loop<T, 4> : (const void*)k_res_loop<T, 6>;
-        CLOWNS_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(sh.grid), dim3(sh.block), args, 0, s));
-        t_launches += 1;
-        return CLOWNS_OK;
-    }
     if (sh.bal && E.M > 1 && E.baltab && (sh.graph == 1 || sh.graph == 2)) {
         // ensembles on the balanced kernels: block tables over the members that iterate
         k_bal_rebuild<<<1, kBalScanThreads, 0, s>>>(E.S, E.M, E.mem_n, (BalBlock*)E.baltab, E.balg, E.ctrl + 4);
@@ -1095,15 +1085,17 @@ static int run_loop(Eng<T> E, const ResBufs<T>& R, const void* work, GridBar* gb
     return CLOWNS_OK;
 }
 
+static int abort_status(int abort) {
+    if (!abort) return CLOWNS_OK;
+    set_last_error_msg("pcgpme: a bounded device wait (grid barrier, staged copy or published row) timed out; the solve was abandoned");
+    return CLOWNS_ERR_NOCONV;
+}
+
 static int check_abort(GridBar* gb, cudaStream_t s) {
     int abort = 0;
     CLOWNS_CUDA_TRY(cudaMemcpyAsync(&abort, &gb->abort, sizeof(int), cudaMemcpyDeviceToHost, s));
     CLOWNS_CUDA_TRY(cudaStreamSynchronize(s));
-    if (abort) {
-        set_last_error_msg("pcgpme: a bounded device wait (grid barrier or staged copy) timed out; the solve was abandoned");
-        return CLOWNS_ERR_NOCONV;
-    }
-    return CLOWNS_OK;
+    return abort_status(abort);
 }
 
 // Autotuner: time kTuneIters iterations of the loop for each candidate -- the
@@ -1115,8 +1107,8 @@ static int check_abort(GridBar* gb, cudaStream_t s) {
 // `prime` re-creates the state the loop starts from.
 constexpr int kTuneIters = 24;
 template <typename T, typename Prime>
-static int tune_loop(Eng<T> E, const ResBufs<T>& R, const void* work, GridBar* gb, long key_nv, int key_prec,
-                     Prime prime, cudaStream_t s, LoopShape* out) {
+static int tune_loop(Eng<T> E, const void* work, GridBar* gb, long key_nv, int key_prec, Prime prime,
+                     cudaStream_t s, LoopShape* out) {
     TraceRange trace_range_("loop autotuner");
     const int forced = forced_loop_mode();
     const bool wave_ok = E.wave != nullptr && E.M == 1;
@@ -1135,12 +1127,6 @@ static int tune_loop(Eng<T> E, const ResBufs<T>& R, const void* work, GridBar* g
         return CLOWNS_OK;
     }
     const auto key = std::make_tuple(key_nv, key_prec, (int)wave_ok, forced);
-    if (R.p && (forced == 4 || forced < 0)) {             // by rule: nothing to time
-        *out = res_shape(E.n1);
-        std::lock_guard<std::mutex> lk(g_loop_mu);
-        g_loop_shapes[key] = *out;                        // for clowns_tuned_shape only
-        return CLOWNS_OK;
-    }
     // CLOWNS_WAVE_PARAMS="K,slack,minb,frac" pins the wavefront candidate (tuning sweeps; read on every call)
     const char* wp = getenv("CLOWNS_WAVE_PARAMS");
     int pk = 0, ps = 0, pm = 0, pf = 0;
@@ -1251,7 +1237,7 @@ static int tune_loop(Eng<T> E, const ResBufs<T>& R, const void* work, GridBar* g
             if (failed[c]) continue;
             prime(s);
             CLOWNS_CUDA_TRY(cudaEventRecord(e0, s));
-            if (run_loop(E, R, work, gb, key_prec, cands[c], s)) {
+            if (run_loop(E, work, gb, key_prec, cands[c], s)) {
                 cudaGetLastError();
                 failed[c] = 1;
                 continue;
@@ -1322,16 +1308,16 @@ static void params(int n, double eps, double parm, int iter, double* eps_o, int*
     *P2 = p1 + 1.0;
 }
 
-// Per-member results; also adds the kernel nodes executed by loop graphs
-// (16 per body, ctrl[0] + ctrl[2] bodies) to the launch count.
-static int read_infos(void* work, const EngLayout& L, cudaStream_t s, clowns_solve_info* info, int mixed,
-                      const LoopShape& sh) {
-    std::vector<MemberScalars> h(L.M);
-    int ctrl[8];
-    CLOWNS_CUDA_TRY(cudaMemcpyAsync(h.data(), (char*)work + L.o_S, sizeof(MemberScalars) * L.M,
-                                    cudaMemcpyDeviceToHost, s));
-    CLOWNS_CUDA_TRY(cudaMemcpyAsync(ctrl, (char*)work + L.o_ctrl, sizeof(ctrl), cudaMemcpyDeviceToHost, s));
+// The abort flag and the per-member results in one copy; also adds the kernel nodes
+// executed by loop graphs (16 per body, ctrl[0] + ctrl[2] bodies) to the launch count.
+static int read_results(void* work, const EngLayout& L, cudaStream_t s, clowns_solve_info* info, int mixed,
+                        const LoopShape& sh) {
+    std::vector<char> t(L.o_bar + sizeof(GridBar) - L.o_ctrl);
+    CLOWNS_CUDA_TRY(cudaMemcpyAsync(t.data(), (char*)work + L.o_ctrl, t.size(), cudaMemcpyDeviceToHost, s));
     CLOWNS_CUDA_TRY(cudaStreamSynchronize(s));
+    const int* ctrl = (const int*)t.data();
+    const MemberScalars* h = (const MemberScalars*)(t.data() + (L.o_S - L.o_ctrl));
+    if (int rc = abort_status(((const GridBar*)(t.data() + (L.o_bar - L.o_ctrl)))->abort)) return rc;
     if (sh.graph == 1) t_launches += loop_launches(sh, (long)ctrl[0] + ctrl[2]);
     if (!info) return CLOWNS_OK;
     for (int m = 0; m < L.M; m++) {
@@ -1375,6 +1361,56 @@ static int check_members(int M, const MemberIn* ins, std::vector<int>& n, int* n
     return CLOWNS_OK;
 }
 
+// Whether a solve runs resident: by rule, unless another execution is forced.
+static bool res_chosen(const EngLayout& L) {
+    const int forced = forced_loop_mode();
+    return L.res && (forced < 0 || forced == 4);
+}
+
+// A solve in three kernels -- setup, composed coefficients, and the whole of the rest
+// resident -- between one upload (tables, inputs, initial scalars, a cleared abort
+// flag) and one read-back (scalars and abort flag).
+template <typename T>
+static int solve_resident(const EngLayout& L, const int* n, const MemberIn* ins, const MemberScalars& init, int nl,
+                          double P1, double P2, double inner_tol, int inner_max, void* work, cudaStream_t s,
+                          clowns_solve_info* info) {
+    constexpr bool mixed = std::is_same<T, float>::value;
+    std::vector<char> t = eng_tables(L, n, ins);
+    for (int m = 0; m < L.M; m++) ((MemberScalars*)(t.data() + L.o_S))[m] = init;
+    const LoopShape sh = res_shape(L.M, n, L.M > 1 ? (BalBlock*)(t.data() + L.o_restab) : nullptr);
+    CLOWNS_CUDA_TRY(cudaMemcpyAsync(work, t.data(), L.o_tables, cudaMemcpyHostToDevice, s));
+    Eng<T> E = eng_bind<T>(work, L);
+    E.nl = nl;
+    E.wave = nullptr;
+    ResBufs<T> R = res_bind<T>(work, L);
+    const int gs = std::min(L.nblk * 2, kEngMaxGrid * 4);
+    if (nl == 6) {
+        k_eng_setup<T, 6><<<gs, kEngBlock, 0, s>>>(E, P1, P2, mixed);
+        k_res_compose<T, 6><<<gs, kEngBlock, 0, s>>>(E, R);
+    } else {
+        k_eng_setup<T, 4><<<gs, kEngBlock, 0, s>>>(E, P1, P2, mixed);
+        k_res_compose<T, 4><<<gs, kEngBlock, 0, s>>>(E, R);
+    }
+    long lim;
+    int absent;
+    wait_params(!mixed, &lim, &absent);
+    if constexpr (mixed) {
+        void* args[] = {(void*)&E, (void*)&R, (void*)&inner_tol, (void*)&inner_max, (void*)&lim, (void*)&absent};
+        const void* fn = nl == 4 ? (const void*)k_res_mixed<4> : (const void*)k_res_mixed<6>;
+        CLOWNS_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(sh.grid), dim3(sh.block), args, 0, s));
+    } else {
+        void* args[] = {(void*)&E, (void*)&R, (void*)&lim, (void*)&absent};
+        const void* fn = nl == 4 ? (const void*)k_res_plain<4> : (const void*)k_res_plain<6>;
+        CLOWNS_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(sh.grid), dim3(sh.block), args, 0, s));
+    }
+    t_launches = 3;
+    {
+        std::lock_guard<std::mutex> lk(g_loop_mu);            // for clowns_tuned_shape
+        g_loop_shapes[std::make_tuple(L.NV, (int)mixed, (int)(L.M == 1), forced_loop_mode())] = sh;
+    }
+    return read_results(work, L, s, info, mixed, sh);
+}
+
 // Plain FP64 (reference method and stop tests) over M members: setup kernel,
 // one persistent launch for PCGPME's start and its whole iteration loop, copy-out.
 int engine_solve_plain(int M, const MemberIn* ins, double eps, double parm, int iter, void* work,
@@ -1401,11 +1437,17 @@ int engine_solve_plain(int M, const MemberIn* ins, double eps, double parm, int 
         eps_r = eps;
         iter_r = iter;
     }
+    if (res_chosen(L)) {
+        MemberScalars init = {};
+        init.EPS = eps_r;
+        init.ITER = iter_r;
+        init.mode = mode;
+        return solve_resident<double>(L, n.data(), ins, init, nl, P1, P2, 0.0, 0, work, s, info);
+    }
     rc = eng_upload_tables(work, L, n.data(), ins, s);
     if (rc) return rc;
     Eng<double> E = eng_bind<double>(work, L);
     E.nl = nl;
-    const ResBufs<double> R = res_bind<double>(work, L);
     bool bal_ok = false;
     rc = upload_bal_tables<double>(work, L, s, &bal_ok);
     if (rc) return rc;
@@ -1417,7 +1459,6 @@ int engine_solve_plain(int M, const MemberIn* ins, double eps, double parm, int 
         k_eng_init_scalars<<<1, 256, 0, cs>>>(E.S, M, e, it, mode, E.ctrl);
         if (nl == 6) k_eng_setup<double, 6><<<gs, kEngBlock, 0, cs>>>(E, P1, P2, 0);
         else k_eng_setup<double, 4><<<gs, kEngBlock, 0, cs>>>(E, P1, P2, 0);
-        if (R.p) res_compose(E, R, gs, cs);
     };
     // PCGPME's start (b^ = PM W b, q = PM A x0, residuals) as plain launches
     const Shape ksh;
@@ -1428,21 +1469,19 @@ int engine_solve_plain(int M, const MemberIn* ins, double eps, double parm, int 
     };
     LoopShape sh;
     // tuning runs: kTuneIters iterations from the real start (not counted as the solve's launches)
-    rc = tune_loop(E, R, work, gb, L.NV, 0, [&](cudaStream_t cs) { prime(cs, 1e-300, kTuneIters); start(cs); }, s, &sh);
+    rc = tune_loop(E, work, gb, L.NV, 0, [&](cudaStream_t cs) { prime(cs, 1e-300, kTuneIters); start(cs); }, s, &sh);
     if (rc) return rc;
     t_launches = 0;
     prime(s, eps_r, iter_r);
     start(s);
     t_launches += 2 + 8;
     CLOWNS_CUDA_TRY(cudaGetLastError());
-    rc = run_loop(E, R, work, gb, 0, sh, s, true);
+    rc = run_loop(E, work, gb, 0, sh, s, true);
     if (rc) return rc;
     k_eng_copy_out<double><<<gs, kEngBlock, 0, s>>>(E);
     t_launches += 1;
     CLOWNS_CUDA_TRY(cudaGetLastError());
-    rc = check_abort(gb, s);
-    if (rc) return rc;
-    return read_infos(work, L, s, info, 0, sh);
+    return read_results(work, L, s, info, 0, sh);
 }
 
 // Default relative reduction per inner solve.  Short FP32 inner solves
@@ -1473,11 +1512,17 @@ int engine_solve_mixed(int M, const MemberIn* ins, double eps, double parm, doub
     if (inner_tol <= 0) inner_tol = kInnerTol;
     if (inner_max <= 0) inner_max = 2000;
     if (max_outer <= 0) max_outer = 30;
+    if (res_chosen(L)) {
+        MemberScalars init = {};
+        init.EPS64 = eps_r;
+        init.OITER = max_outer;
+        init.mode = 1;
+        return solve_resident<float>(L, n.data(), ins, init, nl, P1, P2, inner_tol, inner_max, work, s, info);
+    }
     rc = eng_upload_tables(work, L, n.data(), ins, s);
     if (rc) return rc;
     Eng<float> E = eng_bind<float>(work, L);
     E.nl = nl;
-    const ResBufs<float> R = res_bind<float>(work, L);
     bool bal_ok = false;
     rc = upload_bal_tables<float>(work, L, s, &bal_ok);
     if (rc) return rc;
@@ -1491,7 +1536,6 @@ int engine_solve_mixed(int M, const MemberIn* ins, double eps, double parm, doub
         k_mixed_init_scalars<<<1, 256, 0, cs>>>(E.S, M, eps_r, max_outer, E.ctrl);
         if (nl == 6) k_eng_setup<float, 6><<<gs, kEngBlock, 0, cs>>>(E, P1, P2, 1);
         else k_eng_setup<float, 4><<<gs, kEngBlock, 0, cs>>>(E, P1, P2, 1);
-        if (R.p) res_compose(E, R, gs, cs);
         launch_ldusub64<float, 0>(E, ksh, inner_tol, inner_max, cs);   // BN64 = ||PM W b||^2
     };
     // one refinement sweep up to the inner loop: residual, PM r, ERR test, inner RHS
@@ -1502,7 +1546,7 @@ int engine_solve_mixed(int M, const MemberIn* ins, double eps, double parm, doub
         k_mx_normalize<float><<<kg, ksh.block, 0, cs>>>(E);
     };
     LoopShape sh;
-    rc = tune_loop(E, R, work, gb, L.NV, 1, [&](cudaStream_t cs) { setup(cs); sweep_head(cs, 1e-30, kTuneIters); },
+    rc = tune_loop(E, work, gb, L.NV, 1, [&](cudaStream_t cs) { setup(cs); sweep_head(cs, 1e-30, kTuneIters); },
                    s, &sh);
     if (rc) return rc;
     t_launches = 0;
@@ -1519,7 +1563,7 @@ int engine_solve_mixed(int M, const MemberIn* ins, double eps, double parm, doub
         bool all = true;
         for (int m = 0; m < M; m++) all = all && h[m].odone;
         if (all) break;
-        rc = run_loop(E, R, work, gb, 1, sh, s);
+        rc = run_loop(E, work, gb, 1, sh, s);
         if (rc) return rc;
         k_mx_update<float><<<kg, ksh.block, 0, s>>>(E);
         t_launches += 1;
@@ -1530,7 +1574,7 @@ int engine_solve_mixed(int M, const MemberIn* ins, double eps, double parm, doub
     k_mx_copy_out<float><<<gs, kEngBlock, 0, s>>>(E);
     t_launches += 1;
     CLOWNS_CUDA_TRY(cudaGetLastError());
-    return read_infos(work, L, s, info, 1, sh);
+    return read_results(work, L, s, info, 1, sh);
 }
 
 // Test hooks -------------------------------------------------------------------

@@ -130,8 +130,7 @@ struct Eng {
     MemberScalars* S;
     double* partials;         // 2 per chunk of the row space (chunk totals)
     unsigned* ticket;         // groups summed, one per member
-    int* ctrl;                // [0] loop-body count, [1] max ITER over members, [2] bodies of earlier sweeps,
-                              // [6] first epoch of the next resident loop, [7] epochs used so far
+    int* ctrl;                // [0] loop-body count, [1] max ITER over members, [2] bodies of earlier sweeps
     const BalBlock* baltab;   // ensembles: 16 block tables of the balanced kernels (nullptr: none)
     const int* balg;          // ensembles: the blocks of each table's launch (16)
     int nl;                   // columns the members' matrices fill: 6 (3D) or 4 (2DV, and the 2DH
@@ -420,6 +419,35 @@ __device__ __forceinline__ void finish_xrupdate(MemberScalars* S, const double (
     }
 }
 
+// Outer test of the mixed path, by one thread: ERR64 = sqrt(||PM r||^2 / BN64); stop
+// the member at the outer tolerance or sweep cap, else arm its inner solve (mode 1)
+// with the relative reduction the outer tolerance still needs, halved for margin, but
+// no tighter than inner_tol: the last sweep then stops near EPS64 instead of
+// overshooting by up to inner_tol.
+__device__ __forceinline__ void mx_outer_test(MemberScalars* S, double rr, double inner_tol, int inner_max) {
+    const double err = sqrt(rr / S->BN64);
+    S->ERR64 = err;
+    if (!isfinite(err)) {
+        S->odone = 1;
+        stop_member(S, CLOWNS_STOP_NONFINITE, CLOWNS_IER_NONFINITE);
+    } else if (err <= S->EPS64) {
+        S->odone = 1;
+        stop_member(S, CLOWNS_STOP_TOL, 0);
+    } else if (S->outer >= S->OITER) {
+        S->odone = 1;
+        stop_member(S, CLOWNS_STOP_MAXITER, CLOWNS_IER_MAXITER);
+    } else {
+        S->outer += 1;
+        S->SIGMA = sqrt(rr);
+        S->K = 0;
+        S->ERRP = 0.0;
+        S->done = 0;
+        S->mode = 1;
+        S->EPS = fmax(inner_tol, 0.5 * S->EPS64 / err);
+        S->ITER = inner_max;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Setup: scaling W = P2/(max(sum|AL|,D)+P1 D), scaled copies and the per-row
 // exchange sort (pcgpme_para.F90:77-112).  Explicitly rounded arithmetic so the
@@ -528,7 +556,7 @@ static __global__ void k_eng_init_scalars(MemberScalars* S, int M, double eps, i
         z.mode = mode;
         S[m] = z;
     }
-    if (threadIdx.x == 0) { ctrl[0] = 0; ctrl[1] = iter; ctrl[2] = 0; ctrl[6] = 0; ctrl[7] = 0; }
+    if (threadIdx.x == 0) { ctrl[0] = 0; ctrl[1] = iter; ctrl[2] = 0; }
 }
 
 // ---------------------------------------------------------------------------

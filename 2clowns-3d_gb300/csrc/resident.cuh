@@ -1,4 +1,4 @@
-// resident.cuh -- the iteration loop of small and medium systems as ONE resident
+// resident.cuh -- solves of small and medium systems and ensembles as ONE resident
 // kernel whose blocks exchange vectors through self-validating words.
 //
 // Below about half a million rows an iteration of the kernel-per-phase loop is
@@ -37,7 +37,7 @@
 // A word is overwritten only after a reduction of the same iteration that every
 // reader's own contribution had to precede, so no reader can miss its epoch:
 // the operator's intermediates (a vector of its own for each step) are rewritten
-// once per reduction RQ / AMU, p and e once per iteration, and each of the three reductions has its own totals.
+// once per reduction RQ / AMU, the word of p and e likewise, and each of the three reductions has its own totals.
 // Every poll is bounded: a warp that runs out raises the abort flag, polls of
 // the other warps and blocks then give up too, and the block leaves at the next
 // reduction; the host reports the failure.
@@ -51,6 +51,8 @@ namespace clowns {
 
 constexpr int kResWarps = 28;                    // row warps of a block at most
 constexpr int kResThreads = 32 * kResWarps + 32; // and the scalar warp: 64 registers per thread
+constexpr int kResReds = 5;                      // RQ, AMU, RN, and two of the mixed path's refinement: a
+                                                 // reduction's words are written again only after another one
 constexpr int kResSteps = 3;                     // vectors between the operator's steps (NL / 2 of them used)
 
 // Coefficients and indices of one 32-row group in the resident loop's layout:
@@ -106,9 +108,10 @@ __device__ __forceinline__ unsigned tag_get(const TagWord<float>* p, float& v) {
 // Words and composed coefficients of the resident loop (pointers into the workspace).
 template <typename T>
 struct ResBufs {
-    TagWord<T> *p, *e, *t[kResSteps];   // NV words each
-    TagWord<double>* part;           // 3 reductions x 2 values x (NV / kChunk) chunk totals
-    TagWord<double>* gpart;          // 3 reductions x 2 values x ngrp group totals
+    TagWord<T> *in, *t[kResSteps];   // p or e, and the operator's intermediates: NV words each
+    TagWord<double> *x64, *t64[kResSteps];   // mixed path: the solution, PM's intermediates
+    TagWord<double>* part;           // kResReds reductions x 2 values x (NV / kChunk) chunk totals
+    TagWord<double>* gpart;          // kResReds reductions x 2 values x ngrp group totals
     int ngrp;                        // groups of all members
     T* a;                            // coefficients, kResCoef x 32 per 32-row group
     int* c;                          // indices, kResIdx x 32 per 32-row group
@@ -122,15 +125,19 @@ __global__ void __launch_bounds__(kEngBlock) k_res_compose(Eng<T> E, ResBufs<T> 
     const long NV = E.NV;
     const long stride = (long)gridDim.x * blockDim.x, t0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
     constexpr int NI = kResIdx<NL>;
-    for (long i = t0; i < 6 * (NV / kChunk); i += stride) R.part[i].tag = 0;
-    for (long i = t0; i < 6 * R.ngrp; i += stride) R.gpart[i].tag = 0;
+    for (long i = t0; i < 2 * kResReds * (NV / kChunk); i += stride) R.part[i].tag = 0;
+    for (long i = t0; i < 2 * kResReds * R.ngrp; i += stride) R.gpart[i].tag = 0;
     for (long i = t0; i < NV; i += stride) {
         const int m = E.blk_member[i / kTile];
         if (m < 0) continue;
-        R.p[i].tag = 0;
-        R.e[i].tag = 0;
+        R.in[i].tag = 0;
 #pragma unroll
         for (int k = 0; k < NL / 2; k++) R.t[k][i].tag = 0;
+        if (std::is_same<T, float>::value) {
+            R.x64[i].tag = 0;
+#pragma unroll
+            for (int k = 0; k < NL / 2; k++) R.t64[k][i].tag = 0;
+        }
         T* a = R.a + (i >> 5) * (32 * (NI + 1)) + (i & 31);
         int* c = R.c + (i >> 5) * (32 * NI) + (i & 31);
         auto put = [&](int slot, int sweep, long j) {
@@ -200,6 +207,7 @@ __device__ __forceinline__ bool f64_finite(double x) { return (__double2hiint(x)
 // finish_xrupdate does; at the loop's end ERR is formed from RN in any case.
 struct ResStop {
     double invbn, eps2, q, rn_prev;
+    int tests;           // stop tests taken
 };
 __device__ __noinline__ void res_stop_exact(MemberScalars* S, double RN, double rn_prev) {
     const double ERR = sqrt(RN / S->BN);                         // 215
@@ -220,6 +228,7 @@ __device__ __forceinline__ void res_stop_tests(MemberScalars* S, ResStop& st, do
     S->C1 = C1;
     S->K = K;
     S->total_iter += 1;
+    st.tests++;
     if (!f64_finite(RN) || !f64_finite(C1)) {
         S->ERR = sqrt(RN / S->BN);
         stop_member(S, CLOWNS_STOP_NONFINITE, S->mode != 1 ? CLOWNS_IER_NONFINITE : 0);
@@ -249,11 +258,10 @@ __device__ __forceinline__ void res_stop_tests(MemberScalars* S, ResStop& st, do
     }
 }
 
-// Shared state of one block of the resident loop.
-template <typename T>
+// Shared state of one block.
 struct ResShared {
     MemberScalars s;
-    T y[kResWarps][32], u[kResWarps][32];
+    double y[kResWarps * 32], u[kResWarps * 32];   // rows of the round a reduction folds
     double beta;         // of the iteration that starts (its stop tests may still run)
     ResStop st;
     int fail;            // a poll ran out
@@ -350,49 +358,58 @@ struct ResRow {
     bool ok;
 };
 
+// One block's part of a member's solve.
 template <typename T, int NL>
-__global__ void __launch_bounds__(kResThreads, 1) k_res_loop(Eng<T> E, ResBufs<T> R, long limit, int absent) {
-    if ((int)blockIdx.x == absent) return;
-    __shared__ ResShared<T> sh;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int nw = (blockDim.x >> 5) - 1, ws = nw;      // row warps; the scalar warp
+struct Resident {
+    static constexpr int NI = kResIdx<NL>, NC = NI + 1;
+    const Eng<T>& E;
+    const ResBufs<T>& R;
+    ResShared& sh;
+    ResWait wt;
+    int lane, w, nw, ws;               // nw row warps; ws: the scalar warp
     BalBlock bb;
-    long off;
-    int n, c0, c1;
-    const bool go = bal_block(E, R.tab, bb, off, n, c0, c1);
-    if (!go || sld(&E.S[bb.m].done)) return;            // a stopped member: none of its blocks iterates
-    if (threadIdx.x == 0) sh.fail = 0;
-    copy_scalars(sh.s, E.S + bb.m);
-    const unsigned ep = (unsigned)sld(E.ctrl + 6);
-    const ResWait wt{limit, E.abort, &sh.fail};
-    __syncthreads();
-    if (w == ws && lane == 0) {
-        // EPS^2 with a margin far above the roundings of q (an EPS whose square underflows
-        // gives 0: then q decides, and q = 0 goes to the exact tests)
-        sh.st = ResStop{1.0 / sh.s.BN, sh.s.EPS * sh.s.EPS * (1.0 + 1e-9), 0.0, 0.0};
+    long off, pstride;
+    int n, c0, c1, nc, pad, nq, nround, gstride;
+    unsigned row0;
+    TagWord<double>*part, *gpart;
+
+    // false: a stopped member, none of its blocks works
+    __device__ __forceinline__ Resident(const Eng<T>& E_, const ResBufs<T>& R_, ResShared& sh_, long limit)
+        : E(E_), R(R_), sh(sh_), wt{limit, E_.abort, &sh_.fail} {
+        lane = threadIdx.x & 31;
+        w = threadIdx.x >> 5;
+        nw = ws = (blockDim.x >> 5) - 1;
+        bal_block(E, R.tab, bb, off, n, c0, c1);
+        if (threadIdx.x == 0) sh.fail = sh.stop = 0;
+        copy_scalars(sh.s, E.S + bb.m);
+        __syncthreads();
+        nc = (n + kChunk - 1) / kChunk;
+        pad = (int)off + n;
+        nq = w == ws ? 0 : 4 * (c1 - c0);                   // the scalar warp has no rows
+        nround = (4 * (c1 - c0) + nw - 1) / nw;
+        row0 = (unsigned)(off + (long)c0 * kChunk) + lane;
+        part = R.part + 2 * (off / kChunk);
+        pstride = 2 * (E.NV / kChunk);
+        gpart = R.gpart + 2 * E.mem_grp0[bb.m];
+        gstride = 2 * R.ngrp;
     }
-    constexpr int NI = kResIdx<NL>, NC = NI + 1;
-    const int nc = (n + kChunk - 1) / kChunk, pad = (int)off + n;
-    const int nq = w == ws ? 0 : 4 * (c1 - c0);         // the scalar warp has no rows
-    const int nround = (4 * (c1 - c0) + nw - 1) / nw;
-    const unsigned row0 = (unsigned)(off + (long)c0 * kChunk) + lane;
-    TagWord<double>* part = R.part + 2 * (off / kChunk);
-    const long pstride = 2 * (E.NV / kChunk);
-    TagWord<double>* gpart = R.gpart + 2 * E.mem_grp0[bb.m];
-    const int gstride = 2 * R.ngrp;
-    auto row = [&](int q) {
+    __device__ __forceinline__ ResRow row(int q) const {
         unsigned i = row0 + 32u * q;
         asm volatile("" : "+r"(i));          // addresses are formed in each phase, not carried through all of them
         return ResRow{i, (int)i < pad};
-    };
-    auto coef = [&](const ResRow& rw) { return R.a + (size_t)(rw.i >> 5) * (32 * NC) + lane; };
-    auto idx = [&](const ResRow& rw) { return R.c + (size_t)(rw.i >> 5) * (32 * NI) + lane; };
-    auto self = [&](const ResRow& rw) { return rw.ok ? (int)rw.i : pad; };
-    // t[0] = D in + sum_k AL_k in[LL_k] (as k_bal_axsub)
-    auto axsub = [&](const TagWord<T>* in, const T* own, unsigned tag) {
+    }
+    __device__ __forceinline__ const T* coef(const ResRow& rw) const { return R.a + (size_t)(rw.i >> 5) * (32 * NC) + lane; }
+    __device__ __forceinline__ const int* idx(const ResRow& rw) const { return R.c + (size_t)(rw.i >> 5) * (32 * NI) + lane; }
+    __device__ __forceinline__ int self(const ResRow& rw) const { return rw.ok ? (int)rw.i : pad; }
+    // f(row) over this warp's rows
+    template <typename F>
+    __device__ __forceinline__ void rows(F f) const {
 #pragma unroll 1
-        for (int q = w; q < nq; q += nw) {
-            const ResRow rw = row(q);
+        for (int q = w; q < nq; q += nw) f(row(q));
+    }
+    // t[0] = D in + sum_k AL_k in[LL_k] (as k_bal_axsub); own: the block's rows of `in`
+    __device__ __forceinline__ void axsub(const T* own, unsigned tag) const {
+        rows([&](const ResRow& rw) {
             const T* a = coef(rw);
             const int* cp = idx(rw);
             T g[NL];
@@ -400,203 +417,309 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_loop(Eng<T> E, ResBufs<T
 #pragma unroll
             for (int k = 0; k < NL; k++) c[k] = cp[32 * k];
             T s = own[rw.i] * a[32 * NI];
-            res_gather<T, NL>(in, c, pad, tag, g, wt);
+            res_gather<T, NL>(R.in, c, pad, tag, g, wt);
 #pragma unroll
             for (int k = 0; k < NL; k++) s = fma_rn(a[32 * k], g[k], s);
             if (rw.ok) tag_put(R.t[0] + rw.i, s, tag);
-        }
-    };
+        });
+    }
     // Sweeps S, S + 1 of LDUSUB at a row, from the words `in`; X: the slot of sweep S at
-    // column S + 1.
-    auto pair = [&](const ResRow& rw, const TagWord<T>* in, unsigned tag, auto S, auto X) {
-        constexpr int s = decltype(S)::value - 1, x = decltype(X)::value;
+    // column S + 1.  V: the vectors' type (FP64 vectors on FP32 coefficients in the mixed
+    // path's refinement).
+    template <int S, int X, typename V>
+    __device__ __forceinline__ V pair(const ResRow& rw, const TagWord<V>* in, unsigned tag) const {
+        constexpr int s = S - 1;
         const T* a = coef(rw);
         const int* cp = idx(rw);
-        const int c[4] = {self(rw), cp[32 * s], cp[32 * (s + 1)], cp[32 * x]};
-        T g[4];
-        res_gather<T, 4>(in, c, pad, tag, g, wt);
-        const T o = fnma(a[32 * s], g[1], g[0]);
-        return fnma(a[32 * (s + 1)], fnma(a[32 * x], g[3], g[2]), o);
-    };
-    using std::integral_constant;
-#define RES_K(k) integral_constant<int, k>()
-    // every step of LDUSUB but the last, from t[0]
-    auto step = [&](int k, unsigned tag, auto S, auto X) {
-#pragma unroll 1
-        for (int q = w; q < nq; q += nw) {
-            const ResRow rw = row(q);
-            const T o = pair(rw, R.t[k], tag, S, X);
-            if (rw.ok) tag_put(R.t[k + 1] + rw.i, o, tag);
-        }
-    };
-    auto sweeps = [&](unsigned tag) {
-        step(0, tag, RES_K(1), RES_K(NL));
-        if constexpr (NL == 6) step(1, tag, RES_K(3), RES_K(NL + 1));
-    };
+        const int c[4] = {self(rw), cp[32 * s], cp[32 * (s + 1)], cp[32 * X]};
+        V g[4];
+        res_gather<V, 4>(in, c, pad, tag, g, wt);
+        const V o = fnma((V)a[32 * s], g[1], g[0]);
+        return fnma((V)a[32 * (s + 1)], fnma((V)a[32 * X], g[3], g[2]), o);
+    }
+    // LDUSUB's steps but the last, from the words t[0]
+    template <typename V>
+    __device__ __forceinline__ void sweeps(TagWord<V>* const (&t)[kResSteps], unsigned tag) const {
+        rows([&](const ResRow& rw) {
+            const V o = pair<1, NL, V>(rw, t[0], tag);
+            if (rw.ok) tag_put(t[1] + rw.i, o, tag);
+        });
+        if constexpr (NL == 6)
+            rows([&](const ResRow& rw) {
+                const V o = pair<3, NL + 1, V>(rw, t[1], tag);
+                if (rw.ok) tag_put(t[2] + rw.i, o, tag);
+            });
+    }
     // the last step at one row
-    auto last = [&](const ResRow& rw, unsigned tag) {
+    template <typename V>
+    __device__ __forceinline__ V last(TagWord<V>* const (&t)[kResSteps], const ResRow& rw, unsigned tag) const {
         if constexpr (NL == 4) {
-            return pair(rw, R.t[1], tag, RES_K(3), RES_K(NL + 1));
+            return pair<3, NL + 1, V>(rw, t[1], tag);
         } else {
             const T* a = coef(rw);
             const int* cp = idx(rw);
             const int c[3] = {self(rw), cp[32 * 4], cp[32 * 5]};
-            T g[3];
-            res_gather<T, 3>(R.t[2], c, pad, tag, g, wt);
-            return fnma(a[32 * 5], g[2], fnma(a[32 * 4], g[1], g[0]));
+            V g[3];
+            res_gather<V, 3>(t[2], c, pad, tag, g, wt);
+            return fnma((V)a[32 * 5], g[2], fnma((V)a[32 * 4], g[1], g[0]));
         }
-    };
-    // The chunk totals of one round (nw / 4 chunks, their rows' y and u in shared
-    // memory): lane l of a chunk's warp folds its rows 32 u + l in order, then the
-    // butterfly.  MODE 0: (u, y); 1: (u, y) and (y, y); 2: (y, y) and (y, u), each
-    // total by a warp of its own.
-    auto fold = [&](int rd, int red, unsigned tag, auto mode) {
-        constexpr int MODE = decltype(mode)::value;
-        constexpr int NVAL = MODE == 0 ? 1 : 2;
-        __syncthreads();
-        const int cw = w / NVAL, k = w % NVAL, cc = c0 + rd * (nw / 4) + cw;
-        if (cw < nw / 4 && cc < c1) {
-            const bool square = MODE == 1 ? k == 1 : MODE == 2 ? k == 0 : false;
-            T v = T(0);
-#pragma unroll
-            for (int u = 0; u < kChunkRows; u++) {
-                if ((long)cc * kChunk + 32 * u + lane >= n) continue;
-                const T y = sh.y[4 * cw + u][lane], b = square ? y : sh.u[4 * cw + u][lane];
-                v = fma_rn(b, y, v);
+    }
+    // A reduction over the block's rows: f(row, y, u) gives each row's operands, and lane l
+    // of a chunk's warp folds its rows 32 u + l in order, then the butterfly, in V.
+    // MODE 0: (u, y); 1: (u, y) and (y, y); 2: (y, y) and (y, u); 3: (y, y) -- each total
+    // by a warp of its own.
+    template <int MODE, typename V, typename F>
+    __device__ __forceinline__ void reduce(int red, unsigned tag, F f) const {
+        constexpr int NVAL = MODE == 1 || MODE == 2 ? 2 : 1;
+        V* ys = (V*)sh.y;
+        V* us = (V*)sh.u;
+#pragma unroll 1
+        for (int rd = 0; rd < nround; rd++) {
+            const int q = rd * nw + w;                      // past nq in the scalar warp
+            if (q < nq) {
+                V y, u = V(0);
+                f(row(q), y, u);
+                ys[32 * w + lane] = y;
+                if (MODE != 3) us[32 * w + lane] = u;
             }
+            __syncthreads();
+            const int cw = w / NVAL, k = w % NVAL, cc = c0 + rd * (nw / 4) + cw;
+            if (cw < nw / 4 && cc < c1) {
+                const bool square = MODE == 3 || (MODE == 1 && k == 1) || (MODE == 2 && k == 0);
+                V v = V(0);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) tag_put(part + red * pstride + 2 * cc + k, (double)v, tag);
+                for (int h = 0; h < kChunkRows; h++) {
+                    if ((long)cc * kChunk + 32 * h + lane >= n) continue;
+                    const int at = 32 * (4 * cw + h) + lane;
+                    const V y = ys[at], b = square ? y : us[at];
+                    v = fma_rn(b, y, v);
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0) tag_put(part + red * pstride + 2 * cc + k, (double)v, tag);
+            }
+            if (rd + 1 < nround) __syncthreads();
         }
-        if (rd + 1 < nround) __syncthreads();
-    };
-    unsigned it = 0;
+    }
+    // The member's totals of reduction `red` and what follows from them: fin(totals) in
+    // one thread; every thread then knows whether to go on.
+    template <int NVAL, typename F>
+    __device__ __forceinline__ bool totals(int red, unsigned tag, F fin) const {
+        if (w == ws) {
+            double tot[2];
+            res_totals<NVAL>(part + red * pstride, gpart + red * gstride, nc, c0, c1, tag, wt, tot);
+            if (lane == 0) {
+                fin(tot);
+                sh.stop = sh.s.done || *(volatile int*)&sh.fail;
+            }
+        }
+        __syncthreads();
+        return sh.stop == 0;
+    }
+    // The iterations of one (inner) solve from r = p = r0, xi, BN and C1; ep: epochs used so
+    // far, each iteration takes two.
+    __device__ __forceinline__ void iterate(unsigned& ep) const {
+        if (w == ws && lane == 0)
+            // EPS^2 with a margin far above the roundings of q (an EPS whose square underflows
+            // gives 0: then q decides, and q = 0 goes to the exact tests)
+            sh.st = ResStop{1.0 / sh.s.BN, sh.s.EPS * sh.s.EPS * (1.0 + 1e-9), 0.0, 0.0, 0};
 #pragma unroll 1
-    for (;; it++) {
-        const unsigned ta = 2 * (ep + it) + 1, tb = ta + 1;
-        double tot[2];
-        {                                                   // p = r + BETA (p - AMU q), published
+        for (int it = 0;; it++, ep += 2) {
+            const unsigned ta = ep + 1, tb = ep + 2;
             const T BETA = T(sh.beta);
-#pragma unroll 1
-            for (int q = w; q < nq; q += nw) {
-                const ResRow rw = row(q);
+            rows([&](const ResRow& rw) {                    // p = r + BETA (p - AMU q), published
                 T p = E.p[rw.i];                            // p - AMU q after the first iteration
                 if (it > 0) {
                     p = fma_rn(BETA, p, E.r[rw.i]);
                     if (rw.ok) E.p[rw.i] = p;
                 }
-                if (rw.ok) tag_put(R.p + rw.i, p, ta);
-            }
-        }
-        axsub(R.p, E.p, ta);                                // q = PM A p ; RQ -> ALP
-        sweeps(ta);
-#pragma unroll 1
-        for (int rd = 0; rd < nround; rd++) {
-            const int q = rd * nw + w;                      // past nq in the scalar warp
-            if (q < nq) {
-                const ResRow rw = row(q);
-                const T r0 = E.r0[rw.i];
-                const T y = last(rw, ta);
+                if (rw.ok) tag_put(R.in + rw.i, p, ta);
+            });
+            axsub(E.p, ta);                                 // q = PM A p ; RQ -> ALP
+            sweeps<T>(R.t, ta);
+            reduce<0, T>(0, ta, [&](const ResRow& rw, T& y, T& u) {
+                u = E.r0[rw.i];
+                y = last<T>(R.t, rw, ta);
                 if (rw.ok) E.q[rw.i] = y;
-                sh.y[w][lane] = y;
-                sh.u[w][lane] = r0;
-            }
-            fold(rd, 0, ta, RES_K(0));
-        }
-        if (w == ws) {
-            res_totals<1>(part, gpart, nc, c0, c1, ta, wt, tot);
-            if (lane == 0) {
-                if (!sh.s.done) finish_sweep56<1, true>(&sh.s, tot, &sh.s);   // done: by the last iteration's stop tests
-                sh.stop = sh.s.done || *(volatile int*)&sh.fail;
-            }
-        }
-        __syncthreads();
-        if (sh.stop) break;
-        {                                                   // e = r - ALP q, published
+            });
+            if (!totals<1>(0, ta, [&](const double (&tot)[2]) {
+                    if (!sh.s.done) finish_sweep56<1, true>(&sh.s, tot, &sh.s);   // done: by the last iteration's stop tests
+                }))
+                break;
             const T ALP = T(sh.s.ALP);
-#pragma unroll 1
-            for (int q = w; q < nq; q += nw) {
-                const ResRow rw = row(q);
+            rows([&](const ResRow& rw) {                    // e = r - ALP q, published
                 const T e = fnma(ALP, E.q[rw.i], E.r[rw.i]);
                 if (rw.ok) {
                     E.e[rw.i] = e;
-                    tag_put(R.e + rw.i, e, tb);
+                    tag_put(R.in + rw.i, e, tb);
                 }
-            }
-        }
-        axsub(R.e, E.e, tb);                                // v = PM A e ; AMU
-        sweeps(tb);
-#pragma unroll 1
-        for (int rd = 0; rd < nround; rd++) {
-            const int q = rd * nw + w;                      // past nq in the scalar warp
-            if (q < nq) {
-                const ResRow rw = row(q);
-                const T e = E.e[rw.i];
-                const T y = last(rw, tb);
+            });
+            axsub(E.e, tb);                                 // v = PM A e ; AMU
+            sweeps<T>(R.t, tb);
+            reduce<1, T>(1, tb, [&](const ResRow& rw, T& y, T& u) {
+                u = E.e[rw.i];
+                y = last<T>(R.t, rw, tb);
                 if (rw.ok) E.v[rw.i] = y;
-                sh.y[w][lane] = y;
-                sh.u[w][lane] = e;
-            }
-            fold(rd, 1, tb, RES_K(1));
-        }
-        if (w == ws) {
-            res_totals<2>(part + pstride, gpart + gstride, nc, c0, c1, tb, wt, tot);
-            if (lane == 0) {
-                finish_sweep56<2, true>(&sh.s, tot, &sh.s);
-                sh.stop = sh.s.done || *(volatile int*)&sh.fail;
-            }
-        }
-        __syncthreads();
-        if (sh.stop) break;
-        const T ALP = T(sh.s.ALP), AMU = T(sh.s.AMU);       // x, r ; RN, C1 ; stop tests
-#pragma unroll 1
-        for (int rd = 0; rd < nround; rd++) {
-            const int q = rd * nw + w;                      // past nq in the scalar warp
-            if (q < nq) {
-                const ResRow rw = row(q);
-                const T r0 = E.r0[rw.i];
-                const T rn = fnma(AMU, E.v[rw.i], E.e[rw.i]);
-                if (rw.ok) E.r[rw.i] = rn;
-                sh.y[w][lane] = rn;
-                sh.u[w][lane] = r0;
-            }
-            fold(rd, 2, ta, RES_K(2));
-        }
-#pragma unroll 1
-        for (int q = w; q < nq; q += nw) {                  // while the totals travel
-            const ResRow rw = row(q);
-            if (rw.ok) {
-                const T p = E.p[rw.i];
-                E.xi[rw.i] = fma_rn(AMU, E.e[rw.i], fma_rn(ALP, p, E.xi[rw.i]));
-                E.p[rw.i] = fnma(AMU, E.q[rw.i], p);
-            }
-        }
-        double beta = 0.0;
-        if (w == ws) {
-            res_totals<2>(part + 2 * pstride, gpart + 2 * gstride, nc, c0, c1, ta, wt, tot);
-            if (lane == 0) {                                // 241 (pcgpme_para.F90); pcgpme_2DH.f90:255
-                beta = sh.s.mode == 2 ? tot[1] / (sh.s.AMU * sh.s.RQ) : tot[1] / sh.s.AMU / sh.s.RQ;
+            });
+            if (!totals<2>(1, tb, [&](const double (&tot)[2]) { finish_sweep56<2, true>(&sh.s, tot, &sh.s); })) break;
+            const T AMU = T(sh.s.AMU);                      // x, r ; RN, C1 ; stop tests
+            reduce<2, T>(2, ta, [&](const ResRow& rw, T& y, T& u) {
+                u = E.r0[rw.i];
+                y = fnma(AMU, E.v[rw.i], E.e[rw.i]);
+                if (rw.ok) E.r[rw.i] = y;
+            });
+            rows([&](const ResRow& rw) {                    // while the totals travel
+                if (rw.ok) {
+                    const T p = E.p[rw.i];
+                    E.xi[rw.i] = fma_rn(AMU, E.e[rw.i], fma_rn(ALP, p, E.xi[rw.i]));
+                    E.p[rw.i] = fnma(AMU, E.q[rw.i], p);
+                }
+            });
+            double rn = 0.0, c1n = 0.0, beta = 0.0;
+            totals<2>(2, ta, [&](const double (&tot)[2]) {  // 241 (pcgpme_para.F90); pcgpme_2DH.f90:255
+                rn = tot[0];
+                c1n = tot[1];
+                beta = sh.s.mode == 2 ? c1n / (sh.s.AMU * sh.s.RQ) : c1n / sh.s.AMU / sh.s.RQ;
                 sh.beta = beta;
-            }
+            });
+            if (*(volatile int*)&sh.stop) break;            // a poll ran out
+            // the stop tests, while the row warps start the next iteration; the verdict counts
+            // at its first reduction
+            if (w == ws && lane == 0) res_stop_tests(&sh.s, sh.st, rn, c1n, beta);
+        }
+        ep += 2;
+        if (w == ws && lane == 0 && sh.st.tests > 0 && f64_finite(sh.s.RN)) {
+            // ERR of the last iteration, and ERRP where no stop test kept the older one
+            sh.s.ERR = sqrt(sh.s.RN / sh.s.BN);
+            if (!(sh.s.done && (sh.s.reason == CLOWNS_STOP_STAGNATION || sh.s.reason == CLOWNS_STOP_TOL)))
+                sh.s.ERRP = sh.s.ERR;
         }
         __syncthreads();
-        // the stop tests, while the row warps start the next iteration; the verdict counts
-        // at its first reduction
-        if (w == ws && lane == 0) res_stop_tests(&sh.s, sh.st, tot[0], tot[1], beta);
     }
-#undef RES_K
-    if (bb.j == 0 && w == ws && lane == 0 && sh.s.K > 0 && f64_finite(sh.s.RN)) {
-        // ERR of the last iteration, and ERRP where no stop test kept the older one
-        sh.s.ERR = sqrt(sh.s.RN / sh.s.BN);
-        if (!(sh.s.done && (sh.s.reason == CLOWNS_STOP_STAGNATION || sh.s.reason == CLOWNS_STOP_TOL)))
-            sh.s.ERRP = sh.s.ERR;
+    // the member's scalars for the host, and its solution for the caller
+    __device__ __forceinline__ void finish(const T* x, const double* x64) const {
+        double* out = E.in[bb.m].x - off;
+        rows([&](const ResRow& rw) {
+            if (rw.ok) out[rw.i] = x64 ? x64[rw.i] : (double)x[rw.i];
+        });
+        if (bb.j == 0) {
+            constexpr int W = (int)(sizeof(MemberScalars) / 4);
+            if (threadIdx.x < W) ((int*)(E.S + bb.m))[threadIdx.x] = ((const int*)&sh.s)[threadIdx.x];
+        }
     }
-    __syncthreads();
-    if (bb.j == 0) {                                        // the member's scalars, for the host and later kernels
-        constexpr int W = (int)(sizeof(MemberScalars) / 4);
-        if (threadIdx.x < W) ((int*)(E.S + bb.m))[threadIdx.x] = ((const int*)&sh.s)[threadIdx.x];
-        if (threadIdx.x == 0) atomicMax(E.ctrl + 7, (int)(ep + it + 1));
+};
+
+// A whole FP64 solve after the setup kernels: b^ = PM W b and BN, r = b^ - PM A x0
+// and C1 (pcgpme_para.F90:113-145), the iterations, x to the caller.
+template <int NL>
+__global__ void __launch_bounds__(kResThreads, 1) k_res_plain(const Eng<double> E, const ResBufs<double> R, long limit,
+                                                             int absent) {
+    if ((int)blockIdx.x == absent) return;
+    __shared__ ResShared sh;
+    const Resident<double, NL> S(E, R, sh, limit);
+    S.rows([&](const ResRow& rw) {
+        if (rw.ok) tag_put(R.t[0] + rw.i, E.p[rw.i], 1);    // W b
+    });
+    S.template sweeps<double>(R.t, 1);
+    S.template reduce<3, double>(0, 1, [&](const ResRow& rw, double& y, double&) {
+        y = S.template last<double>(R.t, rw, 1);
+        if (rw.ok) {
+            E.p[rw.i] = y;
+            tag_put(R.in + rw.i, E.xi[rw.i], 2);
+        }
+    });
+    bool go = S.template totals<1>(0, 1, [&](const double (&tot)[2]) { sh.s.BN = tot[0]; });
+    if (go) {
+        S.axsub(E.xi, 2);
+        S.template sweeps<double>(R.t, 2);
+        S.template reduce<3, double>(1, 2, [&](const ResRow& rw, double& y, double&) {
+            y = E.p[rw.i] - S.template last<double>(R.t, rw, 2);
+            if (rw.ok) {
+                E.r[rw.i] = y;
+                E.p[rw.i] = y;
+                E.r0[rw.i] = y;
+            }
+        });
+        go = S.template totals<1>(1, 2, [&](const double (&tot)[2]) { sh.s.C1 = tot[0]; });
     }
+    unsigned ep = 2;
+    if (go) S.iterate(ep);
+    S.finish(E.xi, nullptr);
+}
+
+// A whole mixed-precision solve after the setup kernels: ||PM W b|| on FP64 vectors,
+// then refinement sweeps (as k_mx_residual, k_mx_sweep56, k_mx_normalize, k_mx_update)
+// around the FP32 iterations until the member's outer stop test.
+template <int NL>
+__global__ void __launch_bounds__(kResThreads, 1) k_res_mixed(const Eng<float> E, const ResBufs<float> R,
+                                                             double inner_tol, int inner_max, long limit, int absent) {
+    if ((int)blockIdx.x == absent) return;
+    __shared__ ResShared sh;
+    const Resident<float, NL> S(E, R, sh, limit);
+    const MemberIn in = E.in[S.bb.m];
+    S.rows([&](const ResRow& rw) {
+        if (rw.ok) {
+            tag_put(R.t64[0] + rw.i, E.r64[rw.i], 1);       // W b
+            tag_put(R.x64 + rw.i, E.x64[rw.i], 1);
+        }
+    });
+    S.template sweeps<double>(R.t64, 1);
+    S.template reduce<3, double>(4, 1, [&](const ResRow& rw, double& y, double&) { y = S.template last<double>(R.t64, rw, 1); });
+    bool go = S.template totals<1>(4, 1, [&](const double (&tot)[2]) { sh.s.BN64 = tot[0]; });
+    unsigned ep = 1, xtag = 1;
+#pragma unroll 1
+    while (go) {
+        const unsigned tag = ++ep;
+        S.rows([&](const ResRow& rw) {                      // r64 = W (b - A x64), the caller's matrix
+            const long li = (long)rw.i - S.off;
+            double g[NL];
+            int c[NL];
+#pragma unroll
+            for (int k = 0; k < NL; k++) {
+                const int cc = rw.ok && k < in.nl ? in.ll[k * (long)in.na + li] : 0;
+                c[k] = cc > 0 && cc <= S.n ? (int)S.off + cc - 1 : S.pad;
+            }
+            double s = rw.ok ? in.d[li] * E.x64[rw.i] : 0.0;
+            res_gather<double, NL>(R.x64, c, S.pad, xtag, g, S.wt);
+#pragma unroll
+            for (int k = 0; k < NL; k++)
+                if (c[k] != S.pad) s = fma_rn(in.al[k * (long)in.na + li], g[k], s);
+            if (rw.ok) tag_put(R.t64[0] + rw.i, E.W[rw.i] * (in.b[li] - s), tag);
+        });
+        S.template sweeps<double>(R.t64, tag);
+        S.template reduce<3, double>(3, tag, [&](const ResRow& rw, double& y, double&) {
+            y = S.template last<double>(R.t64, rw, tag);
+            if (rw.ok) E.r64[rw.i] = y;
+        });
+        go = S.template totals<1>(3, tag, [&](const double (&tot)[2]) { mx_outer_test(&sh.s, tot[0], inner_tol, inner_max); });
+        if (!go) break;
+        const double inv = 1.0 / sh.s.SIGMA;
+        S.template reduce<3, double>(4, tag, [&](const ResRow& rw, double& y, double&) {
+            const float v = (float)(E.r64[rw.i] * inv);
+            if (rw.ok) {
+                E.r[rw.i] = v;
+                E.p[rw.i] = v;
+                E.r0[rw.i] = v;
+                E.xi[rw.i] = 0.f;
+            }
+            y = (double)v;
+        });
+        go = S.template totals<1>(4, tag, [&](const double (&tot)[2]) { sh.s.BN = sh.s.C1 = tot[0]; });
+        if (!go) break;
+        S.iterate(ep);
+        xtag = ++ep;
+        const double sg = sh.s.SIGMA;
+        S.rows([&](const ResRow& rw) {                      // x64 += sigma xi, published
+            const double x = fma_rn(sg, (double)E.xi[rw.i], E.x64[rw.i]);
+            if (rw.ok) {
+                E.x64[rw.i] = x;
+                tag_put(R.x64 + rw.i, x, xtag);
+            }
+        });
+        go = *(volatile int*)&sh.fail == 0;
+        go = __syncthreads_and(go);
+    }
+    S.finish(nullptr, E.x64);
 }
 
 }  // namespace clowns

@@ -174,7 +174,7 @@ int clowns_pcgpme_batched_dev(int m, const clowns_member* members, int precision
  * dependent launch), CLOWNS_LOOP_WAVE (one cooperative kernel running
  * (stage, tile) items in wavefront order; single systems only) or
  * CLOWNS_LOOP_RESIDENT (one cooperative kernel whose blocks exchange rows as
- * {value, epoch} words; small and medium single systems, by rule).  block:
+ * {value, epoch} words; small and medium systems and ensembles, by rule).  block:
  * threads per block; grid: blocks of the cooperative kernels (0 for the graph);
  * regs: their register budget per thread (0 for the graph); fused (graph): bit 0
  * set when LDUSUB's sweeps 1-2 and 3-4 run as fused pairs, bit 1 set when the
@@ -205,7 +205,8 @@ int clowns_test_arm_wait_timeout(long polls, int absent_block);
 /* Kernels the calling thread's last solve (plain or mixed, single or batched)
  * launched: host launches plus the kernel nodes its loop graphs executed
  * (per iteration 16 with single LDUSUB sweeps, 12 with fused sweep pairs, the
- * loop guard included), not counting the autotuner's one-time trial runs.
+ * loop guard included; three when the solve runs resident), not counting the
+ * autotuner's one-time trial runs.
  * Engine bookkeeping with no counterpart in the reference. */
 long clowns_last_kernel_launches(void);
 

@@ -66,6 +66,26 @@ def test_resident_equals_graph(gpu, monkeypatch, n, nl, kind):
         assert torch.equal(xr, xg), mixed
 
 
+def test_resident_ensemble_equals_graph(gpu, monkeypatch):
+    """Members from one row to several blocks, four and six columns side by side, one
+    with a NaN right-hand side: each ends as in the graph ensemble."""
+    import torch
+    systems = [_system(n, nl, kind) for n, nl, kind in
+               ((1, 6, "band"), (129, 4, "random"), (4097, 6, "random"), (20001, 6, "band"), (8193, 4, "band"))]
+    systems[2][3][5] = float("nan")
+    sizes = [s[3].numel() for s in systems]
+    for prec in (gpu.PREC_FP64, gpu.PREC_MIXED):
+        got = []
+        for mode in ("graph", "resident"):
+            _force(monkeypatch, mode)
+            xs = [torch.zeros(n, dtype=torch.float64, device="cuda") for n in sizes]
+            infos = gpu.BatchedSolver(sizes, prec).solve(systems, xs, eps=1e-10)
+            got.append(([x.cpu().numpy() for x in xs], [str(i.as_dict()) for i in infos]))
+        assert got[0][1] == got[1][1], prec
+        for a, b in zip(got[0][0], got[1][0]):
+            assert np.array_equal(a, b, equal_nan=True), prec
+
+
 def test_resident_nan_and_cap(gpu, monkeypatch):
     """A NaN right-hand side and an exhausted iteration cap end as in the graph."""
     import torch
