@@ -6,6 +6,7 @@
 // evaluation order, so the assembled matrix is bit-identical to an IEEE
 // evaluation of the Fortran source (the per-row sort inside the solve compares
 // these values, and ties must break the same way).
+#include <algorithm>
 #include <cstring>
 
 #include "common.cuh"
@@ -52,46 +53,96 @@ __device__ __forceinline__ double cal_alu(double fnn, double dx, double dxm) {
     return (fnn - 0.5) * dx / (fnn * dx + dxm * 0.5) * (-1.0);
 }
 
+// Bit tests of doubles: an FP64 comparison costs as much as an addition.
+__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+__device__ __forceinline__ bool is_one(double x) { return __double_as_longlong(x) == 0x3ff0000000000000LL; }
+
 // init_matrix (1sub-matrix.F90:25-65), one thread per cell nnn = 1..inne;
-// columns 2q, 2q+1 hold the minus and plus faces of axis col_axis(q)
-__global__ void __launch_bounds__(kAsmBlock) k_init_matrix(GridIdx g, int inne, const int* __restrict__ mn,
+// columns 2q, 2q+1 hold the minus and plus faces of axis col_axis(q).
+//
+// What bounds it: an FP64 division costs about ten FP64 operations of a pipe that
+// does 1.7 lane operations per clock and SM, and cal_alu_f has three per face: the
+// kernel ran at 1.60 ms for 4.9 M cells (0.6 GB of traffic, 0.09 ms).  The factors
+// depend on one index of one axis, so every block forms the table of all of them in
+// shared memory (TAB; two blocks per SM walk all cells), and a face needs only the
+// products with its area and porosity where these are not 1.
+// TAB = false: grids whose table exceeds shared memory form every factor.
+constexpr int kInitBlock = 512;
+template <int NL, bool TAB>
+__global__ void __launch_bounds__(kInitBlock, 2) k_init_matrix(GridIdx g, int inne, int mx2, const int* __restrict__ mn,
                                                           const int* __restrict__ in_, const int* __restrict__ jn,
                                                           const int* __restrict__ kn, const int* __restrict__ nf,
                                                           const int* __restrict__ nfb, const double* __restrict__ a,
                                                           const double* __restrict__ fb, const double* __restrict__ dx,
                                                           const double* __restrict__ mp_p, double* __restrict__ alu_c,
                                                           int* __restrict__ ll_c, double* __restrict__ de_c) {
+    extern __shared__ double tab[];
     const double mp = *mp_p;
     const long ld = inne;
-    const int nl = g.nl();
+    const int base[3] = {g.is - 1, g.js - 1, g.ks - 1};     // cells lie in ls - 1 .. le + 1
+    const int len[3] = {g.ie - g.is + 3, g.je - g.js + 3, g.ke - g.ks + 3};
+    const int total = len[0] + len[1] + len[2];
+    const int at[3] = {-base[0], len[0] - base[1], len[0] + len[1] - base[2]};
+    if (TAB) {
+        for (int t = threadIdx.x; t < 2 * total; t += blockDim.x) {
+            const int side = t >= total, u = t - side * total;
+            const int l = u < len[0] ? 0 : u < len[0] + len[1] ? 1 : 2, i = u - at[l];
+            if (i + side > mx2) continue;
+            const double d = dx[g.dxo(l, i)], dm = dx[g.dxo(l, i + (side ? 1 : -1))];
+            const double f = 2.0 / d / (d + dm);
+            tab[t] = f;
+            tab[2 * total + t] = -(mp * f);
+        }
+        __syncthreads();
+    }
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < inne; t += (long)gridDim.x * blockDim.x) {
         const int nnn = (int)t + 1;
-        if (nf[nnn] == -1 || fb[nnn] == 0.0) {
-            for (int c = 0; c < nl; c++) { alu_c[c * ld + t] = 0.0; ll_c[c * ld + t] = 0; }
+        const double fbn = fb[nnn];
+        const int fl = nf[nnn];
+        const int i = in_[nnn], j = jn[nnn], k = kn[nnn];
+        if (fl == -1 || is_zero(fbn)) {
+#pragma unroll
+            for (int c = 0; c < NL; c++) { alu_c[c * ld + t] = 0.0; ll_c[c * ld + t] = 0; }
             de_c[t] = 0.0;
             continue;
         }
-        const int i = in_[nnn], j = jn[nnn], k = kn[nnn];
         const int lg[3] = {i, j, k};
-        double de = 0.0;
-        for (int q = 0; q < nl / 2; q++) {
-            const int l = g.col_axis(q);
+        const int self = mn[g.mn_off(i, k, j)];
+        int np[NL], fn[NL];
+        double ar[NL], fbp[NL];
 #pragma unroll
-            for (int side = 0; side < 2; side++) {
-                const int ii = side ? 1 : -1;
-                const int np = mn[g.nbr(i, j, k, l, ii)];
-                const int npp = side ? np : mn[g.mn_off(i, k, j)];
-                const int col = 2 * q + side;      // 0-based; 3D: x-, x+, y-, y+, z-, z+
-                if ((nf[np] == -1 && nfb[np] != 4) || a[3L * npp + l] == 0.0 || fb[np] == 0.0) {
-                    ll_c[col * ld + t] = 0;
-                    alu_c[col * ld + t] = 0.0;
-                } else {
-                    const double v = -(mp * cal_alu_f(dx[g.dxo(l, lg[l])], dx[g.dxo(l, lg[l] + ii)], a[3L * npp + l], fb[nnn]));
-                    ll_c[col * ld + t] = np;
-                    alu_c[col * ld + t] = v;
-                    de = de - v;
-                }
+        for (int c = 0; c < NL; c++) np[c] = mn[g.nbr(i, j, k, g.col_axis(c / 2), c & 1 ? 1 : -1)];
+#pragma unroll
+        for (int c = 0; c < NL; c++) {
+            fn[c] = nf[np[c]];
+            ar[c] = a[3L * (c & 1 ? np[c] : self) + g.col_axis(c / 2)];
+            fbp[c] = fb[np[c]];
+        }
+        const bool full = is_one(fbn);
+        double de = 0.0;
+#pragma unroll
+        for (int c = 0; c < NL; c++) {                      // 3D: x-, x+, y-, y+, z-, z+
+            const int l = g.col_axis(c / 2), side = c & 1;
+            if ((fn[c] == -1 && nfb[np[c]] != 4) || is_zero(ar[c]) || is_zero(fbp[c])) {
+                ll_c[c * ld + t] = 0;
+                alu_c[c * ld + t] = 0.0;
+                continue;
             }
+            double v;
+            if (TAB) {
+                const int o = side * total + at[l] + lg[l];
+                if (full && is_one(ar[c])) v = tab[2 * total + o];
+                else {
+                    v = tab[o] * ar[c];
+                    if (!full) v = v / fbn;
+                    v = -(mp * v);
+                }
+            } else {
+                v = -(mp * cal_alu_f(dx[g.dxo(l, lg[l])], dx[g.dxo(l, lg[l] + (side ? 1 : -1))], ar[c], fbn));
+            }
+            ll_c[c * ld + t] = np[c];
+            alu_c[c * ld + t] = v;
+            de = de - v;
         }
         de_c[t] = de;
     }
@@ -101,51 +152,107 @@ __global__ void __launch_bounds__(kAsmBlock) k_init_matrix(GridIdx g, int inne, 
 // Row numbering (1sub-momentum.F90:273-296): a fluid-list entry becomes a row
 // unless it is air, solid, has zero porosity, or is a surface cell whose
 // normal-side neighbour is solid.  Rows keep fluid-list order (an exclusive scan).
-__global__ void __launch_bounds__(kAsmBlock) k_row_flags(GridIdx g, int ifln, const int* __restrict__ fln,
-                                                        const int* __restrict__ mn, const int* __restrict__ in_,
-                                                        const int* __restrict__ jn, const int* __restrict__ kn,
-                                                        const int* __restrict__ nf, const int* __restrict__ nfb,
-                                                        const double* __restrict__ fb, int* __restrict__ keep) {
-    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < ifln; t += (long)gridDim.x * blockDim.x) {
-        const int nnn = fln[t];
-        int kp = 1;
-        if (nf[nnn] == 0 || nf[nnn] == -1 || fb[nnn] == 0.0) {
-            kp = 0;
-        } else if (nf[nnn] == 2) {
-            const int b = nfb[nnn];
-            const int l = (b < 0 ? -b : b) - 1;
-            const int s = b >= 0 ? 1 : -1;
-            // an orientation of 0 has no defined neighbour in the reference; kept
-            if (l >= 0 && l <= 2 && nf[mn[g.nbr(in_[nnn], jn[nnn], kn[nnn], l, s)]] == -1) kp = 0;
-        }
-        keep[t] = kp;
+__device__ __forceinline__ bool row_kept(const GridIdx& g, int nnn, const int* __restrict__ mn,
+                                         const int* __restrict__ in_, const int* __restrict__ jn,
+                                         const int* __restrict__ kn, const int* __restrict__ nf,
+                                         const int* __restrict__ nfb, const double* __restrict__ fb) {
+    const int fl = nf[nnn];
+    if (fl == 0 || fl == -1 || is_zero(fb[nnn])) return false;
+    if (fl == 2) {
+        const int b = nfb[nnn];
+        const int l = (b < 0 ? -b : b) - 1;
+        const int s = b >= 0 ? 1 : -1;
+        // an orientation of 0 has no defined neighbour in the reference; kept
+        if (l >= 0 && l <= 2 && nf[mn[g.nbr(in_[nnn], jn[nnn], kn[nnn], l, s)]] == -1) return false;
+    }
+    return true;
+}
+
+__global__ void __launch_bounds__(kBitThreads) k_row_flags(GridIdx g, int ifln, const int* __restrict__ fln,
+                                                          const int* __restrict__ mn, const int* __restrict__ in_,
+                                                          const int* __restrict__ jn, const int* __restrict__ kn,
+                                                          const int* __restrict__ nf, const int* __restrict__ nfb,
+                                                          const double* __restrict__ fb, unsigned* __restrict__ mask,
+                                                          int* __restrict__ sums) {
+    const int tile = blockIdx.x;
+    int count = 0;
+#pragma unroll
+    for (int q = 0; q < kBitRounds; q++) {
+        const long t = (long)tile * kBitTile + q * kBitThreads + threadIdx.x;
+        const bool keep = t < ifln && row_kept(g, fln[t], mn, in_, jn, kn, nf, nfb, fb);
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if ((threadIdx.x & 31) == 0) mask[t >> 5] = m;
+        count += __popc(m);
+    }
+    __shared__ int s[kBitThreads / 32];
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = count;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kBitThreads / 32; w++) count += s[w];
+        sums[tile] = count;
     }
 }
 
-__global__ void __launch_bounds__(kAsmBlock) k_row_scatter(GridIdx g, int ifln, const int* __restrict__ fln,
+// rows beyond mm2 are not written (the host reports them)
+__global__ void __launch_bounds__(kBitThreads) k_row_scatter(GridIdx g, int ifln, int mm2, const int* __restrict__ fln,
                                                           const int* __restrict__ in_, const int* __restrict__ jn,
-                                                          const int* __restrict__ kn, const int* __restrict__ keep,
-                                                          const int* __restrict__ pos, int* __restrict__ mno,
+                                                          const int* __restrict__ kn, const unsigned* __restrict__ mask,
+                                                          const int* __restrict__ sums, int* __restrict__ mno,
                                                           int* __restrict__ mno2mn) {
-    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < ifln; t += (long)gridDim.x * blockDim.x) {
-        if (!keep[t]) continue;
-        const int nnn = fln[t];
-        const int row = pos[t] + 1;                     // 1-based row number
+    __shared__ int pre[32];
+    const int tile = blockIdx.x;
+    const unsigned* words = mask + (long)tile * 32;
+    if (threadIdx.x < 32) bit_prefix(words, pre);
+    __syncthreads();
+    const int first = sums[tile];
+#pragma unroll
+    for (int q = 0; q < kBitRounds; q++) {
+        const int w = q * (kBitThreads / 32) + (threadIdx.x >> 5);
+        const unsigned m = words[w], below = m & ((1u << (threadIdx.x & 31)) - 1);
+        if (!(m >> (threadIdx.x & 31) & 1)) continue;
+        const int nnn = fln[(long)tile * kBitTile + q * kBitThreads + threadIdx.x];
+        const int row = first + pre[w] + __popc(below) + 1;       // 1-based row number
+        if (row > mm2) continue;
         mno[g.mno_off(in_[nnn], kn[nnn], jn[nnn])] = row;
-        mno2mn[row - 1] = nnn;                          // mno2mn(row)
+        mno2mn[row - 1] = nnn;                                    // mno2mn(row)
     }
 }
 
-// renzoku_fv (lib/src/math_func.F90:51-54)
-__device__ __forceinline__ double renzoku_fv(double axp, double axm, double ayp, double aym, double azp,
-                                             double azm, double up, double um, double vp, double vm,
-                                             double wp, double wm, double dx, double dy, double dz,
-                                             double fb) {
-    return ((up * axp - um * axm) / dx + (vp * ayp - vm * aym) / dy + (wp * azp - wm * azm) / dz) / fb;
+// a / d with one rounding, given y = 1 / d rounded to nearest: Markstein's method (IBM
+// J. Res. Dev. 34, 1990).  a y, corrected once by its remainder, is within an ulp of the
+// quotient, and such a value corrected by its exact remainder times y rounds to it; the
+// remainders are exact while a and d are far from the ends of the exponent range, and
+// a zero keeps its sign only in a division, so those cases divide.  Five FP64 operations
+// instead of about ten.
+struct Recip {
+    double d, y;
+    bool ok;
+};
+__device__ __forceinline__ bool mid_exponent(double x) {
+    const int e = (__double2hiint(x) >> 20) & 0x7ff;
+    return e > 523 && e < 1523;                          // 2^-500 .. 2^500
+}
+__device__ __forceinline__ Recip make_recip(double d) { return Recip{d, 1.0 / d, mid_exponent(d)}; }
+__device__ __forceinline__ double div_by(double a, const Recip& r) {
+    if (!r.ok || !mid_exponent(a)) return a / r.d;
+    const double q0 = a * r.y;
+    const double q1 = __fma_rn(__fma_rn(-r.d, q0, a), r.y, q0);
+    return __fma_rn(__fma_rn(-r.d, q1, a), r.y, q1);
 }
 
-// RHS of the fluid rows (1sub-momentum.F90:313-360) and dmax = max |DR1|
-__global__ void __launch_bounds__(kAsmBlock) k_rhs(GridIdx g, int mnoe, const int* __restrict__ mno2mn,
+// RHS of the fluid rows (1sub-momentum.F90:313-360) and dmax = max |DR1|, with renzoku_fv
+// (lib/src/math_func.F90:51-54).  Nothing when there are fewer than 10 rows, or no
+// room for the reference's 64 spare ones.
+//
+// What bounds it: seven FP64 divisions per row, on a pipe that does 1.7 lane operations
+// per clock and SM, were most of its 460 us at 2.8 M rows (0.28 GB of traffic, 41 us).
+// The divisors dx, dy, dz and dt are few: their reciprocals come from a table (dx: one
+// per index and axis, in shared memory, TAB) and Markstein's method; 1 - f and its
+// division by dt drop out where f is 1, the division by a porosity of 1 too, and the
+// quotient that is only compared with 1e-15 is formed only near that bound.
+template <bool TAB>
+__global__ void __launch_bounds__(kAsmBlock, 3) k_rhs(GridIdx g, int mm2, const int* __restrict__ mnoe_p,
+                                                  const int* __restrict__ mno2mn,
                                                   const int* __restrict__ mn, const int* __restrict__ in_,
                                                   const int* __restrict__ jn, const int* __restrict__ kn,
                                                   const int* __restrict__ nf, const double* __restrict__ f,
@@ -153,36 +260,78 @@ __global__ void __launch_bounds__(kAsmBlock) k_rhs(GridIdx g, int mnoe, const in
                                                   const double* __restrict__ un, const double* __restrict__ dx,
                                                   const double* __restrict__ mp_p, double dt,
                                                   double* __restrict__ b, unsigned long long* dmax_bits) {
+    extern __shared__ double recip[];                   // 1 / dx(l, i), i = ls - 1 .. le + 1, axis after axis
+    __shared__ long long s_max[kAsmBlock / 32];
+    const int mnoe = *mnoe_p;
+    if (mnoe < 10 || mnoe + 64 > mm2) return;
+    const int nx = g.ie - g.is + 3, ny = g.je - g.js + 3, nz = g.ke - g.ks + 3;
+    const int at[3] = {1 - g.is, nx + 1 - g.js, nx + ny + 1 - g.ks};
+    if (TAB) {
+        for (int t = threadIdx.x; t < nx + ny + nz; t += blockDim.x) {
+            const int l = t < nx ? 0 : t < nx + ny ? 1 : 2;
+            recip[t] = 1.0 / dx[g.dxo(l, t - at[l])];
+        }
+        __syncthreads();
+    }
     const double mp = *mp_p;
-    double local = 0.0;
+    const bool forward = dt > 0.0;
+    const Recip rdt = make_recip(dt);
+    const long long near = __double_as_longlong(1.001e-15 * fabs(dt));
+    long long local = 0;                                // bits of max |DR1|: they order like the values
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < mnoe; t += (long)gridDim.x * blockDim.x) {
         const int c = mno2mn[t];
         if (nf[c] != 1) continue;
         const int i = in_[c], j = jn[c], k = kn[c];
-        const double ff = fmax(-0.001, fmin(1.0 - f[c], 0.001));
+        const double fc = f[c], fbc = fb[c];
         double rz;
-        if (fb[c] != 0.0) {
+        if (!is_zero(fbc)) {
             const int ip = mn[g.mn_off(i + 1, k, j)], jp = mn[g.mn_off(i, k, j + 1)], kp = mn[g.mn_off(i, k + 1, j)];
-            rz = renzoku_fv(a[3L * ip + 0], a[3L * c + 0], a[3L * jp + 1], a[3L * c + 1], a[3L * kp + 2], a[3L * c + 2],
-                            un[3L * ip + 0], un[3L * c + 0], un[3L * jp + 1], un[3L * c + 1], un[3L * kp + 2],
-                            un[3L * c + 2], dx[g.dxo(0, i)], dx[g.dxo(1, j)], dx[g.dxo(2, k)], fb[c]);
+            auto flux = [&](int cell, int l) {              // u a, with most faces fully open
+                const double u = un[3L * cell + l], ar = a[3L * cell + l];
+                return is_one(ar) ? u : u * ar;
+            };
+            const double qx = flux(ip, 0) - flux(c, 0);
+            const double qy = flux(jp, 1) - flux(c, 1);
+            const double qz = flux(kp, 2) - flux(c, 2);
+            if (TAB) {
+                auto rec = [&](int l, int q) {
+                    const double d = dx[g.dxo(l, q)];
+                    return Recip{d, recip[at[l] + q], mid_exponent(d)};
+                };
+                rz = div_by(qx, rec(0, i)) + div_by(qy, rec(1, j)) + div_by(qz, rec(2, k));
+            } else {
+                rz = qx / dx[g.dxo(0, i)] + qy / dx[g.dxo(1, j)] + qz / dx[g.dxo(2, k)];
+            }
+            if (!is_one(fbc)) rz = rz / fbc;
         } else {
             rz = -10000.0;
         }
-        const double dr1 = rz + ff / dt;
-        const double q = dr1 / dt;
-        if (!(fabs(q) <= 1.0e-15 && fabs(q) != 0.0)) b[t] = mp * dr1 / dt;
-        const double ad = fabs(dr1);
-        if (ad > local) local = ad;
+        double src = 0.0;
+        if (!(is_one(fc) && forward)) src = div_by(fmax(-0.001, fmin(1.0 - fc, 0.001)), rdt);
+        const double dr1 = rz + src;
+        const long long ad = __double_as_longlong(fabs(dr1));
+        bool put = true;
+        if (!(ad > near)) {
+            const double q = dr1 / dt;
+            put = !(fabs(q) <= 1.0e-15 && fabs(q) != 0.0);
+        }
+        if (put) b[t] = div_by(mp * dr1, rdt);
+        if (ad > local && ad <= 0x7ff0000000000000LL) local = ad;     // not a NaN
     }
-    // |DR1| >= 0: the IEEE bit pattern orders like the value
-    for (int o = 16; o > 0; o >>= 1) local = fmax(local, __shfl_xor_sync(0xffffffffu, local, o));
-    if ((threadIdx.x & 31) == 0 && local > 0.0) atomicMax(dmax_bits, (unsigned long long)__double_as_longlong(local));
+    for (int o = 16; o > 0; o >>= 1) local = max(local, __shfl_xor_sync(0xffffffffu, local, o));
+    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = local;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kAsmBlock / 32; w++) local = max(local, s_max[w]);
+        if (local > 0) atomicMax(dmax_bits, (unsigned long long)local);
+    }
 }
 
 // ---------------------------------------------------------------------------
 // cal_matrix_element (1sub-momentum.F90:465-551), NORMAL build, one thread per
-// fluid-list entry.
+// fluid-list entry.  Latency-bound (three levels of dependent gathers per column), so
+// the columns' loads are issued together, level by level: 229 us before at 2.8 M rows.
+template <int NL>
 __global__ void __launch_bounds__(kAsmBlock) k_assemble(GridIdx g, int ifln, long inne, long na, long spld,
                                                        const int* __restrict__ fln, const int* __restrict__ in_,
                                                        const int* __restrict__ jn, const int* __restrict__ kn,
@@ -196,10 +345,17 @@ __global__ void __launch_bounds__(kAsmBlock) k_assemble(GridIdx g, int ifln, lon
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < ifln; t += (long)gridDim.x * blockDim.x) {
         const int nnn = fln[t];
         const int i = in_[nnn], j = jn[nnn], k = kn[nnn];
+        const int fl = nf[nnn];
+        int lc[NL], np[NL], fn[NL];
+        double ac[NL];
+#pragma unroll
+        for (int c = 0; c < NL; c++) {
+            lc[c] = nnn <= inne ? ll_c[c * inne + (nnn - 1)] : 0;
+            ac[c] = nnn <= inne ? alu_c[c * inne + (nnn - 1)] : 0.0;
+        }
         const int nn = mno[g.mno_off(i, k, j)];
         if (nn == 0) continue;
         const long r = nn - 1;
-        const int fl = nf[nnn];
         double dd;
         if (fl == 1) {
             dd = de_c[nnn - 1];
@@ -209,34 +365,34 @@ __global__ void __launch_bounds__(kAsmBlock) k_assemble(GridIdx g, int ifln, lon
             atomicCAS(err, 0, nnn);
             continue;
         }
+#pragma unroll
+        for (int c = 0; c < NL; c++) {
+            fn[c] = 0;
+            np[c] = 0;
+            if (lc[c] != 0) {
+                fn[c] = nf[lc[c]];
+                np[c] = mno[g.mno_off(in_[lc[c]], kn[lc[c]], jn[lc[c]])];
+            }
+        }
         const int bl = nfb[nnn];
         const int axis = (bl < 0 ? -bl : bl) - 1;
-        const int nl = g.nl();
-        for (int ll = 1; ll <= nl; ll++) {
-            const long oc = (long)(ll - 1) * inne + (nnn - 1);
-            const long o = (long)(ll - 1) * na + r;
-            const int lc = ll_c[oc];
-            if (lc == 0) {
+#pragma unroll
+        for (int c = 0; c < NL; c++) {
+            const long o = c * na + r;
+            if (lc[c] == 0 || fn[c] == 0 || np[c] == 0) {
                 llu[o] = 0;
                 alu[o] = 0.0;
+                if (lc[c] != 0 && fl == 1 && fn[c] != 2) dd = dd + ac[c];
                 continue;
             }
-            const int np = mno[g.mno_off(in_[lc], kn[lc], jn[lc])];
-            const int fn = nf[lc];
-            if (fn == 0 || np == 0) {
-                llu[o] = 0;
-                alu[o] = 0.0;
-                if (fl == 1 && fn != 2) dd = dd + alu_c[oc];
-                continue;
-            }
-            llu[o] = np;
+            llu[o] = np[c];
             if (fl == 1) {
-                alu[o] = alu_c[oc];
+                alu[o] = ac[c];
             } else {
-                const int l = g.col_axis((ll - 1) / 2);    // 2DV: past the collapsed axis (517-520)
+                const int l = g.col_axis(c / 2);           // 2DV: past the collapsed axis (517-520)
                 if (axis == l) {
                     const int ii = (l == 0) ? i : (l == 1) ? j : k;
-                    const int md = ll % 2;
+                    const int md = (c + 1) % 2;
                     const double fss = (double)(1 - 2 * md) * (x[g.dxo(l, ii - md + 1)] - sp[nnn + spld * l]) / dx[g.dxo(l, ii)];
                     alu[o] = cal_alu(fss, dx[g.dxo(l, ii)], dx[g.dxo(l, ii - 2 * md + 1)]);
                 } else {
@@ -334,14 +490,38 @@ extern "C" int clowns_init_matrix_dev(const int* dims, int inne, int mx2, const 
     // 2DV: x and z when one cell wide in y, y and z when one cell wide in x
     const int axes = g.ie == g.is + 1 ? 6 : g.je == g.js + 1 ? 5 : 7;
     k_min_dx<<<1, 256, 0, s>>>(dx, 3 * mx2, axes, mp);
-    k_init_matrix<<<grid_for(inne), kAsmBlock, 0, s>>>(g, inne, mn, in_, jn, kn, nf, nfb, a, fb, dx, mp, alu_c,
-                                                       ll_c, de_c);
+    const int entries = (g.ie - g.is + 3) + (g.je - g.js + 3) + (g.ke - g.ks + 3);
+    const size_t tab = sizeof(double) * 4 * (size_t)entries;
+    auto launch = [&](auto kern, size_t smem) {
+        const int blocks = (int)std::min<long>((inne + kInitBlock - 1L) / kInitBlock, smem ? 152L * 2 : 152L * 16);
+        kern<<<blocks, kInitBlock, smem, s>>>(g, inne, mx2, mn, in_, jn, kn, nf, nfb, a, fb, dx, mp, alu_c, ll_c, de_c);
+    };
+    // the table fits the shared memory every launch may have up to 1536 cells in i + j + k
+    if (tab <= 48 * 1024) {
+        if (g.nl() == 6) launch(k_init_matrix<6, true>, tab);
+        else launch(k_init_matrix<4, true>, tab);
+    } else {
+        if (g.nl() == 6) launch(k_init_matrix<6, false>, 0);
+        else launch(k_init_matrix<4, false>, 0);
+    }
     CLOWNS_CUDA_TRY(cudaGetLastError());
     return CLOWNS_OK;
 }
 
+namespace clowns {
+// What the row and right-hand-side kernels hand to the host.
+struct RowsOut {
+    unsigned long long dmax_bits;
+    int mnoe, pad;
+};
+}  // namespace clowns
+
+// Workspace: the row mask (a word per 32 list entries, whole tiles), the tiles' counts
+// and what goes to the host.
+static size_t rows_tiles(int ifln) { return ((size_t)(ifln > 0 ? ifln : 1) + kBitTile - 1) / kBitTile; }
+
 extern "C" size_t clowns_rows_rhs_workspace_bytes(int ifln) {
-    return scan_workspace_bytes(ifln) + align_up(sizeof(int) * (size_t)(ifln + 1), 256) * 2 + 256;
+    return align_up(sizeof(unsigned) * 32 * rows_tiles(ifln), 256) + align_up(sizeof(int) * rows_tiles(ifln), 256) + 256;
 }
 
 extern "C" int clowns_rows_rhs_dev(const int* dims, int inne2, int mx2, const int* mn, const int* in_,
@@ -364,54 +544,50 @@ extern "C" int clowns_rows_rhs_dev(const int* dims, int inne2, int mx2, const in
     cudaStream_t s = (cudaStream_t)stream;
     GridIdx g = GridIdx::make(dims);
     char* wb = (char*)work;
-    int* keep = (int*)wb;
-    wb += align_up(sizeof(int) * (size_t)(ifln + 1), 256);
-    int* pos = (int*)wb;
-    wb += align_up(sizeof(int) * (size_t)(ifln + 1), 256);
-    unsigned long long* dmax_bits = (unsigned long long*)wb;
-    wb += 256;
-    void* scan_tmp = wb;
+    unsigned* mask = (unsigned*)wb;
+    wb += align_up(sizeof(unsigned) * 32 * rows_tiles(ifln), 256);
+    int* sums = (int*)wb;
+    wb += align_up(sizeof(int) * rows_tiles(ifln), 256);
+    RowsOut* out = (RowsOut*)wb;
     // 1sub-momentum.F90:267-271 and 276
     CLOWNS_CUDA_TRY(cudaMemsetAsync(b, 0, sizeof(double) * mm2, s));
     CLOWNS_CUDA_TRY(cudaMemsetAsync(xe, 0, sizeof(double) * mm2, s));
     CLOWNS_CUDA_TRY(cudaMemsetAsync(de, 0, sizeof(double) * mm2, s));
     CLOWNS_CUDA_TRY(cudaMemsetAsync(mno, 0, sizeof(int) * (size_t)g.ie * g.ke * g.je, s));
-    CLOWNS_CUDA_TRY(cudaMemsetAsync(dmax_bits, 0, sizeof(unsigned long long), s));
-    int mnoe = 0;
+    CLOWNS_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(RowsOut), s));
     if (ifln > 0) {
-        k_row_flags<<<grid_for(ifln), kAsmBlock, 0, s>>>(g, ifln, fln, mn, in_, jn, kn, nf, nfb, fb, keep);
-        int rc = exclusive_scan_dev(keep, pos, ifln, pos + ifln, scan_tmp, s);
+        // rows, right-hand side and their count in one pass over the stream: the kernels
+        // take the count from the device, the host reads it with dmax at the end
+        const int tiles = (int)rows_tiles(ifln);
+        k_row_flags<<<tiles, kBitThreads, 0, s>>>(g, ifln, fln, mn, in_, jn, kn, nf, nfb, fb, mask, sums);
+        int rc = scan_tiles_dev(1, sums, ifln, nullptr, &out->mnoe, s);
         if (rc) return rc;
-        CLOWNS_CUDA_TRY(cudaMemcpyAsync(&mnoe, pos + ifln, sizeof(int), cudaMemcpyDeviceToHost, s));
-        CLOWNS_CUDA_TRY(cudaStreamSynchronize(s));
-        if (mnoe > mm2) {
-            set_last_error_msg("rows_rhs: mm2 smaller than the number of rows");
-            return CLOWNS_ERR_ARG;
-        }
-        k_row_scatter<<<grid_for(ifln), kAsmBlock, 0, s>>>(g, ifln, fln, in_, jn, kn, keep, pos, mno, mno2mn);
-    }
-    *mnoe_out = mnoe;
-    if (dmax_out) *dmax_out = 0.0;
-    if (mnoe < 10) {                                // 1sub-momentum.F90:297-300
+        k_row_scatter<<<tiles, kBitThreads, 0, s>>>(g, ifln, mm2, fln, in_, jn, kn, mask, sums, mno, mno2mn);
+        // the reciprocals leave three blocks per SM their shared memory up to 3072 cells in i + j + k
+        const int entries = (g.ie - g.is + 3) + (g.je - g.js + 3) + (g.ke - g.ks + 3);
+        auto rhs = [&](auto kern, size_t smem, int nb) {
+            kern<<<nb, kAsmBlock, smem, s>>>(g, mm2, &out->mnoe, mno2mn, mn, in_, jn, kn, nf, f, fb, a, un, dx, mp, dt, b,
+                                             &out->dmax_bits);
+        };
+        if (entries <= 3072) rhs(k_rhs<true>, sizeof(double) * entries, std::min(grid_for(ifln), 152 * 3));
+        else rhs(k_rhs<false>, 0, grid_for(ifln));
         CLOWNS_CUDA_TRY(cudaGetLastError());
-        CLOWNS_CUDA_TRY(cudaStreamSynchronize(s));
-        return CLOWNS_OK;
     }
-    if (mnoe + 64 > mm2) {                          // the reference re-allocates (302-310)
+    RowsOut h = {};
+    CLOWNS_CUDA_TRY(cudaMemcpyAsync(&h, out, sizeof(h), cudaMemcpyDeviceToHost, s));
+    CLOWNS_CUDA_TRY(cudaStreamSynchronize(s));
+    if (h.mnoe > mm2) {
+        set_last_error_msg("rows_rhs: mm2 smaller than the number of rows");
+        return CLOWNS_ERR_ARG;
+    }
+    *mnoe_out = h.mnoe;
+    if (dmax_out) *dmax_out = 0.0;
+    if (h.mnoe < 10) return CLOWNS_OK;              // 1sub-momentum.F90:297-300
+    if (h.mnoe + 64 > mm2) {                        // the reference re-allocates (302-310)
         set_last_error_msg("rows_rhs: mm2 must exceed the number of rows by at least 64");
         return CLOWNS_ERR_ARG;
     }
-    k_rhs<<<grid_for(mnoe), kAsmBlock, 0, s>>>(g, mnoe, mno2mn, mn, in_, jn, kn, nf, f, fb, a, un, dx, mp, dt, b,
-                                              dmax_bits);
-    CLOWNS_CUDA_TRY(cudaGetLastError());
-    if (dmax_out) {
-        unsigned long long bits = 0;
-        CLOWNS_CUDA_TRY(cudaMemcpyAsync(&bits, dmax_bits, sizeof(bits), cudaMemcpyDeviceToHost, s));
-        CLOWNS_CUDA_TRY(cudaStreamSynchronize(s));
-        double v;
-        memcpy(&v, &bits, sizeof(v));
-        *dmax_out = v;
-    }
+    if (dmax_out) memcpy(dmax_out, &h.dmax_bits, sizeof(double));
     return CLOWNS_OK;
 }
 
@@ -435,9 +611,9 @@ extern "C" int clowns_assemble_dev(const int* dims, int inne, int inne2, int mx2
     GridIdx g = GridIdx::make(dims);
     CLOWNS_CUDA_TRY(cudaMemsetAsync(err_cell, 0, sizeof(int), s));
     if (ifln > 0)
-        k_assemble<<<grid_for(ifln), kAsmBlock, 0, s>>>(g, ifln, inne, mm2, (long)inne2 + 2, fln, in_, jn, kn, nf,
-                                                        nfb, x, dx, sp, mno, alu_c, ll_c, de_c, alu, llu, de,
-                                                        err_cell);
+        (g.nl() == 6 ? k_assemble<6> : k_assemble<4>)<<<grid_for(ifln), kAsmBlock, 0, s>>>(
+            g, ifln, inne, mm2, (long)inne2 + 2, fln, in_, jn, kn, nf, nfb, x, dx, sp, mno, alu_c, ll_c, de_c, alu, llu,
+            de, err_cell);
     CLOWNS_CUDA_TRY(cudaGetLastError());
     return CLOWNS_OK;
 }

@@ -1,5 +1,5 @@
-// grid_index.cuh -- index arithmetic for the reference's dense arrays, plus a
-// device-wide exclusive scan used to number rows and list cells.
+// grid_index.cuh -- index arithmetic for the reference's dense arrays, plus the
+// compaction of decisions used to number rows and list cells.
 #pragma once
 
 #include "common.cuh"
@@ -61,8 +61,28 @@ inline bool grid_dims_ok(const int* d) {
     return d && d[0] >= 3 && d[1] >= 3 && d[2] >= 3 && d[3] > d[0] && d[4] > d[1] && d[5] > d[2];
 }
 
-// Exclusive scan of n int32 flags/counts: out[t] = sum_{u<t} in[u], *total = sum.
-size_t scan_workspace_bytes(long n);
-int exclusive_scan_dev(const int* in, int* out, long n, int* total, void* tmp, cudaStream_t s);
+// Compaction of n decisions: tiles of kBitTile = 1024 positions by blocks of
+// kBitThreads, position tile * 1024 + 256 round + thread, so that a warp's 32
+// positions are one word of the mask and the tile's 32 words are in position order.
+constexpr int kBitTile = 1024;
+constexpr int kBitThreads = 256;
+constexpr int kBitRounds = kBitTile / kBitThreads;
+
+// Rank of the set bits inside a tile: pre[w] = set bits in the words before word w.
+// Called by one warp.
+__device__ __forceinline__ void bit_prefix(const unsigned* words, int* pre) {
+    const int lane = threadIdx.x & 31;
+    const int c = __popc(words[lane]);
+    int x = c;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    pre[lane] = x - c;
+}
+
+// Exclusive scan of the tiles' counts (`lists` of them, 1 or 2, interleaved) in place
+// and their totals; nt_p: the number of tiles on the device (nullptr: all of n).
+int scan_tiles_dev(int lists, int* sums, long n, const int* nt_p, int* totals, cudaStream_t s);
 
 }  // namespace clowns

@@ -42,21 +42,37 @@ struct NfArgs {
 };
 
 // ---- nfd2015.F90:35-59 --------------------------------------------------
-__global__ void k_vof_flags(NfArgs A, const double* __restrict__ f, int* __restrict__ dec, int* imax_k) {
+// imax_k: the largest i and k of a wet cell, one pair of atomics per block.
+__global__ void __launch_bounds__(kNfBlock) k_vof_flags(NfArgs A, const double* __restrict__ f, int* __restrict__ dec,
+                                                        int* imax_k) {
+    int mi = 0, mk = 0;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < A.inne; t += (long)gridDim.x * blockDim.x) {
         const int nn = (int)t + 1;
         if (A.nf[nn] == -1) { dec[nn] = -1; continue; }
-        const int i = A.in_[nn], j = A.jn[nn], k = A.kn[nn];
+        const int i = A.in_[nn], k = A.kn[nn];
         const double fv = f[nn];
-        const bool air = fv <= 1.0e-12 ||
-                         (fv * A.fb[nn] < 1.0e-3 && A.nf[A.mn[A.g.mn_off(i, k - 1, j)]] == -1 &&
-                          f[A.mn[A.g.mn_off(i, k + 1, j)]] == 0.0);
+        bool air = fv <= 1.0e-12;
+        if (!air && fv * A.fb[nn] < 1.0e-3) {
+            const int j = A.jn[nn];
+            air = A.nf[A.mn[A.g.mn_off(i, k - 1, j)]] == -1 && f[A.mn[A.g.mn_off(i, k + 1, j)]] == 0.0;
+        }
         dec[nn] = air ? 0 : 1;
         if (!air) {
-            atomicMax(imax_k + 0, i);
-            atomicMax(imax_k + 1, k);
+            mi = max(mi, i);
+            mk = max(mk, k);
         }
     }
+    __shared__ int s[2];
+    if (threadIdx.x < 2) s[threadIdx.x] = 0;
+    __syncthreads();
+    mi = __reduce_max_sync(0xffffffffu, mi);
+    mk = __reduce_max_sync(0xffffffffu, mk);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(s, mi);
+        atomicMax(s + 1, mk);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 && s[threadIdx.x] > 0) atomicMax(imax_k + threadIdx.x, s[threadIdx.x]);
 }
 
 __global__ void k_vof_apply(NfArgs A, double* __restrict__ f, const int* __restrict__ dec) {
@@ -70,52 +86,105 @@ __global__ void k_vof_apply(NfArgs A, double* __restrict__ f, const int* __restr
     }
 }
 
-// ---- nfd2015.F90:66-102: wet cells and surface detection over the k,j,i box --
+// Counters shared by the passes, on the device (zeroed before each classification).
+enum { kCtrImax, kCtrKmax, kCtrWet, kCtrSurf, kCtrUnsettled, kCtrPrune, kCtrSweep, kCtrRemoved, kCtrDropped, kCtrCount };
+
+// ---- nfd2015.F90:66-102: wet cells and surface detection over the k,j,i box, whose
+// upper corner follows from the wet cells' largest i and k (kept on the device: the
+// host launches for the largest box, and blocks past the box's tiles return)
 struct Box {
-    int ks, kmax, js, je1, is, imax;
-    long nbi, nbj, nbk, total;
-    __device__ __forceinline__ void ijk(long t, int& i, int& j, int& k) const {
-        i = is + (int)(t % nbi);
-        long r = t / nbi;
-        j = js + (int)(r % nbj);
-        k = ks + (int)(r / nbj);
+    int is, js, ks, ni, nj;
+    long total;
+    __device__ __forceinline__ Box(const GridIdx& g, const int* ctr) {
+        const int imax = min(ctr[kCtrImax] + 1, g.ie - 1), kmax = min(ctr[kCtrKmax] + 1, g.ke - 1);
+        is = g.is; js = g.js; ks = g.ks;
+        ni = max(0, imax - g.is + 1);
+        nj = g.je - g.js;
+        total = (long)ni * nj * max(0, kmax - g.ks + 1);
+    }
+    __device__ __forceinline__ void ijk(unsigned t, int& i, int& j, int& k) const {
+        const unsigned r = t / (unsigned)ni;
+        i = is + (int)(t - r * (unsigned)ni);
+        k = ks + (int)(r / (unsigned)nj);
+        j = js + (int)(r % (unsigned)nj);
     }
 };
 
-__global__ void k_surface_flags(NfArgs A, Box B, int* __restrict__ wet, int* __restrict__ surf) {
-    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < B.total; t += (long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        B.ijk(t, i, j, k);
-        const int nn = A.mn[A.g.mn_off(i, k, j)];
-        const int fl = A.nf[nn];
-        int w = 0, s = 0;
-        if (fl >= 1) {
-            w = 1;
-            for (int l = 0; l < 3 && !s; l++) {
-                const int p = A.mn[A.g.nbr(i, j, k, l, +1)];
-                if (A.nf[p] == 0 && A.a[3L * p + l] > 0.0) s = 1;
-                if (!s) {
-                    const int m = A.mn[A.g.nbr(i, j, k, l, -1)];
-                    if (A.nf[m] == 0 && A.a[3L * nn + l] > 0.0) s = 1;
+// Bit masks of the wet and the surface cells, their counts per tile (pairs).
+__global__ void __launch_bounds__(kBitThreads) k_surface_flags(NfArgs A, const int* __restrict__ ctr,
+                                                               unsigned* __restrict__ wet, unsigned* __restrict__ surf,
+                                                               int* __restrict__ sums) {
+    const Box B(A.g, ctr);
+    const int tile = blockIdx.x;
+    if ((long)tile * kBitTile >= B.total) {
+        if (threadIdx.x < 2) sums[2 * tile + threadIdx.x] = 0;
+        return;
+    }
+    int cw = 0, cs = 0;
+#pragma unroll
+    for (int q = 0; q < kBitRounds; q++) {
+        const long t = (long)tile * kBitTile + q * kBitThreads + threadIdx.x;
+        bool w = false, s = false;
+        if (t < B.total) {
+            int i, j, k;
+            B.ijk((unsigned)t, i, j, k);
+            const int nn = A.mn[A.g.mn_off(i, k, j)];
+            w = A.nf[nn] >= 1;
+            if (w) {
+                for (int l = 0; l < 3 && !s; l++) {
+                    const int p = A.mn[A.g.nbr(i, j, k, l, +1)];
+                    if (A.nf[p] == 0 && A.a[3L * p + l] > 0.0) s = true;
+                    if (!s) {
+                        const int m = A.mn[A.g.nbr(i, j, k, l, -1)];
+                        if (A.nf[m] == 0 && A.a[3L * nn + l] > 0.0) s = true;
+                    }
                 }
             }
         }
-        wet[t] = w;
-        surf[t] = s;
+        const unsigned mw = __ballot_sync(0xffffffffu, w), ms = __ballot_sync(0xffffffffu, s);
+        if ((threadIdx.x & 31) == 0) {
+            wet[t >> 5] = mw;
+            surf[t >> 5] = ms;
+        }
+        cw += __popc(mw);
+        cs += __popc(ms);
     }
+    __shared__ int sum[2];
+    if (threadIdx.x < 2) sum[threadIdx.x] = 0;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(sum, cw);
+        atomicAdd(sum + 1, cs);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) sums[2 * tile + threadIdx.x] = sum[threadIdx.x];
 }
 
-__global__ void k_surface_scatter(NfArgs A, Box B, const int* __restrict__ wet, const int* __restrict__ surf,
-                                  const int* __restrict__ wpos, const int* __restrict__ spos_box,
-                                  int* __restrict__ fln, int* __restrict__ sfn, int* __restrict__ spos_cell) {
-    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < B.total; t += (long)gridDim.x * blockDim.x) {
-        if (!wet[t]) continue;
+__global__ void __launch_bounds__(kBitThreads) k_surface_scatter(NfArgs A, const int* __restrict__ ctr,
+                                                                 const unsigned* __restrict__ wet,
+                                                                 const unsigned* __restrict__ surf,
+                                                                 const int* __restrict__ sums, int* __restrict__ fln,
+                                                                 int* __restrict__ sfn, int* __restrict__ spos_cell) {
+    const Box B(A.g, ctr);
+    const int tile = blockIdx.x;
+    if ((long)tile * kBitTile >= B.total) return;
+    __shared__ int prew[32], pres[32];
+    const unsigned *ww = wet + (long)tile * 32, *sw = surf + (long)tile * 32;
+    if (threadIdx.x < 32) bit_prefix(ww, prew);
+    else if (threadIdx.x < 64) bit_prefix(sw, pres);
+    __syncthreads();
+    const int w0 = sums[2 * tile], s0 = sums[2 * tile + 1];
+#pragma unroll
+    for (int q = 0; q < kBitRounds; q++) {
+        const int word = q * (kBitThreads / 32) + (threadIdx.x >> 5), bit = threadIdx.x & 31;
+        const unsigned mw = ww[word], ms = sw[word], below = (1u << bit) - 1;
+        if (!(mw >> bit & 1)) continue;
         int i, j, k;
-        B.ijk(t, i, j, k);
+        B.ijk((unsigned)((long)tile * kBitTile + q * kBitThreads + threadIdx.x), i, j, k);
         const int nn = A.mn[A.g.mn_off(i, k, j)];
-        fln[wpos[t]] = nn;
-        if (surf[t]) {
-            const int p = spos_box[t];
+        fln[w0 + prew[word] + __popc(mw & below)] = nn;
+        if (ms >> bit & 1) {
+            const int p = s0 + pres[word] + __popc(ms & below);
             sfn[p] = nn;
             spos_cell[nn] = p;
             A.nf[nn] = 2;
@@ -128,19 +197,19 @@ __global__ void k_surface_scatter(NfArgs A, Box B, const int* __restrict__ wet, 
 }
 
 // ---- nfd2015.F90:107-131: first pruning (order-independent) -------------------
+__device__ __forceinline__ int prune1(const NfArgs& A, int nn) {
+    const int i = A.in_[nn], j = A.jn[nn], k = A.kn[nn];
+    if (A.nf[A.mn[A.g.mn_off(i, k - 1, j)]] == -1) return 0;
+    int keep = 0;
+    for (int l = 0; l < 3 && !keep; l++) {
+        if (A.nf[A.mn[A.g.nbr(i, j, k, l, +1)]] == 1) keep = 1;
+        else if (A.nf[A.mn[A.g.nbr(i, j, k, l, -1)]] == 1) keep = 1;
+    }
+    return !keep;
+}
 __global__ void k_prune1(NfArgs A, int isfn, const int* __restrict__ sfn, int* __restrict__ rem, int* count) {
     for (long p = (long)blockIdx.x * blockDim.x + threadIdx.x; p < isfn; p += (long)gridDim.x * blockDim.x) {
-        const int nn = sfn[p];
-        const int i = A.in_[nn], j = A.jn[nn], k = A.kn[nn];
-        int r = 0;
-        if (A.nf[A.mn[A.g.mn_off(i, k - 1, j)]] != -1) {
-            int keep = 0;
-            for (int l = 0; l < 3 && !keep; l++) {
-                if (A.nf[A.mn[A.g.nbr(i, j, k, l, +1)]] == 1) keep = 1;
-                else if (A.nf[A.mn[A.g.nbr(i, j, k, l, -1)]] == 1) keep = 1;
-            }
-            r = !keep;
-        }
+        const int r = prune1(A, sfn[p]);
         rem[p] = r;
         if (r) atomicAdd(count, 1);
     }
@@ -158,10 +227,11 @@ __global__ void k_remove(NfArgs A, int isfn, const int* __restrict__ sfn, const 
 
 // Flag of cell q as seen by list position p in a loop walked from the end of
 // the list: cells later in the list (already visited) show their removal.
+// state == nullptr: nothing removed.
 __device__ __forceinline__ int nf_seen(const NfArgs& A, int q, long p, const int* __restrict__ spos_cell,
                                        const int* __restrict__ state) {
     const int fl = A.nf[q];
-    if (fl == 2) {
+    if (fl == 2 && state) {
         const int pq = spos_cell[q];
         if (pq > p && state[pq]) return 0;
     }
@@ -169,23 +239,24 @@ __device__ __forceinline__ int nf_seen(const NfArgs& A, int q, long p, const int
 }
 
 // ---- nfd2015.F90:133-158: second pruning, serial semantics ---------------------
+__device__ __forceinline__ int prune2(const NfArgs& A, int nn, long p, const int* __restrict__ spos_cell,
+                                      const int* __restrict__ st) {
+    const int i = A.in_[nn], j = A.jn[nn], k = A.kn[nn];
+    const int below = nf_seen(A, A.mn[A.g.mn_off(i, k - 1, j)], p, spos_cell, st);
+    const int above = nf_seen(A, A.mn[A.g.mn_off(i, k + 1, j)], p, spos_cell, st);
+    if (below == -1 && above == 0) return 0;
+    int keep = 0;
+    for (int l = 0; l < 3 && !keep; l++) {
+        const int pv = nf_seen(A, A.mn[A.g.nbr(i, j, k, l, +1)], p, spos_cell, st);
+        const int mv = nf_seen(A, A.mn[A.g.nbr(i, j, k, l, -1)], p, spos_cell, st);
+        if ((pv == 1 && mv == 0) || (mv == 1 && pv == 0)) keep = 1;
+    }
+    return !keep;
+}
 __global__ void k_prune2_sweep(NfArgs A, int isfn, const int* __restrict__ sfn, const int* __restrict__ spos_cell,
                                const int* __restrict__ st_in, int* __restrict__ st_out, int* changed) {
     for (long p = (long)blockIdx.x * blockDim.x + threadIdx.x; p < isfn; p += (long)gridDim.x * blockDim.x) {
-        const int nn = sfn[p];
-        const int i = A.in_[nn], j = A.jn[nn], k = A.kn[nn];
-        int r = 0;
-        const int below = nf_seen(A, A.mn[A.g.mn_off(i, k - 1, j)], p, spos_cell, st_in);
-        const int above = nf_seen(A, A.mn[A.g.mn_off(i, k + 1, j)], p, spos_cell, st_in);
-        if (!(below == -1 && above == 0)) {
-            int keep = 0;
-            for (int l = 0; l < 3 && !keep; l++) {
-                const int pv = nf_seen(A, A.mn[A.g.nbr(i, j, k, l, +1)], p, spos_cell, st_in);
-                const int mv = nf_seen(A, A.mn[A.g.nbr(i, j, k, l, -1)], p, spos_cell, st_in);
-                if ((pv == 1 && mv == 0) || (mv == 1 && pv == 0)) keep = 1;
-            }
-            r = !keep;
-        }
+        const int r = prune2(A, sfn[p], p, spos_cell, st_in);
         st_out[p] = r;
         if (r != st_in[p]) atomicAdd(changed, 1);
     }
@@ -216,58 +287,89 @@ __device__ double fxx1_dev(const NfArgs& A, const double* __restrict__ f, int ix
 }
 
 // ---- nfd2015.F90:163-244: orientation, serial semantics ------------------------
+// Orientation b of list position p; true when the cell has none and becomes air.
+__device__ __forceinline__ bool orient(const NfArgs& A, const double* __restrict__ f, int nn, long p,
+                                       const int* __restrict__ spos_cell, const int* __restrict__ st_in, int& b) {
+    const int i = A.in_[nn], j = A.jn[nn], k = A.kn[nn];
+    int ix[3] = {0, 0, 0};
+    for (int l = 0; l < 3; l++) {
+        const int m = A.mn[A.g.nbr(i, j, k, l, -1)], pc = A.mn[A.g.nbr(i, j, k, l, +1)];
+        const int mv = nf_seen(A, m, p, spos_cell, st_in), pv = nf_seen(A, pc, p, spos_cell, st_in);
+        if (mv == 1 && pv == 0 && A.a[3L * pc + l] > 0.0) ix[l] = -1;
+        else if (mv == 0 && pv == 1 && A.a[3L * nn + l] > 0.0) ix[l] = 1;
+    }
+    if (abs(ix[0]) + abs(ix[1]) + abs(ix[2]) == 0) {
+        const int below = nf_seen(A, A.mn[A.g.mn_off(i, k - 1, j)], p, spos_cell, st_in);
+        const int above = nf_seen(A, A.mn[A.g.mn_off(i, k + 1, j)], p, spos_cell, st_in);
+        if (below == -1 && above == 0) {
+            if (A.objno[nn] != 0 || A.fb[nn] != 0.0) {
+                ix[2] = -1;
+            } else {
+                for (int l = 0; l <= 1; l++) {
+                    const int m = A.mn[A.g.nbr(i, j, k, l, -1)], pc = A.mn[A.g.nbr(i, j, k, l, +1)];
+                    const int mv = nf_seen(A, m, p, spos_cell, st_in), pv = nf_seen(A, pc, p, spos_cell, st_in);
+                    if (mv > 0 && pv == 0 && A.a[3L * pc + l] > 0.0) ix[l] = -1;
+                    else if (mv == 0 && pv > 0 && A.a[3L * nn + l] > 0.0) ix[l] = 1;
+                }
+                if (abs(ix[0]) + abs(ix[1]) == 0) ix[2] = -1;
+            }
+        }
+    }
+    const int s = abs(ix[0]) + abs(ix[1]) + abs(ix[2]);
+    int g = 0;
+    b = 0;
+    if (s == 1) {
+        int dir = 1, best = abs(ix[0]);
+        for (int l = 1; l <= 2; l++)
+            if (abs(ix[l]) > best) { best = abs(ix[l]); dir = l + 1; }
+        b = dir * ix[dir - 1];
+    } else if (s == 0) {
+        g = 1;
+    } else {
+        double fx[3];
+        for (int l = 0; l < 3; l++) fx[l] = ix[l] == 0 ? 0.0 : fxx1_dev(A, f, ix[l], l, i, j, k);
+        int dir = 1;
+        double best = fx[0];
+        for (int l = 1; l <= 2; l++)
+            if (fx[l] > best) { best = fx[l]; dir = l + 1; }
+        b = dir * ix[dir - 1];
+    }
+    return g != 0;
+}
 __global__ void k_orient_sweep(NfArgs A, const double* __restrict__ f, int isfn, const int* __restrict__ sfn,
                                const int* __restrict__ spos_cell, const int* __restrict__ st_in,
                                int* __restrict__ st_out, int* __restrict__ bout, int* changed) {
     for (long p = (long)blockIdx.x * blockDim.x + threadIdx.x; p < isfn; p += (long)gridDim.x * blockDim.x) {
-        const int nn = sfn[p];
-        const int i = A.in_[nn], j = A.jn[nn], k = A.kn[nn];
-        int ix[3] = {0, 0, 0};
-        for (int l = 0; l < 3; l++) {
-            const int m = A.mn[A.g.nbr(i, j, k, l, -1)], pc = A.mn[A.g.nbr(i, j, k, l, +1)];
-            const int mv = nf_seen(A, m, p, spos_cell, st_in), pv = nf_seen(A, pc, p, spos_cell, st_in);
-            if (mv == 1 && pv == 0 && A.a[3L * pc + l] > 0.0) ix[l] = -1;
-            else if (mv == 0 && pv == 1 && A.a[3L * nn + l] > 0.0) ix[l] = 1;
-        }
-        if (abs(ix[0]) + abs(ix[1]) + abs(ix[2]) == 0) {
-            const int below = nf_seen(A, A.mn[A.g.mn_off(i, k - 1, j)], p, spos_cell, st_in);
-            const int above = nf_seen(A, A.mn[A.g.mn_off(i, k + 1, j)], p, spos_cell, st_in);
-            if (below == -1 && above == 0) {
-                if (A.objno[nn] != 0 || A.fb[nn] != 0.0) {
-                    ix[2] = -1;
-                } else {
-                    for (int l = 0; l <= 1; l++) {
-                        const int m = A.mn[A.g.nbr(i, j, k, l, -1)], pc = A.mn[A.g.nbr(i, j, k, l, +1)];
-                        const int mv = nf_seen(A, m, p, spos_cell, st_in), pv = nf_seen(A, pc, p, spos_cell, st_in);
-                        if (mv > 0 && pv == 0 && A.a[3L * pc + l] > 0.0) ix[l] = -1;
-                        else if (mv == 0 && pv > 0 && A.a[3L * nn + l] > 0.0) ix[l] = 1;
-                    }
-                    if (abs(ix[0]) + abs(ix[1]) == 0) ix[2] = -1;
-                }
-            }
-        }
-        const int s = abs(ix[0]) + abs(ix[1]) + abs(ix[2]);
-        int g = 0, b = 0;
-        if (s == 1) {
-            int dir = 1, best = abs(ix[0]);
-            for (int l = 1; l <= 2; l++)
-                if (abs(ix[l]) > best) { best = abs(ix[l]); dir = l + 1; }
-            b = dir * ix[dir - 1];
-        } else if (s == 0) {
-            g = 1;
-        } else {
-            double fx[3];
-            for (int l = 0; l < 3; l++) fx[l] = ix[l] == 0 ? 0.0 : fxx1_dev(A, f, ix[l], l, i, j, k);
-            int dir = 1;
-            double best = fx[0];
-            for (int l = 1; l <= 2; l++)
-                if (fx[l] > best) { best = fx[l]; dir = l + 1; }
-            b = dir * ix[dir - 1];
-        }
+        int b;
+        const int g = orient(A, f, sfn[p], p, spos_cell, st_in, b);
         st_out[p] = g;
         bout[p] = b;
         if (g != st_in[p]) atomicAdd(changed, 1);
     }
+}
+
+// The three loops at once for a surface that none of them changes, the usual case:
+// the first pruning removes nothing, and a first sweep of the second and of the
+// orientation from "nothing removed" finds nothing to remove either, so each has
+// settled.  ctr[kCtrUnsettled] counts the positions where that fails; they leave all
+// flags as they were and the loops run one by one.
+__global__ void k_surface_check(NfArgs A, const double* __restrict__ f, const int* __restrict__ sfn,
+                                const int* __restrict__ spos_cell, int* __restrict__ bout, int* ctr) {
+    const int isfn = ctr[kCtrSurf];
+    int bad = 0;
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < isfn; p += gridDim.x * blockDim.x) {
+        const int nn = sfn[p];
+        int b = 0;
+        bad |= prune1(A, nn) || prune2(A, nn, p, spos_cell, nullptr) || orient(A, f, nn, p, spos_cell, nullptr, b);
+        bout[p] = b;
+    }
+    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicAdd(ctr + kCtrUnsettled, 1);
+}
+__global__ void k_surface_settle(NfArgs A, const int* __restrict__ sfn, const int* __restrict__ bout,
+                                 const int* __restrict__ ctr) {
+    if (ctr[kCtrUnsettled]) return;
+    const int isfn = ctr[kCtrSurf];
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < isfn; p += gridDim.x * blockDim.x) A.nfb[sfn[p]] = bout[p];
 }
 
 __global__ void k_orient_apply(NfArgs A, int isfn, const int* __restrict__ sfn, const int* __restrict__ st,
@@ -293,40 +395,41 @@ __global__ void k_fill(int* p, long n, int v) {
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) p[t] = v;
 }
 
-// Workspace: box-sized flag and position arrays, the per-cell list position,
-// the Jacobi state buffers and scan scratch.
+// Workspace: the wet and surface masks with their tiles' counts, the per-cell list
+// position and the per-position states of the surface loops.
 struct NfWs {
-    int *wet, *surf, *wpos, *spos_box, *spos_cell, *st0, *st1, *bout, *ctr;
-    void* scan_tmp;
+    unsigned *wet, *surf;
+    int *sums, *spos_cell, *st0, *st1, *bout, *ctr;
 };
 
+static size_t nf_box(const int* dims) {
+    const GridIdx g = GridIdx::make(dims);
+    const long box = (long)(g.ie - g.is) * (g.je - g.js) * (g.ke - g.ks);
+    return box < 1 ? 1 : (size_t)box;
+}
+static size_t nf_tiles(const int* dims) { return (nf_box(dims) + kBitTile - 1) / kBitTile; }
+
 static size_t nf_layout(const int* dims, int inne2, NfWs* w, char* base) {
-    GridIdx g = GridIdx::make(dims);
-    long box = (long)(g.ie - g.is) * (g.je - g.js) * (g.ke - g.ks);
-    if (box < 1) box = 1;
+    const size_t box = nf_box(dims), tiles = nf_tiles(dims);
     size_t o = 0;
     auto take = [&](size_t bytes) { size_t at = o; o = align_up(o + bytes, 256); return at; };
-    size_t o_wet = take(sizeof(int) * (box + 1));
-    size_t o_surf = take(sizeof(int) * (box + 1));
-    size_t o_wpos = take(sizeof(int) * (box + 1));
-    size_t o_spos = take(sizeof(int) * (box + 1));
-    size_t o_cell = take(sizeof(int) * ((size_t)inne2 + 2));
-    size_t o_st0 = take(sizeof(int) * (box + 1));
-    size_t o_st1 = take(sizeof(int) * (box + 1));
-    size_t o_b = take(sizeof(int) * (box + 1));
-    size_t o_ctr = take(sizeof(int) * 16);
-    size_t o_scan = take(scan_workspace_bytes(box + 1));
+    const size_t o_wet = take(sizeof(unsigned) * 32 * tiles);
+    const size_t o_surf = take(sizeof(unsigned) * 32 * tiles);
+    const size_t o_sums = take(sizeof(int) * 2 * tiles);
+    const size_t o_cell = take(sizeof(int) * ((size_t)inne2 + 2));
+    const size_t o_st0 = take(sizeof(int) * box);
+    const size_t o_st1 = take(sizeof(int) * box);
+    const size_t o_b = take(sizeof(int) * box);
+    const size_t o_ctr = take(sizeof(int) * 16);
     if (w && base) {
-        w->wet = (int*)(base + o_wet);
-        w->surf = (int*)(base + o_surf);
-        w->wpos = (int*)(base + o_wpos);
-        w->spos_box = (int*)(base + o_spos);
+        w->wet = (unsigned*)(base + o_wet);
+        w->surf = (unsigned*)(base + o_surf);
+        w->sums = (int*)(base + o_sums);
         w->spos_cell = (int*)(base + o_cell);
         w->st0 = (int*)(base + o_st0);
         w->st1 = (int*)(base + o_st1);
         w->bout = (int*)(base + o_b);
         w->ctr = (int*)(base + o_ctr);
-        w->scan_tmp = base + o_scan;
     }
     return o;
 }
@@ -371,23 +474,11 @@ extern "C" int clowns_set_nflag_dev(const int* dims, int inne, int inne2, int mx
     A.mn = mn; A.in_ = in_; A.jn = jn; A.kn = kn; A.nf = nf; A.nfb = nfb;
     A.fb = fb; A.a = a; A.dx = dx; A.objno = objno;
 
-    // VOF pass; W.wet doubles as the per-cell decision array here (size >= inne2+2
-    // is not guaranteed, so use spos_cell which is).
+    // VOF pass (spos_cell holds the per-cell decisions until the lists are numbered)
     CLOWNS_CUDA_TRY(cudaMemsetAsync(W.ctr, 0, sizeof(int) * 16, s));
     k_vof_flags<<<nf_grid(inne), kNfBlock, 0, s>>>(A, f, W.spos_cell, W.ctr);
     k_vof_apply<<<nf_grid(inne), kNfBlock, 0, s>>>(A, f, W.spos_cell);
-    int ik[2];
-    CLOWNS_CUDA_TRY(cudaMemcpyAsync(ik, W.ctr, sizeof(int) * 2, cudaMemcpyDeviceToHost, s));
-    CLOWNS_CUDA_TRY(cudaStreamSynchronize(s));
-    const GridIdx& g = A.g;
-    int imax = ik[0] + 1 < g.ie - 1 ? ik[0] + 1 : g.ie - 1;
-    int kmax = ik[1] + 1 < g.ke - 1 ? ik[1] + 1 : g.ke - 1;
-    Box B;
-    B.ks = g.ks; B.kmax = kmax; B.js = g.js; B.je1 = g.je - 1; B.is = g.is; B.imax = imax;
-    B.nbi = imax >= g.is ? imax - g.is + 1 : 0;
-    B.nbj = g.je - g.js;
-    B.nbk = kmax >= g.ks ? kmax - g.ks + 1 : 0;
-    B.total = B.nbi * B.nbj * B.nbk;
+    const int tiles = (int)nf_tiles(dims);
 
     int passes = 0, ifln = 0, isfn = 0;
     const int kMaxPasses = 100000;
@@ -396,30 +487,26 @@ extern "C" int clowns_set_nflag_dev(const int* dims, int inne, int inne2, int mx
             set_last_error_msg("set_nflag: classification did not settle");
             return CLOWNS_ERR_NOCONV;
         }
-        ifln = 0;
-        isfn = 0;
-        if (B.total > 0) {
-            const int gb = nf_grid(B.total);
-            k_surface_flags<<<gb, kNfBlock, 0, s>>>(A, B, W.wet, W.surf);
-            int rc = exclusive_scan_dev(W.wet, W.wpos, B.total, W.ctr + 2, W.scan_tmp, s);
-            if (rc) return rc;
-            rc = exclusive_scan_dev(W.surf, W.spos_box, B.total, W.ctr + 3, W.scan_tmp, s);
-            if (rc) return rc;
-            k_surface_scatter<<<gb, kNfBlock, 0, s>>>(A, B, W.wet, W.surf, W.wpos, W.spos_box, fln, sfn,
-                                                      W.spos_cell);
-            int cnt[2];
-            CLOWNS_CUDA_TRY(cudaMemcpyAsync(cnt, W.ctr + 2, sizeof(int) * 2, cudaMemcpyDeviceToHost, s));
-            CLOWNS_CUDA_TRY(cudaStreamSynchronize(s));
-            ifln = cnt[0];
-            isfn = cnt[1];
-        }
-        if (isfn == 0) break;
+        // the lists, and the surface loops as far as they change nothing, with one read-back
+        CLOWNS_CUDA_TRY(cudaMemsetAsync(W.ctr + kCtrUnsettled, 0, sizeof(int), s));
+        k_surface_flags<<<tiles, kBitThreads, 0, s>>>(A, W.ctr, W.wet, W.surf, W.sums);
+        int rc = scan_tiles_dev(2, W.sums, (long)nf_box(dims), nullptr, W.ctr + kCtrWet, s);
+        if (rc) return rc;
+        k_surface_scatter<<<tiles, kBitThreads, 0, s>>>(A, W.ctr, W.wet, W.surf, W.sums, fln, sfn, W.spos_cell);
+        k_surface_check<<<152 * 4, kNfBlock, 0, s>>>(A, f, sfn, W.spos_cell, W.bout, W.ctr);
+        k_surface_settle<<<152 * 4, kNfBlock, 0, s>>>(A, sfn, W.bout, W.ctr);
+        int h[kCtrUnsettled + 1];
+        CLOWNS_CUDA_TRY(cudaMemcpyAsync(h, W.ctr, sizeof(h), cudaMemcpyDeviceToHost, s));
+        CLOWNS_CUDA_TRY(cudaStreamSynchronize(s));
+        ifln = h[kCtrWet];
+        isfn = h[kCtrSurf];
+        if (!h[kCtrUnsettled]) break;
         const int gs = nf_grid(isfn);
         // first pruning
-        CLOWNS_CUDA_TRY(cudaMemsetAsync(W.ctr + 4, 0, sizeof(int), s));
-        k_prune1<<<gs, kNfBlock, 0, s>>>(A, isfn, sfn, W.st0, W.ctr + 4);
+        CLOWNS_CUDA_TRY(cudaMemsetAsync(W.ctr + kCtrPrune, 0, sizeof(int), s));
+        k_prune1<<<gs, kNfBlock, 0, s>>>(A, isfn, sfn, W.st0, W.ctr + kCtrPrune);
         int removed = 0;
-        int rc = read_int(W.ctr + 4, s, &removed);
+        rc = read_int(W.ctr + kCtrPrune, s, &removed);
         if (rc) return rc;
         if (removed) {
             k_remove<<<gs, kNfBlock, 0, s>>>(A, isfn, sfn, W.st0);
@@ -431,10 +518,10 @@ extern "C" int clowns_set_nflag_dev(const int* dims, int inne, int inne2, int mx
         int* nxt = W.st1;
         bool settled = false;
         for (int sweep = 0; sweep <= isfn + 1; sweep++) {
-            CLOWNS_CUDA_TRY(cudaMemsetAsync(W.ctr + 5, 0, sizeof(int), s));
-            k_prune2_sweep<<<gs, kNfBlock, 0, s>>>(A, isfn, sfn, W.spos_cell, cur, nxt, W.ctr + 5);
+            CLOWNS_CUDA_TRY(cudaMemsetAsync(W.ctr + kCtrSweep, 0, sizeof(int), s));
+            k_prune2_sweep<<<gs, kNfBlock, 0, s>>>(A, isfn, sfn, W.spos_cell, cur, nxt, W.ctr + kCtrSweep);
             int changed = 0;
-            rc = read_int(W.ctr + 5, s, &changed);
+            rc = read_int(W.ctr + kCtrSweep, s, &changed);
             if (rc) return rc;
             int* tmp = cur; cur = nxt; nxt = tmp;
             if (!changed) { settled = true; break; }
@@ -444,11 +531,11 @@ extern "C" int clowns_set_nflag_dev(const int* dims, int inne, int inne2, int mx
             return CLOWNS_ERR_NOCONV;
         }
         // apply the removals of the settled state
-        CLOWNS_CUDA_TRY(cudaMemsetAsync(W.ctr + 6, 0, sizeof(int), s));
-        k_count_nonzero<<<gs, kNfBlock, 0, s>>>(cur, isfn, W.ctr + 6);
+        CLOWNS_CUDA_TRY(cudaMemsetAsync(W.ctr + kCtrRemoved, 0, sizeof(int), s));
+        k_count_nonzero<<<gs, kNfBlock, 0, s>>>(cur, isfn, W.ctr + kCtrRemoved);
         k_remove<<<gs, kNfBlock, 0, s>>>(A, isfn, sfn, cur);
         int removed2 = 0;
-        rc = read_int(W.ctr + 6, s, &removed2);
+        rc = read_int(W.ctr + kCtrRemoved, s, &removed2);
         if (rc) return rc;
         if (removed2) continue;
         // orientation: Jacobi to the serial fixed point
@@ -457,10 +544,10 @@ extern "C" int clowns_set_nflag_dev(const int* dims, int inne, int inne2, int mx
         nxt = W.st1;
         settled = false;
         for (int sweep = 0; sweep <= isfn + 1; sweep++) {
-            CLOWNS_CUDA_TRY(cudaMemsetAsync(W.ctr + 5, 0, sizeof(int), s));
-            k_orient_sweep<<<gs, kNfBlock, 0, s>>>(A, f, isfn, sfn, W.spos_cell, cur, nxt, W.bout, W.ctr + 5);
+            CLOWNS_CUDA_TRY(cudaMemsetAsync(W.ctr + kCtrSweep, 0, sizeof(int), s));
+            k_orient_sweep<<<gs, kNfBlock, 0, s>>>(A, f, isfn, sfn, W.spos_cell, cur, nxt, W.bout, W.ctr + kCtrSweep);
             int changed = 0;
-            rc = read_int(W.ctr + 5, s, &changed);
+            rc = read_int(W.ctr + kCtrSweep, s, &changed);
             if (rc) return rc;
             int* tmp = cur; cur = nxt; nxt = tmp;
             if (!changed) { settled = true; break; }
@@ -469,10 +556,10 @@ extern "C" int clowns_set_nflag_dev(const int* dims, int inne, int inne2, int mx
             set_last_error_msg("set_nflag: orientation did not settle");
             return CLOWNS_ERR_NOCONV;
         }
-        CLOWNS_CUDA_TRY(cudaMemsetAsync(W.ctr + 9, 0, sizeof(int), s));
-        k_orient_apply<<<gs, kNfBlock, 0, s>>>(A, isfn, sfn, cur, W.bout, W.ctr + 9);
+        CLOWNS_CUDA_TRY(cudaMemsetAsync(W.ctr + kCtrDropped, 0, sizeof(int), s));
+        k_orient_apply<<<gs, kNfBlock, 0, s>>>(A, isfn, sfn, cur, W.bout, W.ctr + kCtrDropped);
         int igai = 0;
-        rc = read_int(W.ctr + 9, s, &igai);
+        rc = read_int(W.ctr + kCtrDropped, s, &igai);
         if (rc) return rc;
         if (igai) continue;
         break;
