@@ -237,6 +237,7 @@ static inline int member_groups(int n) {
 constexpr int kResMaxRowsFp64 = 500000;
 constexpr int kResMaxRowsMixed = 750000;
 constexpr int kResMaxBlocks = kNumSMs;
+constexpr int kResMaxSmem = 200 * 1024;      // a reduction's operands: 100 chunks per block
 
 static bool res_serves(int M, const int* n, int mixed) {
     long rows = 0;
@@ -601,7 +602,7 @@ static int device_sms() {
 // in proportion to their chunks (each block takes its member's next even share), with
 // the warps that a block's 32-row groups fill, or the fewest rounds of at most
 // kResWarps that cover them, and the scalar warp.
-static LoopShape res_shape(int M, const int* n, BalBlock* tab) {
+static LoopShape res_shape(int M, const int* n, BalBlock* tab, size_t* smem) {
     std::vector<int> nc(M), g(M);
     long total = 0;
     for (int m = 0; m < M; m++) total += nc[m] = (n[m] + kChunk - 1) / kChunk;
@@ -632,6 +633,7 @@ static LoopShape res_shape(int M, const int* n, BalBlock* tab) {
     }
     const int most = kResWarps / kChunkRows, rounds = (per + most - 1) / most;
     sh.block = kChunk * ((per + rounds - 1) / rounds) + 32;
+    *smem = sizeof(double) * 2 * kChunk * per;                  // a reduction's operands
     return sh;
 }
 
@@ -1367,6 +1369,12 @@ static bool res_chosen(const EngLayout& L) {
     return L.res && (forced < 0 || forced == 4);
 }
 
+// Dynamic shared memory beyond the 48 KB a kernel may have without asking.
+static cudaError_t res_smem(const void* fn, size_t bytes) {
+    if (bytes <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResMaxSmem);
+}
+
 // A solve in three kernels -- setup, composed coefficients, and the whole of the rest
 // resident -- between one upload (tables, inputs, initial scalars, a cleared abort
 // flag) and one read-back (scalars and abort flag).
@@ -1377,7 +1385,8 @@ static int solve_resident(const EngLayout& L, const int* n, const MemberIn* ins,
     constexpr bool mixed = std::is_same<T, float>::value;
     std::vector<char> t = eng_tables(L, n, ins);
     for (int m = 0; m < L.M; m++) ((MemberScalars*)(t.data() + L.o_S))[m] = init;
-    const LoopShape sh = res_shape(L.M, n, L.M > 1 ? (BalBlock*)(t.data() + L.o_restab) : nullptr);
+    size_t smem = 0;
+    const LoopShape sh = res_shape(L.M, n, L.M > 1 ? (BalBlock*)(t.data() + L.o_restab) : nullptr, &smem);
     CLOWNS_CUDA_TRY(cudaMemcpyAsync(work, t.data(), L.o_tables, cudaMemcpyHostToDevice, s));
     Eng<T> E = eng_bind<T>(work, L);
     E.nl = nl;
@@ -1397,11 +1406,13 @@ static int solve_resident(const EngLayout& L, const int* n, const MemberIn* ins,
     if constexpr (mixed) {
         void* args[] = {(void*)&E, (void*)&R, (void*)&inner_tol, (void*)&inner_max, (void*)&lim, (void*)&absent};
         const void* fn = nl == 4 ? (const void*)k_res_mixed<4> : (const void*)k_res_mixed<6>;
-        CLOWNS_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(sh.grid), dim3(sh.block), args, 0, s));
+        CLOWNS_CUDA_TRY(res_smem(fn, smem));
+        CLOWNS_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(sh.grid), dim3(sh.block), args, smem, s));
     } else {
         void* args[] = {(void*)&E, (void*)&R, (void*)&lim, (void*)&absent};
         const void* fn = nl == 4 ? (const void*)k_res_plain<4> : (const void*)k_res_plain<6>;
-        CLOWNS_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(sh.grid), dim3(sh.block), args, 0, s));
+        CLOWNS_CUDA_TRY(res_smem(fn, smem));
+        CLOWNS_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(sh.grid), dim3(sh.block), args, smem, s));
     }
     t_launches = 3;
     {

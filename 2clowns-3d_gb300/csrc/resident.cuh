@@ -261,7 +261,6 @@ __device__ __forceinline__ void res_stop_tests(MemberScalars* S, ResStop& st, do
 // Shared state of one block.
 struct ResShared {
     MemberScalars s;
-    double y[kResWarps * 32], u[kResWarps * 32];   // rows of the round a reduction folds
     double beta;         // of the iteration that starts (its stop tests may still run)
     ResStop st;
     int fail;            // a poll ran out
@@ -362,20 +361,22 @@ struct ResRow {
 template <typename T, int NL>
 struct Resident {
     static constexpr int NI = kResIdx<NL>, NC = NI + 1;
+    static constexpr bool kWide = sizeof(T) == 4;     // FP64 rows take twice the registers
     const Eng<T>& E;
     const ResBufs<T>& R;
     ResShared& sh;
+    double* ybuf;                      // the operands y, u of a reduction: the block's rows each
     ResWait wt;
     int lane, w, nw, ws;               // nw row warps; ws: the scalar warp
     BalBlock bb;
     long off, pstride;
-    int n, c0, c1, nc, pad, nq, nround, gstride;
+    int n, c0, c1, nc, pad, nq, gstride;
     unsigned row0;
     TagWord<double>*part, *gpart;
 
     // false: a stopped member, none of its blocks works
-    __device__ __forceinline__ Resident(const Eng<T>& E_, const ResBufs<T>& R_, ResShared& sh_, long limit)
-        : E(E_), R(R_), sh(sh_), wt{limit, E_.abort, &sh_.fail} {
+    __device__ __forceinline__ Resident(const Eng<T>& E_, const ResBufs<T>& R_, ResShared& sh_, double* ybuf_, long limit)
+        : E(E_), R(R_), sh(sh_), ybuf(ybuf_), wt{limit, E_.abort, &sh_.fail} {
         lane = threadIdx.x & 31;
         w = threadIdx.x >> 5;
         nw = ws = (blockDim.x >> 5) - 1;
@@ -386,7 +387,6 @@ struct Resident {
         nc = (n + kChunk - 1) / kChunk;
         pad = (int)off + n;
         nq = w == ws ? 0 : 4 * (c1 - c0);                   // the scalar warp has no rows
-        nround = (4 * (c1 - c0) + nw - 1) / nw;
         row0 = (unsigned)(off + (long)c0 * kChunk) + lane;
         part = R.part + 2 * (off / kChunk);
         pstride = 2 * (E.NV / kChunk);
@@ -407,98 +407,199 @@ struct Resident {
 #pragma unroll 1
         for (int q = w; q < nq; q += nw) f(row(q));
     }
+    // f(NR rows of this warp at once): NR = 1, or two where the block's rows take more than
+    // one round of its warps, so that two rows' gathers are in flight per lane (a row
+    // alone past the end comes twice, the second time not ok)
+    template <typename F>
+    __device__ __forceinline__ void rows2(F f) const {
+        if (kWide && nq > nw) {
+#pragma unroll 1
+            for (int q = w; q < nq; q += 2 * nw) {
+                const ResRow a = row(q), b = q + nw < nq ? row(q + nw) : ResRow{a.i, false};
+                const ResRow rw[2] = {a, b};
+                f(rw);
+            }
+        } else {
+#pragma unroll 1
+            for (int q = w; q < nq; q += nw) {
+                const ResRow rw[1] = {row(q)};
+                f(rw);
+            }
+        }
+    }
     // t[0] = D in + sum_k AL_k in[LL_k] (as k_bal_axsub); own: the block's rows of `in`
     __device__ __forceinline__ void axsub(const T* own, unsigned tag) const {
-        rows([&](const ResRow& rw) {
-            const T* a = coef(rw);
-            const int* cp = idx(rw);
-            T g[NL];
-            int c[NL];
+        rows2([&](const auto& rw) {
+            constexpr int NR = std::extent<std::remove_reference_t<decltype(rw)>>::value;
+            T g[NR * NL], s[NR];
+            int c[NR * NL];
 #pragma unroll
-            for (int k = 0; k < NL; k++) c[k] = cp[32 * k];
-            T s = own[rw.i] * a[32 * NI];
-            res_gather<T, NL>(R.in, c, pad, tag, g, wt);
+            for (int r = 0; r < NR; r++) {
+                const int* cp = idx(rw[r]);
 #pragma unroll
-            for (int k = 0; k < NL; k++) s = fma_rn(a[32 * k], g[k], s);
-            if (rw.ok) tag_put(R.t[0] + rw.i, s, tag);
+                for (int k = 0; k < NL; k++) c[r * NL + k] = cp[32 * k];
+                s[r] = own[rw[r].i] * coef(rw[r])[32 * NI];
+            }
+            res_gather<T, NR * NL>(R.in, c, pad, tag, g, wt);
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                const T* a = coef(rw[r]);
+#pragma unroll
+                for (int k = 0; k < NL; k++) s[r] = fma_rn(a[32 * k], g[r * NL + k], s[r]);
+                if (rw[r].ok) tag_put(R.t[0] + rw[r].i, s[r], tag);
+            }
         });
     }
-    // Sweeps S, S + 1 of LDUSUB at a row, from the words `in`; X: the slot of sweep S at
+    // Sweeps S, S + 1 of LDUSUB at NR rows, from the words `in`; X: the slot of sweep S at
     // column S + 1.  V: the vectors' type (FP64 vectors on FP32 coefficients in the mixed
     // path's refinement).
-    template <int S, int X, typename V>
-    __device__ __forceinline__ V pair(const ResRow& rw, const TagWord<V>* in, unsigned tag) const {
+    template <int S, int X, typename V, int NR>
+    __device__ __forceinline__ void pair(const ResRow (&rw)[NR], const TagWord<V>* in, unsigned tag, V (&o)[NR]) const {
         constexpr int s = S - 1;
-        const T* a = coef(rw);
-        const int* cp = idx(rw);
-        const int c[4] = {self(rw), cp[32 * s], cp[32 * (s + 1)], cp[32 * X]};
-        V g[4];
-        res_gather<V, 4>(in, c, pad, tag, g, wt);
-        const V o = fnma((V)a[32 * s], g[1], g[0]);
-        return fnma((V)a[32 * (s + 1)], fnma((V)a[32 * X], g[3], g[2]), o);
+        V g[NR * 4];
+        int c[NR * 4];
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            const int* cp = idx(rw[r]);
+            c[4 * r] = self(rw[r]);
+            c[4 * r + 1] = cp[32 * s];
+            c[4 * r + 2] = cp[32 * (s + 1)];
+            c[4 * r + 3] = cp[32 * X];
+        }
+        res_gather<V, NR * 4>(in, c, pad, tag, g, wt);
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            const T* a = coef(rw[r]);
+            const V o1 = fnma((V)a[32 * s], g[4 * r + 1], g[4 * r]);
+            o[r] = fnma((V)a[32 * (s + 1)], fnma((V)a[32 * X], g[4 * r + 3], g[4 * r + 2]), o1);
+        }
+    }
+    template <int S, int X, typename V>
+    __device__ __forceinline__ void step(const TagWord<V>* in, TagWord<V>* out, unsigned tag) const {
+        auto f = [&](const auto& rw) {
+            constexpr int NR = std::extent<std::remove_reference_t<decltype(rw)>>::value;
+            V o[NR];
+            pair<S, X, V, NR>(rw, in, tag, o);
+#pragma unroll
+            for (int r = 0; r < NR; r++)
+                if (rw[r].ok) tag_put(out + rw[r].i, o[r], tag);
+        };
+        if constexpr (std::is_same<V, T>::value) rows2(f);
+        else rows([&](const ResRow& r1) {
+            const ResRow rw[1] = {r1};
+            f(rw);
+        });
     }
     // LDUSUB's steps but the last, from the words t[0]
     template <typename V>
     __device__ __forceinline__ void sweeps(TagWord<V>* const (&t)[kResSteps], unsigned tag) const {
-        rows([&](const ResRow& rw) {
-            const V o = pair<1, NL, V>(rw, t[0], tag);
-            if (rw.ok) tag_put(t[1] + rw.i, o, tag);
-        });
-        if constexpr (NL == 6)
-            rows([&](const ResRow& rw) {
-                const V o = pair<3, NL + 1, V>(rw, t[1], tag);
-                if (rw.ok) tag_put(t[2] + rw.i, o, tag);
-            });
+        step<1, NL, V>(t[0], t[1], tag);
+        if constexpr (NL == 6) step<3, NL + 1, V>(t[1], t[2], tag);
     }
-    // the last step at one row
-    template <typename V>
-    __device__ __forceinline__ V last(TagWord<V>* const (&t)[kResSteps], const ResRow& rw, unsigned tag) const {
+    // the last step at NR rows
+    template <typename V, int NR>
+    __device__ __forceinline__ void last(TagWord<V>* const (&t)[kResSteps], const ResRow (&rw)[NR], unsigned tag,
+                                         V (&o)[NR]) const {
         if constexpr (NL == 4) {
-            return pair<3, NL + 1, V>(rw, t[1], tag);
+            pair<3, NL + 1, V, NR>(rw, t[1], tag, o);
         } else {
-            const T* a = coef(rw);
-            const int* cp = idx(rw);
-            const int c[3] = {self(rw), cp[32 * 4], cp[32 * 5]};
-            V g[3];
-            res_gather<V, 3>(t[2], c, pad, tag, g, wt);
-            return fnma((V)a[32 * 5], g[2], fnma((V)a[32 * 4], g[1], g[0]));
+            V g[NR * 3];
+            int c[NR * 3];
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                const int* cp = idx(rw[r]);
+                c[3 * r] = self(rw[r]);
+                c[3 * r + 1] = cp[32 * 4];
+                c[3 * r + 2] = cp[32 * 5];
+            }
+            res_gather<V, NR * 3>(t[2], c, pad, tag, g, wt);
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                const T* a = coef(rw[r]);
+                o[r] = fnma((V)a[32 * 5], g[3 * r + 2], fnma((V)a[32 * 4], g[3 * r + 1], g[3 * r]));
+            }
         }
     }
-    // A reduction over the block's rows: f(row, y, u) gives each row's operands, and lane l
-    // of a chunk's warp folds its rows 32 u + l in order, then the butterfly, in V.
-    // MODE 0: (u, y); 1: (u, y) and (y, y); 2: (y, y) and (y, u); 3: (y, y) -- each total
-    // by a warp of its own.
+    template <typename V>
+    __device__ __forceinline__ V last1(TagWord<V>* const (&t)[kResSteps], const ResRow& r1, unsigned tag) const {
+        const ResRow rw[1] = {r1};
+        V o[1];
+        last<V, 1>(t, rw, tag, o);
+        return o[0];
+    }
+    // Fold B chunk totals (numbers v0 .. v0 + B - 1; total v is value v % NVAL of the block's
+    // chunk v / NVAL) in one warp: lane l folds a chunk's rows 32 h + l in order, then the
+    // butterfly, in V.
+    template <int MODE, int B, typename V>
+    __device__ __forceinline__ void fold(int v0, int red, unsigned tag) const {
+        constexpr int NVAL = MODE == 1 || MODE == 2 ? 2 : 1;
+        const V *ys = (const V*)ybuf, *us = ys + (c1 - c0) * kChunk;
+        V v[B];
+#pragma unroll
+        for (int b = 0; b < B; b++) {
+            v[b] = V(0);
+            const int ch = (v0 + b) / NVAL, k = (v0 + b) % NVAL;
+            if (ch >= c1 - c0) continue;
+            const bool square = MODE == 3 || (MODE == 1 && k == 1) || (MODE == 2 && k == 0);
+#pragma unroll
+            for (int h = 0; h < kChunkRows; h++) {
+                const int at = ch * kChunk + 32 * h + lane;
+                if ((long)c0 * kChunk + at >= n) continue;
+                const V y = ys[at], u = square ? y : us[at];
+                v[b] = fma_rn(u, y, v[b]);
+            }
+        }
+        int id;
+        const V s = warp_tsum<V, B>(v, id);
+        const int vv = v0 + id;
+        if ((lane & (32 / B - 1)) == 0 && vv / NVAL < c1 - c0)
+            tag_put(part + red * pstride + 2 * (c0 + vv / NVAL) + vv % NVAL, (double)s, tag);
+    }
+    // A reduction over the block's rows: f(row, y, u) gives each row's operands.
+    // MODE 0: (u, y); 1: (u, y) and (y, y); 2: (y, y) and (y, u); 3: (y, y).
     template <int MODE, typename V, typename F>
     __device__ __forceinline__ void reduce(int red, unsigned tag, F f) const {
-        constexpr int NVAL = MODE == 1 || MODE == 2 ? 2 : 1;
-        V* ys = (V*)sh.y;
-        V* us = (V*)sh.u;
+        V *ys = (V*)ybuf, *us = ys + (c1 - c0) * kChunk;
+        rows([&](const ResRow& rw) {
+            V y, u = V(0);
+            f(rw, y, u);
+            ys[rw.i - row0 + lane] = y;
+            if (MODE != 3) us[rw.i - row0 + lane] = u;
+        });
+        fold_all<MODE, V>(red, tag);
+    }
+    // The same for the operator's last step, y = that step's result, at NR rows at once;
+    // put(row, y) keeps it and gives u.
+    template <int MODE, typename F>
+    __device__ __forceinline__ void reduce_last(int red, unsigned tag, F put) const {
+        T *ys = (T*)ybuf, *us = ys + (c1 - c0) * kChunk;
+        rows2([&](const auto& rw) {
+            constexpr int NR = std::extent<std::remove_reference_t<decltype(rw)>>::value;
+            T o[NR];
+            last<T, NR>(R.t, rw, tag, o);
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                if (NR == 2 && !rw[r].ok) continue;          // the end's double, or padding
+                const T u = put(rw[r], o[r]);
+                ys[rw[r].i - row0 + lane] = o[r];
+                us[rw[r].i - row0 + lane] = u;
+            }
+        });
+        fold_all<MODE, T>(red, tag);
+    }
+    // A warp takes one total at a time, or four by a transposed butterfly (6 additions
+    // instead of 20) once there are more than five per SM sub-partition.
+    template <int MODE, typename V>
+    __device__ __forceinline__ void fold_all(int red, unsigned tag) const {
+        __syncthreads();
+        const int total = (c1 - c0) * (MODE == 1 || MODE == 2 ? 2 : 1);
+        if (w == ws) return;
+        if (total > 20) {
 #pragma unroll 1
-        for (int rd = 0; rd < nround; rd++) {
-            const int q = rd * nw + w;                      // past nq in the scalar warp
-            if (q < nq) {
-                V y, u = V(0);
-                f(row(q), y, u);
-                ys[32 * w + lane] = y;
-                if (MODE != 3) us[32 * w + lane] = u;
-            }
-            __syncthreads();
-            const int cw = w / NVAL, k = w % NVAL, cc = c0 + rd * (nw / 4) + cw;
-            if (cw < nw / 4 && cc < c1) {
-                const bool square = MODE == 3 || (MODE == 1 && k == 1) || (MODE == 2 && k == 0);
-                V v = V(0);
-#pragma unroll
-                for (int h = 0; h < kChunkRows; h++) {
-                    if ((long)cc * kChunk + 32 * h + lane >= n) continue;
-                    const int at = 32 * (4 * cw + h) + lane;
-                    const V y = ys[at], b = square ? y : us[at];
-                    v = fma_rn(b, y, v);
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                if (lane == 0) tag_put(part + red * pstride + 2 * cc + k, (double)v, tag);
-            }
-            if (rd + 1 < nround) __syncthreads();
+            for (int v = 4 * w; v < total; v += 4 * nw) fold<MODE, 4, V>(v, red, tag);
+        } else {
+#pragma unroll 1
+            for (int v = w; v < total; v += nw) fold<MODE, 1, V>(v, red, tag);
         }
     }
     // The member's totals of reduction `red` and what follows from them: fin(totals) in
@@ -537,10 +638,9 @@ struct Resident {
             });
             axsub(E.p, ta);                                 // q = PM A p ; RQ -> ALP
             sweeps<T>(R.t, ta);
-            reduce<0, T>(0, ta, [&](const ResRow& rw, T& y, T& u) {
-                u = E.r0[rw.i];
-                y = last<T>(R.t, rw, ta);
+            reduce_last<0>(0, ta, [&](const ResRow& rw, T y) {
                 if (rw.ok) E.q[rw.i] = y;
+                return E.r0[rw.i];
             });
             if (!totals<1>(0, ta, [&](const double (&tot)[2]) {
                     if (!sh.s.done) finish_sweep56<1, true>(&sh.s, tot, &sh.s);   // done: by the last iteration's stop tests
@@ -556,10 +656,9 @@ struct Resident {
             });
             axsub(E.e, tb);                                 // v = PM A e ; AMU
             sweeps<T>(R.t, tb);
-            reduce<1, T>(1, tb, [&](const ResRow& rw, T& y, T& u) {
-                u = E.e[rw.i];
-                y = last<T>(R.t, rw, tb);
+            reduce_last<1>(1, tb, [&](const ResRow& rw, T y) {
                 if (rw.ok) E.v[rw.i] = y;
+                return E.e[rw.i];
             });
             if (!totals<2>(1, tb, [&](const double (&tot)[2]) { finish_sweep56<2, true>(&sh.s, tot, &sh.s); })) break;
             const T AMU = T(sh.s.AMU);                      // x, r ; RN, C1 ; stop tests
@@ -616,13 +715,14 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_plain(const Eng<double> 
                                                              int absent) {
     if ((int)blockIdx.x == absent) return;
     __shared__ ResShared sh;
-    const Resident<double, NL> S(E, R, sh, limit);
+    extern __shared__ double ybuf[];
+    const Resident<double, NL> S(E, R, sh, ybuf, limit);
     S.rows([&](const ResRow& rw) {
         if (rw.ok) tag_put(R.t[0] + rw.i, E.p[rw.i], 1);    // W b
     });
     S.template sweeps<double>(R.t, 1);
     S.template reduce<3, double>(0, 1, [&](const ResRow& rw, double& y, double&) {
-        y = S.template last<double>(R.t, rw, 1);
+        y = S.template last1<double>(R.t, rw, 1);
         if (rw.ok) {
             E.p[rw.i] = y;
             tag_put(R.in + rw.i, E.xi[rw.i], 2);
@@ -633,7 +733,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_plain(const Eng<double> 
         S.axsub(E.xi, 2);
         S.template sweeps<double>(R.t, 2);
         S.template reduce<3, double>(1, 2, [&](const ResRow& rw, double& y, double&) {
-            y = E.p[rw.i] - S.template last<double>(R.t, rw, 2);
+            y = E.p[rw.i] - S.template last1<double>(R.t, rw, 2);
             if (rw.ok) {
                 E.r[rw.i] = y;
                 E.p[rw.i] = y;
@@ -655,7 +755,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_mixed(const Eng<float> E
                                                              double inner_tol, int inner_max, long limit, int absent) {
     if ((int)blockIdx.x == absent) return;
     __shared__ ResShared sh;
-    const Resident<float, NL> S(E, R, sh, limit);
+    extern __shared__ double ybuf[];
+    const Resident<float, NL> S(E, R, sh, ybuf, limit);
     const MemberIn in = E.in[S.bb.m];
     S.rows([&](const ResRow& rw) {
         if (rw.ok) {
@@ -664,7 +765,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_mixed(const Eng<float> E
         }
     });
     S.template sweeps<double>(R.t64, 1);
-    S.template reduce<3, double>(4, 1, [&](const ResRow& rw, double& y, double&) { y = S.template last<double>(R.t64, rw, 1); });
+    S.template reduce<3, double>(4, 1, [&](const ResRow& rw, double& y, double&) { y = S.template last1<double>(R.t64, rw, 1); });
     bool go = S.template totals<1>(4, 1, [&](const double (&tot)[2]) { sh.s.BN64 = tot[0]; });
     unsigned ep = 1, xtag = 1;
 #pragma unroll 1
@@ -688,7 +789,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_mixed(const Eng<float> E
         });
         S.template sweeps<double>(R.t64, tag);
         S.template reduce<3, double>(3, tag, [&](const ResRow& rw, double& y, double&) {
-            y = S.template last<double>(R.t64, rw, tag);
+            y = S.template last1<double>(R.t64, rw, tag);
             if (rw.ok) E.r64[rw.i] = y;
         });
         go = S.template totals<1>(3, tag, [&](const double (&tot)[2]) { mx_outer_test(&sh.s, tot[0], inner_tol, inner_max); });
