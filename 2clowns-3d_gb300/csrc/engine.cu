@@ -229,20 +229,70 @@ static inline int member_groups(int n) {
 
 // Systems and ensembles of up to this many rows in all are solved resident, without
 // tuning.  Measured (ms per solve, the tuned graph / resident): single systems FP64
-// 2.7 / 0.8 at 4 k rows, 6.8 / 2.3 at 74 k, 10.6 / 5.6 at 239 k, 12.1 / 9.5 at 413 k,
-// 23.5 / 23.5-31 at 660 k; mixed 3.7 / 1.1, 5.8 / 2.0, 9.1 / 4.0, 11.0 / 7.4, 17.1 / 13.1;
-// ensembles FP64 5.5 / 2.6 at 16 members of 214 k rows, 9.2 / 5.8 at 12 of 407 k, 8.8 /
-// 7.9 at 70 of 552 k, 13.1 / 15.9 at 40 of 1.01 M; mixed 5.7 / 2.1, 7.1 / 4.4, 7.5 / 5.5,
-// 10.7 / 11.8.  Beyond, words, matrix and vectors no longer fit L2.
-constexpr int kResMaxRowsFp64 = 500000;
-constexpr int kResMaxRowsMixed = 750000;
+// 2.7 / 0.8 at 4 k rows, 6.8 / 2.2 at 74 k, 10.5 / 5.2 at 239 k, 12.1 / 7.9 at 413 k,
+// 23.5 / 20.6 at 660 k (a block's vectors fill its shared memory at 720 k); mixed 3.7 /
+// 1.1, 5.8 / 1.9, 9.1 / 3.8, 10.9 / 6.0, 17.3 / 10.7, 19.7 / 15.1 at 960 k, 21.2 / 22.6
+// at 1.15 M (words and matrix no longer fit L2); ensembles FP64 5.5 / 2.5 at 16 members
+// of 214 k rows, 9.2 / 5.0 at 12 of 407 k, 8.8 / 6.3 at 70 of 552 k; mixed 5.7 / 2.1, 7.0
+// / 3.5, 7.6 / 4.4, 10.8 / 7.5 at 40 of 1.01 M, 14.5 / 11.8 at 12 of 1.16 M.
+constexpr int kResMaxRowsFp64 = 700000;
+constexpr int kResMaxRowsMixed = 1100000;
+constexpr int kResEnsRowsMixed = 1250000;
 constexpr int kResMaxBlocks = kNumSMs;
-constexpr int kResMaxSmem = 200 * 1024;      // a reduction's operands: 100 chunks per block
+constexpr size_t kResMaxSmem = 224 * 1024;      // a block's rows of its vectors: 37 chunks in FP64, 74 in FP32
+
+static int device_sms() {
+    static const int sms = [] {
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1) {
+            cudaGetLastError();
+            v = kNumSMs;
+        }
+        return v;
+    }();
+    return sms;
+}
+
+// Blocks of each member in the resident solve: at most one per SM, dealt in proportion
+// to the members' chunks (a block takes its member's next even share).  Returns the
+// largest number of chunks of a block.
+static int res_blocks(int M, const int* n, std::vector<int>& g) {
+    std::vector<int> nc(M);
+    g.assign(M, 0);
+    long total = 0;
+    for (int m = 0; m < M; m++) total += nc[m] = (n[m] + kChunk - 1) / kChunk;
+    const int G = (int)std::min<long>(total, std::min(device_sms(), kResMaxBlocks));
+    int used = 0;
+    for (int m = 0; m < M; m++) used += g[m] = (int)std::max<long>(1, std::min<long>(nc[m], (long)G * nc[m] / total));
+    // the largest share per block gets the next block; a surplus comes from the smallest
+    for (; used < G; used++) {
+        int best = -1;
+        for (int m = 0; m < M; m++)
+            if (g[m] < nc[m] && (best < 0 || (long)nc[m] * g[best] > (long)nc[best] * g[m])) best = m;
+        if (best < 0) break;
+        g[best]++;
+    }
+    for (; used > G; used--) {
+        int best = -1;
+        for (int m = 0; m < M; m++)
+            if (g[m] > 1 && (best < 0 || (long)nc[m] * g[best] < (long)nc[best] * g[m])) best = m;
+        g[best]--;
+    }
+    int per = 0;
+    for (int m = 0; m < M; m++) per = std::max(per, (nc[m] + g[m] - 1) / g[m]);
+    return per;
+}
+static size_t res_smem_bytes(int per, int tsize) { return (size_t)tsize * kResVecs * kChunk * per; }
 
 static bool res_serves(int M, const int* n, int mixed) {
     long rows = 0;
     for (int m = 0; m < M; m++) rows += n[m];
-    return 2 * M <= kResMaxBlocks && rows <= (mixed ? kResMaxRowsMixed : kResMaxRowsFp64);
+    if (2 * M > std::min(device_sms(), kResMaxBlocks) || 
+        rows > (!mixed ? kResMaxRowsFp64 : M == 1 ? kResMaxRowsMixed : kResEnsRowsMixed))
+        return false;
+    std::vector<int> g;
+    return res_smem_bytes(res_blocks(M, n, g), mixed ? 4 : 8) <= kResMaxSmem;
 }
 
 struct EngLayout {
@@ -585,55 +635,19 @@ static const void* wave_fn(int minb) {
     return minb == 12 ? (const void*)k_eng_wave<T, 12> : (const void*)k_eng_wave<T, 8>;
 }
 
-static int device_sms() {
-    static const int sms = [] {
-        int dev = 0, v = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1) {
-            cudaGetLastError();
-            v = kNumSMs;
-        }
-        return v;
-    }();
-    return sms;
-}
-
-// Launch shape of the resident solve: at most one block per SM, dealt to the members
-// in proportion to their chunks (each block takes its member's next even share), with
-// the warps that a block's 32-row groups fill, or the fewest rounds of at most
-// kResWarps that cover them, and the scalar warp.
-static LoopShape res_shape(int M, const int* n, BalBlock* tab, size_t* smem) {
-    std::vector<int> nc(M), g(M);
-    long total = 0;
-    for (int m = 0; m < M; m++) total += nc[m] = (n[m] + kChunk - 1) / kChunk;
-    const int G = (int)std::min<long>(total, std::min(device_sms(), kResMaxBlocks));
-    int used = 0;
-    for (int m = 0; m < M; m++) used += g[m] = (int)std::max<long>(1, std::min<long>(nc[m], (long)G * nc[m] / total));
-    // the largest share per block gets the next block; a surplus comes from the smallest
-    for (; used < G; used++) {
-        int best = -1;
-        for (int m = 0; m < M; m++)
-            if (g[m] < nc[m] && (best < 0 || (long)nc[m] * g[best] > (long)nc[best] * g[m])) best = m;
-        if (best < 0) break;
-        g[best]++;
-    }
-    for (; used > G; used--) {
-        int best = -1;
-        for (int m = 0; m < M; m++)
-            if (g[m] > 1 && (best < 0 || (long)nc[m] * g[best] < (long)nc[best] * g[m])) best = m;
-        g[best]--;
-    }
+// Launch shape of the resident solve (g: blocks of each member).
+static LoopShape res_shape(int M, const std::vector<int>& g, int per, BalBlock* tab) {
     LoopShape sh;
     sh.graph = 4;
-    sh.grid = used;
-    int per = 0, b = 0;
+    int b = 0;
     for (int m = 0; m < M; m++) {
-        per = std::max(per, (nc[m] + g[m] - 1) / g[m]);
-        for (int j = 0; tab && j < g[m]; j++, b++) tab[b] = BalBlock{m, j, g[m], b - j};
+        for (int j = 0; tab && j < g[m]; j++) tab[b + j] = BalBlock{m, j, g[m], b};
+        b += g[m];
     }
+    sh.grid = b;
     const int most = kResWarps / kChunkRows, rounds = (per + most - 1) / most;
-    sh.block = kChunk * ((per + rounds - 1) / rounds) + 32;
-    *smem = sizeof(double) * 2 * kChunk * per;                  // a reduction's operands
+    sh.block = kChunk * ((per + rounds - 1) / rounds) + 32;      // a block's 32-row groups, or the fewest rounds
+                                                                 // that cover them, and the scalar warp
     return sh;
 }
 
@@ -1369,10 +1383,10 @@ static bool res_chosen(const EngLayout& L) {
     return L.res && (forced < 0 || forced == 4);
 }
 
-// Dynamic shared memory beyond the 48 KB a kernel may have without asking.
+// Shared memory (the static part included) beyond the 48 KB a kernel may have without asking.
 static cudaError_t res_smem(const void* fn, size_t bytes) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResMaxSmem);
+    if (bytes + sizeof(ResShared) <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResMaxSmem);
 }
 
 // A solve in three kernels -- setup, composed coefficients, and the whole of the rest
@@ -1385,8 +1399,10 @@ static int solve_resident(const EngLayout& L, const int* n, const MemberIn* ins,
     constexpr bool mixed = std::is_same<T, float>::value;
     std::vector<char> t = eng_tables(L, n, ins);
     for (int m = 0; m < L.M; m++) ((MemberScalars*)(t.data() + L.o_S))[m] = init;
-    size_t smem = 0;
-    const LoopShape sh = res_shape(L.M, n, L.M > 1 ? (BalBlock*)(t.data() + L.o_restab) : nullptr, &smem);
+    std::vector<int> g;
+    const int per = res_blocks(L.M, n, g);
+    const size_t smem = res_smem_bytes(per, L.tsize);
+    const LoopShape sh = res_shape(L.M, g, per, L.M > 1 ? (BalBlock*)(t.data() + L.o_restab) : nullptr);
     CLOWNS_CUDA_TRY(cudaMemcpyAsync(work, t.data(), L.o_tables, cudaMemcpyHostToDevice, s));
     Eng<T> E = eng_bind<T>(work, L);
     E.nl = nl;

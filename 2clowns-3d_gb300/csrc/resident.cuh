@@ -38,6 +38,8 @@
 // reader's own contribution had to precede, so no reader can miss its epoch:
 // the operator's intermediates (a vector of its own for each step) are rewritten
 // once per reduction RQ / AMU, the word of p and e likewise, and each of the three reductions has its own totals.
+// The vectors no other block reads (q, r / v, p, e, r0, x) live in shared memory, in 48
+// (FP64) or 24 bytes per row, which leaves L2 to the matrix and the words.
 // Every poll is bounded: a warp that runs out raises the abort flag, polls of
 // the other warps and blocks then give up too, and the block leaves at the next
 // reduction; the host reports the failure.
@@ -53,6 +55,7 @@ constexpr int kResWarps = 28;                    // row warps of a block at most
 constexpr int kResThreads = 32 * kResWarps + 32; // and the scalar warp: 64 registers per thread
 constexpr int kResReds = 5;                      // RQ, AMU, RN, and two of the mixed path's refinement: a
                                                  // reduction's words are written again only after another one
+constexpr int kResVecs = 6;                      // vectors a block keeps in shared memory
 constexpr int kResSteps = 3;                     // vectors between the operator's steps (NL / 2 of them used)
 
 // Coefficients and indices of one 32-row group in the resident loop's layout:
@@ -353,7 +356,8 @@ __device__ __forceinline__ void res_totals(const TagWord<double>* part, TagWord<
 // row numbers inside its padding (zero coefficients, indices at the zero row):
 // they compute zeros and store nothing.
 struct ResRow {
-    unsigned i;
+    unsigned i;          // row of the row space
+    int l;               // of the block
     bool ok;
 };
 
@@ -365,7 +369,8 @@ struct Resident {
     const Eng<T>& E;
     const ResBufs<T>& R;
     ResShared& sh;
-    double* ybuf;                      // the operands y, u of a reduction: the block's rows each
+    T *p, *q, *e, *rv, *r0, *x;        // the block's rows of these vectors, in shared memory; rv: r from the
+                                       // update of r until e is formed, v until the update of r
     ResWait wt;
     int lane, w, nw, ws;               // nw row warps; ws: the scalar warp
     BalBlock bb;
@@ -375,8 +380,8 @@ struct Resident {
     TagWord<double>*part, *gpart;
 
     // false: a stopped member, none of its blocks works
-    __device__ __forceinline__ Resident(const Eng<T>& E_, const ResBufs<T>& R_, ResShared& sh_, double* ybuf_, long limit)
-        : E(E_), R(R_), sh(sh_), ybuf(ybuf_), wt{limit, E_.abort, &sh_.fail} {
+    __device__ __forceinline__ Resident(const Eng<T>& E_, const ResBufs<T>& R_, ResShared& sh_, double* vecs, long limit)
+        : E(E_), R(R_), sh(sh_), wt{limit, E_.abort, &sh_.fail} {
         lane = threadIdx.x & 31;
         w = threadIdx.x >> 5;
         nw = ws = (blockDim.x >> 5) - 1;
@@ -386,6 +391,13 @@ struct Resident {
         __syncthreads();
         nc = (n + kChunk - 1) / kChunk;
         pad = (int)off + n;
+        const int rows_b = (c1 - c0) * kChunk;
+        q = (T*)vecs;
+        rv = q + rows_b;
+        p = rv + rows_b;
+        e = p + rows_b;
+        r0 = e + rows_b;
+        x = r0 + rows_b;
         nq = w == ws ? 0 : 4 * (c1 - c0);                   // the scalar warp has no rows
         row0 = (unsigned)(off + (long)c0 * kChunk) + lane;
         part = R.part + 2 * (off / kChunk);
@@ -396,7 +408,7 @@ struct Resident {
     __device__ __forceinline__ ResRow row(int q) const {
         unsigned i = row0 + 32u * q;
         asm volatile("" : "+r"(i));          // addresses are formed in each phase, not carried through all of them
-        return ResRow{i, (int)i < pad};
+        return ResRow{i, 32 * q + lane, (int)i < pad};
     }
     __device__ __forceinline__ const T* coef(const ResRow& rw) const { return R.a + (size_t)(rw.i >> 5) * (32 * NC) + lane; }
     __device__ __forceinline__ const int* idx(const ResRow& rw) const { return R.c + (size_t)(rw.i >> 5) * (32 * NI) + lane; }
@@ -415,7 +427,7 @@ struct Resident {
         if (kWide && nq > nw) {
 #pragma unroll 1
             for (int q = w; q < nq; q += 2 * nw) {
-                const ResRow a = row(q), b = q + nw < nq ? row(q + nw) : ResRow{a.i, false};
+                const ResRow a = row(q), b = q + nw < nq ? row(q + nw) : ResRow{a.i, a.l, false};
                 const ResRow rw[2] = {a, b};
                 f(rw);
             }
@@ -438,7 +450,7 @@ struct Resident {
                 const int* cp = idx(rw[r]);
 #pragma unroll
                 for (int k = 0; k < NL; k++) c[r * NL + k] = cp[32 * k];
-                s[r] = own[rw[r].i] * coef(rw[r])[32 * NI];
+                s[r] = own[rw[r].l] * coef(rw[r])[32 * NI];
             }
             res_gather<T, NR * NL>(R.in, c, pad, tag, g, wt);
 #pragma unroll
@@ -531,9 +543,8 @@ struct Resident {
     // chunk v / NVAL) in one warp: lane l folds a chunk's rows 32 h + l in order, then the
     // butterfly, in V.
     template <int MODE, int B, typename V>
-    __device__ __forceinline__ void fold(int v0, int red, unsigned tag) const {
+    __device__ __forceinline__ void fold(const V* ys, const V* us, int v0, int red, unsigned tag) const {
         constexpr int NVAL = MODE == 1 || MODE == 2 ? 2 : 1;
-        const V *ys = (const V*)ybuf, *us = ys + (c1 - c0) * kChunk;
         V v[B];
 #pragma unroll
         for (int b = 0; b < B; b++) {
@@ -555,52 +566,33 @@ struct Resident {
         if ((lane & (32 / B - 1)) == 0 && vv / NVAL < c1 - c0)
             tag_put(part + red * pstride + 2 * (c0 + vv / NVAL) + vv % NVAL, (double)s, tag);
     }
-    // A reduction over the block's rows: f(row, y, u) gives each row's operands.
-    // MODE 0: (u, y); 1: (u, y) and (y, y); 2: (y, y) and (y, u); 3: (y, y).
-    template <int MODE, typename V, typename F>
-    __device__ __forceinline__ void reduce(int red, unsigned tag, F f) const {
-        V *ys = (V*)ybuf, *us = ys + (c1 - c0) * kChunk;
-        rows([&](const ResRow& rw) {
-            V y, u = V(0);
-            f(rw, y, u);
-            ys[rw.i - row0 + lane] = y;
-            if (MODE != 3) us[rw.i - row0 + lane] = u;
-        });
-        fold_all<MODE, V>(red, tag);
-    }
-    // The same for the operator's last step, y = that step's result, at NR rows at once;
-    // put(row, y) keeps it and gives u.
-    template <int MODE, typename F>
-    __device__ __forceinline__ void reduce_last(int red, unsigned tag, F put) const {
-        T *ys = (T*)ybuf, *us = ys + (c1 - c0) * kChunk;
-        rows2([&](const auto& rw) {
-            constexpr int NR = std::extent<std::remove_reference_t<decltype(rw)>>::value;
-            T o[NR];
-            last<T, NR>(R.t, rw, tag, o);
-#pragma unroll
-            for (int r = 0; r < NR; r++) {
-                if (NR == 2 && !rw[r].ok) continue;          // the end's double, or padding
-                const T u = put(rw[r], o[r]);
-                ys[rw[r].i - row0 + lane] = o[r];
-                us[rw[r].i - row0 + lane] = u;
-            }
-        });
-        fold_all<MODE, T>(red, tag);
-    }
+    // A reduction over the block's rows of y and u (in shared memory, written before the
+    // barrier).  MODE 0: (u, y); 1: (u, y) and (y, y); 2: (y, y) and (y, u); 3: (y, y).
     // A warp takes one total at a time, or four by a transposed butterfly (6 additions
     // instead of 20) once there are more than five per SM sub-partition.
     template <int MODE, typename V>
-    __device__ __forceinline__ void fold_all(int red, unsigned tag) const {
+    __device__ __forceinline__ void reduce(const V* ys, const V* us, int red, unsigned tag) const {
         __syncthreads();
         const int total = (c1 - c0) * (MODE == 1 || MODE == 2 ? 2 : 1);
         if (w == ws) return;
         if (total > 20) {
 #pragma unroll 1
-            for (int v = 4 * w; v < total; v += 4 * nw) fold<MODE, 4, V>(v, red, tag);
+            for (int v = 4 * w; v < total; v += 4 * nw) fold<MODE, 4, V>(ys, us, v, red, tag);
         } else {
 #pragma unroll 1
-            for (int v = w; v < total; v += nw) fold<MODE, 1, V>(v, red, tag);
+            for (int v = w; v < total; v += nw) fold<MODE, 1, V>(ys, us, v, red, tag);
         }
+    }
+    // the operator's last step over the block's rows
+    __device__ __forceinline__ void last_to(T* out, unsigned tag) const {
+        rows2([&](const auto& rw) {
+            constexpr int NR = std::extent<std::remove_reference_t<decltype(rw)>>::value;
+            T o[NR];
+            last<T, NR>(R.t, rw, tag, o);
+#pragma unroll
+            for (int r = 0; r < NR; r++)
+                if (rw[r].ok) out[rw[r].l] = o[r];
+        });
     }
     // The member's totals of reduction `red` and what follows from them: fin(totals) in
     // one thread; every thread then knows whether to go on.
@@ -617,7 +609,7 @@ struct Resident {
         __syncthreads();
         return sh.stop == 0;
     }
-    // The iterations of one (inner) solve from r = p = r0, xi, BN and C1; ep: epochs used so
+    // The iterations of one (inner) solve from r = p = r0, x, BN and C1; ep: epochs used so
     // far, each iteration takes two.
     __device__ __forceinline__ void iterate(unsigned& ep) const {
         if (w == ws && lane == 0)
@@ -629,50 +621,47 @@ struct Resident {
             const unsigned ta = ep + 1, tb = ep + 2;
             const T BETA = T(sh.beta);
             rows([&](const ResRow& rw) {                    // p = r + BETA (p - AMU q), published
-                T p = E.p[rw.i];                            // p - AMU q after the first iteration
+                if (!rw.ok) return;
+                T pn = p[rw.l];                             // p - AMU q after the first iteration
                 if (it > 0) {
-                    p = fma_rn(BETA, p, E.r[rw.i]);
-                    if (rw.ok) E.p[rw.i] = p;
+                    pn = fma_rn(BETA, pn, rv[rw.l]);
+                    p[rw.l] = pn;
                 }
-                if (rw.ok) tag_put(R.in + rw.i, p, ta);
+                tag_put(R.in + rw.i, pn, ta);
             });
-            axsub(E.p, ta);                                 // q = PM A p ; RQ -> ALP
+            axsub(p, ta);                                   // q = PM A p ; RQ -> ALP
             sweeps<T>(R.t, ta);
-            reduce_last<0>(0, ta, [&](const ResRow& rw, T y) {
-                if (rw.ok) E.q[rw.i] = y;
-                return E.r0[rw.i];
-            });
+            last_to(q, ta);
+            reduce<0, T>(q, r0, 0, ta);
             if (!totals<1>(0, ta, [&](const double (&tot)[2]) {
                     if (!sh.s.done) finish_sweep56<1, true>(&sh.s, tot, &sh.s);   // done: by the last iteration's stop tests
                 }))
                 break;
             const T ALP = T(sh.s.ALP);
             rows([&](const ResRow& rw) {                    // e = r - ALP q, published
-                const T e = fnma(ALP, E.q[rw.i], E.r[rw.i]);
-                if (rw.ok) {
-                    E.e[rw.i] = e;
-                    tag_put(R.in + rw.i, e, tb);
-                }
+                if (!rw.ok) return;
+                const T en = fnma(ALP, q[rw.l], rv[rw.l]);
+                e[rw.l] = en;
+                tag_put(R.in + rw.i, en, tb);
             });
-            axsub(E.e, tb);                                 // v = PM A e ; AMU
+            axsub(e, tb);                                   // v = PM A e ; AMU
             sweeps<T>(R.t, tb);
-            reduce_last<1>(1, tb, [&](const ResRow& rw, T y) {
-                if (rw.ok) E.v[rw.i] = y;
-                return E.e[rw.i];
-            });
+            last_to(rv, tb);
+            reduce<1, T>(rv, e, 1, tb);
             if (!totals<2>(1, tb, [&](const double (&tot)[2]) { finish_sweep56<2, true>(&sh.s, tot, &sh.s); })) break;
             const T AMU = T(sh.s.AMU);                      // x, r ; RN, C1 ; stop tests
-            reduce<2, T>(2, ta, [&](const ResRow& rw, T& y, T& u) {
-                u = E.r0[rw.i];
-                y = fnma(AMU, E.v[rw.i], E.e[rw.i]);
-                if (rw.ok) E.r[rw.i] = y;
+            rows([&](const ResRow& rw) {
+                if (!rw.ok) return;
+                const T rn = fnma(AMU, rv[rw.l], e[rw.l]);
+                rv[rw.l] = rn;
+                if (sh.s.mode == 2) E.r[rw.i] = rn;         // PCGPME_WILL's caller reads the residual
             });
+            reduce<2, T>(rv, r0, 2, ta);
             rows([&](const ResRow& rw) {                    // while the totals travel
-                if (rw.ok) {
-                    const T p = E.p[rw.i];
-                    E.xi[rw.i] = fma_rn(AMU, E.e[rw.i], fma_rn(ALP, p, E.xi[rw.i]));
-                    E.p[rw.i] = fnma(AMU, E.q[rw.i], p);
-                }
+                if (!rw.ok) return;
+                const T pn = p[rw.l];
+                x[rw.l] = fma_rn(AMU, e[rw.l], fma_rn(ALP, pn, x[rw.l]));
+                p[rw.l] = fnma(AMU, q[rw.l], pn);
             });
             double rn = 0.0, c1n = 0.0, beta = 0.0;
             totals<2>(2, ta, [&](const double (&tot)[2]) {  // 241 (pcgpme_para.F90); pcgpme_2DH.f90:255
@@ -695,16 +684,11 @@ struct Resident {
         }
         __syncthreads();
     }
-    // the member's scalars for the host, and its solution for the caller
-    __device__ __forceinline__ void finish(const T* x, const double* x64) const {
-        double* out = E.in[bb.m].x - off;
-        rows([&](const ResRow& rw) {
-            if (rw.ok) out[rw.i] = x64 ? x64[rw.i] : (double)x[rw.i];
-        });
-        if (bb.j == 0) {
-            constexpr int W = (int)(sizeof(MemberScalars) / 4);
-            if (threadIdx.x < W) ((int*)(E.S + bb.m))[threadIdx.x] = ((const int*)&sh.s)[threadIdx.x];
-        }
+    // the member's scalars for the host
+    __device__ __forceinline__ void finish() const {
+        if (bb.j) return;
+        constexpr int W = (int)(sizeof(MemberScalars) / 4);
+        if (threadIdx.x < W) ((int*)(E.S + bb.m))[threadIdx.x] = ((const int*)&sh.s)[threadIdx.x];
     }
 };
 
@@ -715,36 +699,41 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_plain(const Eng<double> 
                                                              int absent) {
     if ((int)blockIdx.x == absent) return;
     __shared__ ResShared sh;
-    extern __shared__ double ybuf[];
-    const Resident<double, NL> S(E, R, sh, ybuf, limit);
+    extern __shared__ double vecs[];
+    const Resident<double, NL> S(E, R, sh, vecs, limit);
     S.rows([&](const ResRow& rw) {
-        if (rw.ok) tag_put(R.t[0] + rw.i, E.p[rw.i], 1);    // W b
+        if (!rw.ok) return;
+        const double x0 = E.xi[rw.i];
+        S.x[rw.l] = x0;
+        tag_put(R.t[0] + rw.i, E.p[rw.i], 1);               // W b
+        tag_put(R.in + rw.i, x0, 2);
     });
     S.template sweeps<double>(R.t, 1);
-    S.template reduce<3, double>(0, 1, [&](const ResRow& rw, double& y, double&) {
-        y = S.template last1<double>(R.t, rw, 1);
-        if (rw.ok) {
-            E.p[rw.i] = y;
-            tag_put(R.in + rw.i, E.xi[rw.i], 2);
-        }
-    });
+    S.last_to(S.p, 1);
+    S.template reduce<3, double>(S.p, nullptr, 0, 1);
     bool go = S.template totals<1>(0, 1, [&](const double (&tot)[2]) { sh.s.BN = tot[0]; });
     if (go) {
-        S.axsub(E.xi, 2);
+        S.axsub(S.x, 2);
         S.template sweeps<double>(R.t, 2);
-        S.template reduce<3, double>(1, 2, [&](const ResRow& rw, double& y, double&) {
-            y = E.p[rw.i] - S.template last1<double>(R.t, rw, 2);
-            if (rw.ok) {
-                E.r[rw.i] = y;
-                E.p[rw.i] = y;
-                E.r0[rw.i] = y;
-            }
+        S.last_to(S.q, 2);
+        S.rows([&](const ResRow& rw) {
+            if (!rw.ok) return;
+            const double r = S.p[rw.l] - S.q[rw.l];
+            S.rv[rw.l] = r;
+            S.p[rw.l] = r;
+            S.r0[rw.l] = r;
+            if (sh.s.mode == 2) E.r[rw.i] = r;
         });
+        S.template reduce<3, double>(S.rv, nullptr, 1, 2);
         go = S.template totals<1>(1, 2, [&](const double (&tot)[2]) { sh.s.C1 = tot[0]; });
     }
     unsigned ep = 2;
     if (go) S.iterate(ep);
-    S.finish(E.xi, nullptr);
+    double* out = E.in[S.bb.m].x - S.off;
+    S.rows([&](const ResRow& rw) {
+        if (rw.ok) out[rw.i] = S.x[rw.l];
+    });
+    S.finish();
 }
 
 // A whole mixed-precision solve after the setup kernels: ||PM W b|| on FP64 vectors,
@@ -755,17 +744,18 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_mixed(const Eng<float> E
                                                              double inner_tol, int inner_max, long limit, int absent) {
     if ((int)blockIdx.x == absent) return;
     __shared__ ResShared sh;
-    extern __shared__ double ybuf[];
-    const Resident<float, NL> S(E, R, sh, ybuf, limit);
+    extern __shared__ double vecs[];
+    const Resident<float, NL> S(E, R, sh, vecs, limit);
     const MemberIn in = E.in[S.bb.m];
+    double* y64 = vecs;                                     // FP64 operands lie over q and rv, dead between the sweeps
     S.rows([&](const ResRow& rw) {
-        if (rw.ok) {
-            tag_put(R.t64[0] + rw.i, E.r64[rw.i], 1);       // W b
-            tag_put(R.x64 + rw.i, E.x64[rw.i], 1);
-        }
+        if (!rw.ok) return;
+        tag_put(R.t64[0] + rw.i, E.r64[rw.i], 1);           // W b
+        tag_put(R.x64 + rw.i, E.x64[rw.i], 1);
     });
     S.template sweeps<double>(R.t64, 1);
-    S.template reduce<3, double>(4, 1, [&](const ResRow& rw, double& y, double&) { y = S.template last1<double>(R.t64, rw, 1); });
+    S.rows([&](const ResRow& rw) { y64[rw.l] = S.template last1<double>(R.t64, rw, 1); });
+    S.template reduce<3, double>(y64, nullptr, 4, 1);
     bool go = S.template totals<1>(4, 1, [&](const double (&tot)[2]) { sh.s.BN64 = tot[0]; });
     unsigned ep = 1, xtag = 1;
 #pragma unroll 1
@@ -788,39 +778,43 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_mixed(const Eng<float> E
             if (rw.ok) tag_put(R.t64[0] + rw.i, E.W[rw.i] * (in.b[li] - s), tag);
         });
         S.template sweeps<double>(R.t64, tag);
-        S.template reduce<3, double>(3, tag, [&](const ResRow& rw, double& y, double&) {
-            y = S.template last1<double>(R.t64, rw, tag);
+        S.rows([&](const ResRow& rw) {
+            const double y = S.template last1<double>(R.t64, rw, tag);
+            y64[rw.l] = y;
             if (rw.ok) E.r64[rw.i] = y;
         });
+        S.template reduce<3, double>(y64, nullptr, 3, tag);
         go = S.template totals<1>(3, tag, [&](const double (&tot)[2]) { mx_outer_test(&sh.s, tot[0], inner_tol, inner_max); });
         if (!go) break;
         const double inv = 1.0 / sh.s.SIGMA;
-        S.template reduce<3, double>(4, tag, [&](const ResRow& rw, double& y, double&) {
-            const float v = (float)(E.r64[rw.i] * inv);
-            if (rw.ok) {
-                E.r[rw.i] = v;
-                E.p[rw.i] = v;
-                E.r0[rw.i] = v;
-                E.xi[rw.i] = 0.f;
-            }
-            y = (double)v;
+        S.rows([&](const ResRow& rw) {
+            const float v = rw.ok ? (float)(E.r64[rw.i] * inv) : 0.f;
+            S.p[rw.l] = v;
+            S.r0[rw.l] = v;
+            S.x[rw.l] = 0.f;
+            y64[rw.l] = (double)v;
         });
+        S.template reduce<3, double>(y64, nullptr, 4, tag);
         go = S.template totals<1>(4, tag, [&](const double (&tot)[2]) { sh.s.BN = sh.s.C1 = tot[0]; });
         if (!go) break;
+        S.rows([&](const ResRow& rw) { S.rv[rw.l] = S.p[rw.l]; });   // r, where the operands were
+        __syncthreads();
         S.iterate(ep);
         xtag = ++ep;
         const double sg = sh.s.SIGMA;
         S.rows([&](const ResRow& rw) {                      // x64 += sigma xi, published
-            const double x = fma_rn(sg, (double)E.xi[rw.i], E.x64[rw.i]);
-            if (rw.ok) {
-                E.x64[rw.i] = x;
-                tag_put(R.x64 + rw.i, x, xtag);
-            }
+            if (!rw.ok) return;
+            const double x = fma_rn(sg, (double)S.x[rw.l], E.x64[rw.i]);
+            E.x64[rw.i] = x;
+            tag_put(R.x64 + rw.i, x, xtag);
         });
         go = *(volatile int*)&sh.fail == 0;
         go = __syncthreads_and(go);
     }
-    S.finish(nullptr, E.x64);
+    S.rows([&](const ResRow& rw) {
+        if (rw.ok) in.x[(long)rw.i - S.off] = E.x64[rw.i];
+    });
+    S.finish();
 }
 
 }  // namespace clowns

@@ -5,7 +5,7 @@ bit for bit, in FP64 and mixed precision, on matrices with six and four columns,
 with neighbours near by (band) and anywhere (random: self references, repeated
 columns and empty slots among them).  Sizes sit at the edges of its mapping: a
 lane, a 32-row group, a 128-row chunk, a reduction group of 64 chunks, one chunk
-per SM and one round of a block's warps.  A wait that runs out is reported and
+per SM and one round of a block's warps, several rounds.  A wait that runs out is reported and
 leaves the context usable."""
 import ctypes as C
 import itertools
@@ -15,7 +15,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 31, 33, 127, 128, 129, 4097, 8192, 8193, 19456, 19457, 136192, 136193]
+SIZES = [1, 31, 33, 127, 128, 129, 4097, 8192, 8193, 19456, 19457, 136192, 136193, 300000]
 
 
 def _system(n, nl, kind):
