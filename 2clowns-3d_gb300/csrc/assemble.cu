@@ -218,28 +218,6 @@ __global__ void __launch_bounds__(kBitThreads) k_row_scatter(GridIdx g, int ifln
     }
 }
 
-// a / d with one rounding, given y = 1 / d rounded to nearest: Markstein's method (IBM
-// J. Res. Dev. 34, 1990).  a y, corrected once by its remainder, is within an ulp of the
-// quotient, and such a value corrected by its exact remainder times y rounds to it; the
-// remainders are exact while a and d are far from the ends of the exponent range, and
-// a zero keeps its sign only in a division, so those cases divide.  Five FP64 operations
-// instead of about ten.
-struct Recip {
-    double d, y;
-    bool ok;
-};
-__device__ __forceinline__ bool mid_exponent(double x) {
-    const int e = (__double2hiint(x) >> 20) & 0x7ff;
-    return e > 523 && e < 1523;                          // 2^-500 .. 2^500
-}
-__device__ __forceinline__ Recip make_recip(double d) { return Recip{d, 1.0 / d, mid_exponent(d)}; }
-__device__ __forceinline__ double div_by(double a, const Recip& r) {
-    if (!r.ok || !mid_exponent(a)) return a / r.d;
-    const double q0 = a * r.y;
-    const double q1 = __fma_rn(__fma_rn(-r.d, q0, a), r.y, q0);
-    return __fma_rn(__fma_rn(-r.d, q1, a), r.y, q1);
-}
-
 // RHS of the fluid rows (1sub-momentum.F90:313-360) and dmax = max |DR1|, with renzoku_fv
 // (lib/src/math_func.F90:51-54).  Nothing when there are fewer than 10 rows, or no
 // room for the reference's 64 spare ones.

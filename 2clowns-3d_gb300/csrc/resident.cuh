@@ -201,6 +201,25 @@ __device__ __forceinline__ void res_gather(const TagWord<T>* __restrict__ buf, c
 __device__ __forceinline__ bool f64_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
 __device__ __forceinline__ bool f64_finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
 
+// finish_sweep56's finalisations.
+template <int MODE>
+__device__ __forceinline__ void res_finish56(MemberScalars* S, const double (&tot)[2]) {
+    double ratio;
+    if (MODE == 1) {
+        ratio = S->C1 / tot[0];                                  // 167
+        S->RQ = tot[0];
+        S->ALP = ratio;
+    } else {
+        ratio = tot[0] / tot[1];                                 // 197
+        S->SS = tot[1];
+        S->AMU = ratio;
+    }
+    if (!f64_finite(tot[MODE - 1]) || !f64_finite(ratio)) {
+        S->K += 1;
+        stop_member(S, CLOWNS_STOP_NONFINITE, S->mode != 1 ? CLOWNS_IER_NONFINITE : 0);
+    }
+}
+
 // finish_xrupdate's stop tests (pcgpme_para.F90:215-254) by one thread, BETA
 // already formed.  ERR = sqrt(RN / BN) takes a division and a square root, some 2000
 // cycles in which the next reduction would wait; but with q = RN (1 / BN), within a
@@ -266,9 +285,31 @@ struct ResShared {
     MemberScalars s;
     double beta;         // of the iteration that starts (its stop tests may still run)
     ResStop st;
+    Recip rq, amu;       // reciprocals for BETA, formed while others compute
     int fail;            // a poll ran out
     int stop;            // the scalar warp's verdict at the last reduction: leave the loop
 };
+
+// The butterfly over lanes of which only the first cnt hold terms: the levels that
+// would add zeros are left out (no total here is -0: every sum starts from +0 or is one
+// of a tree).  NVAL = 2: value k in lanes 16 k .. 16 k + 15.
+template <int NVAL>
+__device__ __forceinline__ double res_butterfly(const double (&a)[NVAL], int cnt) {
+    double s = a[0];
+    if (NVAL == 2) {
+        const bool hi = (threadIdx.x & 16) != 0;
+        const double other = __shfl_xor_sync(0xffffffffu, hi ? a[0] : a[NVAL - 1], 16);
+        if (hi) s = a[NVAL - 1];
+        if (cnt > 16) s += other;
+        else if (hi) s = other;
+    } else if (cnt > 16) {
+        s += __shfl_xor_sync(0xffffffffu, s, 16);
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+        if (cnt > o) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
 
 // The sum of up to 64 tagged pairs by one warp, along the canonical tree of a
 // group: lane l adds words l and l + 32, then the butterfly.  NVAL = 2: value k in
@@ -297,56 +338,54 @@ __device__ __forceinline__ double res_group(const TagWord<double>* p, int cnt, u
             for (int k = 0; k < NVAL; k++) a[0][k] += a[1][k];
         __syncwarp();
     }
-    return NVAL == 1 ? warp_sum(a[0][0]) : warp_pair_sum(a[0][0], a[0][NVAL - 1]);
+    return res_butterfly<NVAL>(a[0], cnt);
 }
 
-// Member totals of one reduction (epoch tag), by the scalar warp of every block.
-// Up to 64 chunks (one group) each block sums the chunk totals itself; otherwise
-// a group is summed by one block -- the one that holds its first chunk -- and its
-// total published, and every block sums the groups: 152 blocks polling every
-// chunk total held up the stores they waited for (3-6 us per reduction at 27 k -
-// 74 k rows).  Totals in every lane.
+// Member totals of one reduction (epoch tag), by the scalar warp of every block, in
+// every lane of it.  The block that holds a group's first chunk sums the group and
+// publishes its total, and every block sums the groups: 152 blocks polling every chunk
+// total held up the stores they waited for (3-6 us per reduction at 27 k - 74 k rows).
 template <int NVAL>
 __device__ __forceinline__ void res_totals(const TagWord<double>* part, TagWord<double>* gpart, int nc, int c0, int c1,
                                            unsigned tag, const ResWait& wt, double (&tot)[2]) {
     const int lane = threadIdx.x & 31;
     const int ng = (nc + kGroupChunks - 1) / kGroupChunks;
-    double s;
-    if (ng == 1) {
-        s = res_group<NVAL>(part, nc, tag, wt);
-        s += 0.0;                             // the member sum starts from 0
-    } else {
-#pragma unroll 1
-        for (int g = (c0 + kGroupChunks - 1) / kGroupChunks; g * kGroupChunks < c1; g++) {
-            const double t = res_group<NVAL>(part + 2L * g * kGroupChunks, min(kGroupChunks, nc - g * kGroupChunks),
-                                             tag, wt);
-            if ((lane & (32 / NVAL - 1)) == 0) tag_put(gpart + 2 * g + lane / (32 / NVAL), t, tag);
-        }
-        double a[NVAL];
-#pragma unroll
-        for (int k = 0; k < NVAL; k++) a[k] = 0.0;
-        long spins = 0;
-#pragma unroll 1
-        for (int j = lane; j < ((ng + 31) & ~31); j += 32) {      // lane l: groups l, l + 32, ... in order
-            double v[NVAL];
-#pragma unroll 1
-            for (;;) {
-                unsigned bad = 0;
-#pragma unroll
-                for (int k = 0; k < NVAL; k++) {
-                    v[k] = 0.0;
-                    if (j < ng) bad |= tag_get(gpart + 2 * j + k, v[k]) ^ tag;
-                }
-                if (__all_sync(0xffffffffu, bad == 0)) break;
-                if (!__all_sync(0xffffffffu, wt.more(spins))) break;
-            }
-            if (j < ng)
-#pragma unroll
-                for (int k = 0; k < NVAL; k++) a[k] += v[k];
-        }
-        __syncwarp();
-        s = NVAL == 1 ? warp_sum(a[0]) : warp_pair_sum(a[0], a[NVAL - 1]);
+    if (ng == 1) {                                // one group: every block sums its chunks itself
+        double s = res_group<NVAL>(part, nc, tag, wt);
+        s += 0.0;                                 // the member's sum starts from +0
+        tot[0] = __shfl_sync(0xffffffffu, s, 0);
+        tot[1] = __shfl_sync(0xffffffffu, s, 16);
+        return;
     }
+#pragma unroll 1
+    for (int g = (c0 + kGroupChunks - 1) / kGroupChunks; g * kGroupChunks < c1; g++) {
+        const double t = res_group<NVAL>(part + 2L * g * kGroupChunks, min(kGroupChunks, nc - g * kGroupChunks), tag, wt);
+        if ((lane & (32 / NVAL - 1)) == 0) tag_put(gpart + 2 * g + lane / (32 / NVAL), t, tag);
+    }
+    double a[NVAL];
+#pragma unroll
+    for (int k = 0; k < NVAL; k++) a[k] = 0.0;
+    long spins = 0;
+#pragma unroll 1
+    for (int j = lane; j < ((ng + 31) & ~31); j += 32) {          // lane l: groups l, l + 32, ... in order
+        double v[NVAL];
+#pragma unroll 1
+        for (;;) {
+            unsigned bad = 0;
+#pragma unroll
+            for (int k = 0; k < NVAL; k++) {
+                v[k] = 0.0;
+                if (j < ng) bad |= tag_get(gpart + 2 * j + k, v[k]) ^ tag;
+            }
+            if (__all_sync(0xffffffffu, bad == 0)) break;
+            if (!__all_sync(0xffffffffu, wt.more(spins))) break;
+        }
+        if (j < ng)
+#pragma unroll
+            for (int k = 0; k < NVAL; k++) a[k] += v[k];
+    }
+    __syncwarp();
+    const double s = res_butterfly<NVAL>(a, ng);
     tot[0] = __shfl_sync(0xffffffffu, s, 0);
     tot[1] = __shfl_sync(0xffffffffu, s, 16);
 }
@@ -572,9 +611,9 @@ struct Resident {
     // instead of 20) once there are more than five per SM sub-partition.
     template <int MODE, typename V>
     __device__ __forceinline__ void reduce(const V* ys, const V* us, int red, unsigned tag) const {
-        __syncthreads();
+        if (w == ws) return;                                // the scalar warp has neither rows nor totals to fold
+        asm volatile("bar.sync 1, %0;" ::"r"(32 * nw) : "memory");
         const int total = (c1 - c0) * (MODE == 1 || MODE == 2 ? 2 : 1);
-        if (w == ws) return;
         if (total > 20) {
 #pragma unroll 1
             for (int v = 4 * w; v < total; v += 4 * nw) fold<MODE, 4, V>(ys, us, v, red, tag);
@@ -634,9 +673,10 @@ struct Resident {
             last_to(q, ta);
             reduce<0, T>(q, r0, 0, ta);
             if (!totals<1>(0, ta, [&](const double (&tot)[2]) {
-                    if (!sh.s.done) finish_sweep56<1, true>(&sh.s, tot, &sh.s);   // done: by the last iteration's stop tests
+                    if (!sh.s.done) res_finish56<1>(&sh.s, tot);    // done: by the last iteration's stop tests
                 }))
                 break;
+            if (w == ws && lane == 0) sh.rq = make_recip(sh.s.RQ);
             const T ALP = T(sh.s.ALP);
             rows([&](const ResRow& rw) {                    // e = r - ALP q, published
                 if (!rw.ok) return;
@@ -648,7 +688,8 @@ struct Resident {
             sweeps<T>(R.t, tb);
             last_to(rv, tb);
             reduce<1, T>(rv, e, 1, tb);
-            if (!totals<2>(1, tb, [&](const double (&tot)[2]) { finish_sweep56<2, true>(&sh.s, tot, &sh.s); })) break;
+            if (!totals<2>(1, tb, [&](const double (&tot)[2]) { res_finish56<2>(&sh.s, tot); })) break;
+            if (w == ws && lane == 0) sh.amu = make_recip(sh.s.mode == 2 ? sh.s.AMU * sh.s.RQ : sh.s.AMU);
             const T AMU = T(sh.s.AMU);                      // x, r ; RN, C1 ; stop tests
             rows([&](const ResRow& rw) {
                 if (!rw.ok) return;
@@ -667,7 +708,8 @@ struct Resident {
             totals<2>(2, ta, [&](const double (&tot)[2]) {  // 241 (pcgpme_para.F90); pcgpme_2DH.f90:255
                 rn = tot[0];
                 c1n = tot[1];
-                beta = sh.s.mode == 2 ? c1n / (sh.s.AMU * sh.s.RQ) : c1n / sh.s.AMU / sh.s.RQ;
+                beta = div_by(c1n, sh.amu);                 // by AMU RQ in mode 2
+                if (sh.s.mode != 2) beta = div_by(beta, sh.rq);
                 sh.beta = beta;
             });
             if (*(volatile int*)&sh.stop) break;            // a poll ran out
