@@ -176,6 +176,19 @@ struct ResWait {
     }
 };
 
+// A coefficient's load, issued where it stands: before the poll whose wait hides it
+// (the compiler leaves plain loads behind the loop that precedes their use).
+__device__ __forceinline__ double ld_here(const double* p) {
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_here(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
 // Gather N words written at epoch `tag` (index `pad`: the zero row, not read).
 // Every lane of the warp calls it.
 template <typename T, int N>
@@ -482,21 +495,23 @@ struct Resident {
     __device__ __forceinline__ void axsub(const T* own, unsigned tag) const {
         rows2([&](const auto& rw) {
             constexpr int NR = std::extent<std::remove_reference_t<decltype(rw)>>::value;
-            T g[NR * NL], s[NR];
+            T g[NR * NL], a[NR * NL], s[NR];
             int c[NR * NL];
 #pragma unroll
             for (int r = 0; r < NR; r++) {
                 const int* cp = idx(rw[r]);
+                const T* ap = coef(rw[r]);
 #pragma unroll
                 for (int k = 0; k < NL; k++) c[r * NL + k] = cp[32 * k];
-                s[r] = own[rw[r].l] * coef(rw[r])[32 * NI];
+#pragma unroll
+                for (int k = 0; k < NL; k++) a[r * NL + k] = ld_here(ap + 32 * k);
+                s[r] = own[rw[r].l] * ap[32 * NI];
             }
             res_gather<T, NR * NL>(R.in, c, pad, tag, g, wt);
 #pragma unroll
             for (int r = 0; r < NR; r++) {
-                const T* a = coef(rw[r]);
 #pragma unroll
-                for (int k = 0; k < NL; k++) s[r] = fma_rn(a[32 * k], g[r * NL + k], s[r]);
+                for (int k = 0; k < NL; k++) s[r] = fma_rn(a[r * NL + k], g[r * NL + k], s[r]);
                 if (rw[r].ok) tag_put(R.t[0] + rw[r].i, s[r], tag);
             }
         });
@@ -508,10 +523,15 @@ struct Resident {
     __device__ __forceinline__ void pair(const ResRow (&rw)[NR], const TagWord<V>* in, unsigned tag, V (&o)[NR]) const {
         constexpr int s = S - 1;
         V g[NR * 4];
+        T a[NR * 3];
         int c[NR * 4];
 #pragma unroll
         for (int r = 0; r < NR; r++) {
             const int* cp = idx(rw[r]);
+            const T* ap = coef(rw[r]);
+            a[3 * r] = ld_here(ap + 32 * s);
+            a[3 * r + 1] = ld_here(ap + 32 * (s + 1));
+            a[3 * r + 2] = ld_here(ap + 32 * X);
             c[4 * r] = self(rw[r]);
             c[4 * r + 1] = cp[32 * s];
             c[4 * r + 2] = cp[32 * (s + 1)];
@@ -520,9 +540,8 @@ struct Resident {
         res_gather<V, NR * 4>(in, c, pad, tag, g, wt);
 #pragma unroll
         for (int r = 0; r < NR; r++) {
-            const T* a = coef(rw[r]);
-            const V o1 = fnma((V)a[32 * s], g[4 * r + 1], g[4 * r]);
-            o[r] = fnma((V)a[32 * (s + 1)], fnma((V)a[32 * X], g[4 * r + 3], g[4 * r + 2]), o1);
+            const V o1 = fnma((V)a[3 * r], g[4 * r + 1], g[4 * r]);
+            o[r] = fnma((V)a[3 * r + 1], fnma((V)a[3 * r + 2], g[4 * r + 3], g[4 * r + 2]), o1);
         }
     }
     template <int S, int X, typename V>
@@ -555,20 +574,21 @@ struct Resident {
             pair<3, NL + 1, V, NR>(rw, t[1], tag, o);
         } else {
             V g[NR * 3];
+            T a[NR * 2];
             int c[NR * 3];
 #pragma unroll
             for (int r = 0; r < NR; r++) {
                 const int* cp = idx(rw[r]);
+                a[2 * r] = ld_here(coef(rw[r]) + 32 * 4);
+                a[2 * r + 1] = ld_here(coef(rw[r]) + 32 * 5);
                 c[3 * r] = self(rw[r]);
                 c[3 * r + 1] = cp[32 * 4];
                 c[3 * r + 2] = cp[32 * 5];
             }
             res_gather<V, NR * 3>(t[2], c, pad, tag, g, wt);
 #pragma unroll
-            for (int r = 0; r < NR; r++) {
-                const T* a = coef(rw[r]);
-                o[r] = fnma((V)a[32 * 5], g[3 * r + 2], fnma((V)a[32 * 4], g[3 * r + 1], g[3 * r]));
-            }
+            for (int r = 0; r < NR; r++)
+                o[r] = fnma((V)a[2 * r + 1], g[3 * r + 2], fnma((V)a[2 * r], g[3 * r + 1], g[3 * r]));
         }
     }
     template <typename V>
