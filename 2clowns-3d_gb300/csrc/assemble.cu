@@ -53,10 +53,6 @@ __device__ __forceinline__ double cal_alu(double fnn, double dx, double dxm) {
     return (fnn - 0.5) * dx / (fnn * dx + dxm * 0.5) * (-1.0);
 }
 
-// Bit tests of doubles: an FP64 comparison costs as much as an addition.
-__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
-__device__ __forceinline__ bool is_one(double x) { return __double_as_longlong(x) == 0x3ff0000000000000LL; }
-
 // init_matrix (1sub-matrix.F90:25-65), one thread per cell nnn = 1..inne;
 // columns 2q, 2q+1 hold the minus and plus faces of axis col_axis(q).
 //
@@ -64,12 +60,13 @@ __device__ __forceinline__ bool is_one(double x) { return __double_as_longlong(x
 // does 1.7 lane operations per clock and SM, and cal_alu_f has three per face: the
 // kernel ran at 1.60 ms for 4.9 M cells (0.6 GB of traffic, 0.09 ms).  The factors
 // depend on one index of one axis, so every block forms the table of all of them in
-// shared memory (TAB; two blocks per SM walk all cells), and a face needs only the
-// products with its area and porosity where these are not 1.
+// shared memory (TAB; one block per SM walks its cells), and a face needs only the
+// products with its area and porosity where these are not 1; the six quotients by one
+// porosity take its reciprocal (Markstein).
 // TAB = false: grids whose table exceeds shared memory form every factor.
-constexpr int kInitBlock = 512;
+constexpr int kInitBlock = 1024;
 template <int NL, bool TAB>
-__global__ void __launch_bounds__(kInitBlock, 2) k_init_matrix(GridIdx g, int inne, int mx2, const int* __restrict__ mn,
+__global__ void __launch_bounds__(kInitBlock, 1) k_init_matrix(GridIdx g, int inne, int mx2, const int* __restrict__ mn,
                                                           const int* __restrict__ in_, const int* __restrict__ jn,
                                                           const int* __restrict__ kn, const int* __restrict__ nf,
                                                           const int* __restrict__ nfb, const double* __restrict__ a,
@@ -119,6 +116,8 @@ __global__ void __launch_bounds__(kInitBlock, 2) k_init_matrix(GridIdx g, int in
             fbp[c] = fb[np[c]];
         }
         const bool full = is_one(fbn);
+        Recip rfb = {};
+        if (TAB && !full) rfb = make_recip(fbn);
         double de = 0.0;
 #pragma unroll
         for (int c = 0; c < NL; c++) {                      // 3D: x-, x+, y-, y+, z-, z+
@@ -134,7 +133,7 @@ __global__ void __launch_bounds__(kInitBlock, 2) k_init_matrix(GridIdx g, int in
                 if (full && is_one(ar[c])) v = tab[2 * total + o];
                 else {
                     v = tab[o] * ar[c];
-                    if (!full) v = v / fbn;
+                    if (!full) v = div_by(v, rfb);
                     v = -(mp * v);
                 }
             } else {
@@ -266,7 +265,7 @@ __global__ void __launch_bounds__(kAsmBlock, 3) k_rhs(GridIdx g, int mm2, const 
             const int ip = mn[g.mn_off(i + 1, k, j)], jp = mn[g.mn_off(i, k, j + 1)], kp = mn[g.mn_off(i, k + 1, j)];
             auto flux = [&](int cell, int l) {              // u a, with most faces fully open
                 const double u = un[3L * cell + l], ar = a[3L * cell + l];
-                return is_one(ar) ? u : u * ar;
+                return unless(is_one(ar), u, [&] { return u * ar; });
             };
             const double qx = flux(ip, 0) - flux(c, 0);
             const double qy = flux(jp, 1) - flux(c, 1);
@@ -280,7 +279,7 @@ __global__ void __launch_bounds__(kAsmBlock, 3) k_rhs(GridIdx g, int mm2, const 
             } else {
                 rz = qx / dx[g.dxo(0, i)] + qy / dx[g.dxo(1, j)] + qz / dx[g.dxo(2, k)];
             }
-            if (!is_one(fbc)) rz = rz / fbc;
+            rz = unless(is_one(fbc), rz, [&] { return rz / fbc; });
         } else {
             rz = -10000.0;
         }
@@ -310,7 +309,7 @@ __global__ void __launch_bounds__(kAsmBlock, 3) k_rhs(GridIdx g, int mm2, const 
 // fluid-list entry.  Latency-bound (three levels of dependent gathers per column), so
 // the columns' loads are issued together, level by level: 229 us before at 2.8 M rows.
 template <int NL>
-__global__ void __launch_bounds__(kAsmBlock) k_assemble(GridIdx g, int ifln, long inne, long na, long spld,
+__global__ void __launch_bounds__(kAsmBlock, 4) k_assemble(GridIdx g, int ifln, long inne, long na, long spld,
                                                        const int* __restrict__ fln, const int* __restrict__ in_,
                                                        const int* __restrict__ jn, const int* __restrict__ kn,
                                                        const int* __restrict__ nf, const int* __restrict__ nfb,
@@ -471,7 +470,7 @@ extern "C" int clowns_init_matrix_dev(const int* dims, int inne, int mx2, const 
     const int entries = (g.ie - g.is + 3) + (g.je - g.js + 3) + (g.ke - g.ks + 3);
     const size_t tab = sizeof(double) * 4 * (size_t)entries;
     auto launch = [&](auto kern, size_t smem) {
-        const int blocks = (int)std::min<long>((inne + kInitBlock - 1L) / kInitBlock, smem ? 152L * 2 : 152L * 16);
+        const int blocks = (int)std::min<long>((inne + kInitBlock - 1L) / kInitBlock, smem ? 152L : 152L * 16);
         kern<<<blocks, kInitBlock, smem, s>>>(g, inne, mx2, mn, in_, jn, kn, nf, nfb, a, fb, dx, mp, alu_c, ll_c, de_c);
     };
     // the table fits the shared memory every launch may have up to 1536 cells in i + j + k

@@ -90,11 +90,27 @@ __device__ __forceinline__ void warp_sum_partials(const double* partials, int co
     for (int q = 0; q < NV; q++) out[q] = warp_sum(out[q]);
 }
 
+// Tests of doubles in integer registers: an FP64 comparison costs as much as an
+// addition.  (By words: the compiler turns a test of the whole 64 bits back into one.)
+__device__ __forceinline__ bool is_zero(double x) { return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0; }
+__device__ __forceinline__ bool is_one(double x) { return (__double2hiint(x) ^ 0x3ff00000 | __double2loint(x)) == 0; }
+
+// x when `skip`, else f(), which is not evaluated for a warp that skips it throughout
+// (the compiler would evaluate it for all and select).
+template <typename F>
+__device__ __forceinline__ double unless(bool skip, double x, F f) {
+    if (!skip) {
+        x = f();
+        asm volatile("" : "+d"(x));
+    }
+    return x;
+}
+
 // a / d with one rounding, given y = 1 / d rounded to nearest: Markstein's method (IBM
 // J. Res. Dev. 34, 1990).  a y, corrected once by its remainder, is within an ulp of the
 // quotient, and such a value corrected by its exact remainder times y rounds to it; the
-// remainders are exact while a and d are far from the ends of the exponent range, and
-// a zero keeps its sign only in a division, so those cases divide.  Five FP64 operations
+// remainders are exact while a and d are far from the ends of the exponent range;
+// outside they divide.  A zero's quotient is a y.  Five FP64 operations
 // instead of about ten.
 struct Recip {
     double d, y;
@@ -106,7 +122,7 @@ __device__ __forceinline__ bool mid_exponent(double x) {
 }
 __device__ __forceinline__ Recip make_recip(double d) { return Recip{d, 1.0 / d, mid_exponent(d)}; }
 __device__ __forceinline__ double div_by(double a, const Recip& r) {
-    if (!r.ok || !mid_exponent(a)) return a / r.d;
+    if (!r.ok || !mid_exponent(a)) return r.ok && is_zero(a) ? __dmul_rn(a, r.y) : a / r.d;
     const double q0 = __dmul_rn(a, r.y);
     const double q1 = __fma_rn(__fma_rn(-r.d, q0, a), r.y, q0);
     return __fma_rn(__fma_rn(-r.d, q1, a), r.y, q1);

@@ -210,8 +210,6 @@ __device__ __forceinline__ void res_gather(const TagWord<T>* __restrict__ buf, c
     }
 }
 
-// Integer forms of the scalar tests: an FP64 comparison costs as much as an addition.
-__device__ __forceinline__ bool f64_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
 __device__ __forceinline__ bool f64_finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
 
 // finish_sweep56's finalisations.
@@ -276,9 +274,9 @@ __device__ __forceinline__ void res_stop_tests(MemberScalars* S, ResStop& st, do
     st.q = q;
     st.rn_prev = RN;
     if (S->done) return;
-    if (f64_zero(S->AMU)) {                                      // 234
+    if (is_zero(S->AMU)) {                                      // 234
         stop_member(S, CLOWNS_STOP_AMU_ZERO, 0);
-    } else if (f64_zero(C1)) {                                   // 240
+    } else if (is_zero(C1)) {                                   // 240
         stop_member(S, CLOWNS_STOP_C1_ZERO, 0);
     } else {
         S->BETA = BETA;
