@@ -89,17 +89,7 @@ static int upload(void* dst, const void* src, size_t bytes, cudaStream_t s) {
     return CLOWNS_OK;
 }
 
-// A copy into host memory that no page backs yet (a fresh allocation) faults page by
-// page from the device's side: 27 ms for the 30 MB of a 128x128x48 session's fields,
-// against 0.8 ms into mapped memory.  The host maps it first.
-static void map_pages(void* p, size_t bytes) {
-    volatile char* c = (volatile char*)p;
-    for (size_t o = 0; o < bytes; o += 4096) c[o] = c[o];
-    if (bytes) c[bytes - 1] = c[bytes - 1];
-}
-
 static int download(void* dst, const void* src, size_t bytes, cudaStream_t s) {
-    map_pages(dst, bytes);
     CLOWNS_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
     return CLOWNS_OK;
 }
