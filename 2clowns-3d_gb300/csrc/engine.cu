@@ -288,7 +288,7 @@ static size_t res_smem_bytes(int per, int tsize) { return (size_t)tsize * kResVe
 static bool res_serves(int M, const int* n, int mixed) {
     long rows = 0;
     for (int m = 0; m < M; m++) rows += n[m];
-    if (2 * M > std::min(device_sms(), kResMaxBlocks) || 
+    if (2 * M > std::min(device_sms(), kResMaxBlocks) ||
         rows > (!mixed ? kResMaxRowsFp64 : M == 1 ? kResMaxRowsMixed : kResEnsRowsMixed))
         return false;
     std::vector<int> g;
@@ -839,7 +839,7 @@ static void g_iteration_bal(bool pdl, const Eng<T>& E, const Shape& sh, cudaStre
     apply((const T*)E.p, E.q, 1);                                                    // q = PM A p ; RQ ; ALP
     klaunch(pdl, k_bal_eupdate<T, R>, grid(kBalEu), B, s, E, tab(kBalEu));          // e = r - ALP q
     apply((const T*)E.e, E.v, 2);                                                    // v = PM A e ; AMU
-    klaunch(pdl, k_bal_xrupdate<T, R>, grid(kBalXr), B, s, E, tab(kBalXr));         // x, r ; RN, C1 ; stop tests
+    klaunch(pdl, k_bal_xrupdate<T, R>, grid(kBalXr), B, s, E, tab(kBalXr));         // r ; RN, C1 ; stop tests ; x, p - AMU q
     klaunch(pdl, k_bal_pupdate<T, R>, grid(kBalPu), B, s, E, tab(kBalPu));          // p
 }
 

@@ -1691,6 +1691,15 @@ __global__ void __launch_bounds__(kEngBlock, kBalMinBlocks<T, R>) k_bal_eupdate(
     }
 }
 
+// r and its dot products first; x, and p - AMU q for the p update, once the block's chunk
+// totals are out.  A dot-product kernel is bound by its tail: the chain of tickets from
+// the last chunk to the member's scalars (6-8 us), in which the other SMs had nothing to
+// do.  Here they stream x, p and q meanwhile, from the last chunk back, whose e is the
+// likeliest to be in L2 still; that costs 16 B more per row and saves 8 in the p update.
+// us per iteration before / now: FP64 125.2 / 119.0 at 826 k rows, 156.5 / 153.0 at 1.15 M,
+// 302.8 / 301.0 at 2.8 M (bound by HBM and the FP64 pipe); mixed 104.3 / 101.6 and 197.5 /
+// 192.1.  (Only x in the second part: 121.4, 154.8, 303.5; mixed 104.3, 195.6.  Second
+// part upwards: 302.7 at 2.8 M.)
 template <typename T, int R>
 __global__ void __launch_bounds__(kEngBlock, kBalMinBlocks<T, R>) k_bal_xrupdate(Eng<T> E, const BalBlock* __restrict__ tab) {
     pdl_trigger();
@@ -1698,8 +1707,6 @@ __global__ void __launch_bounds__(kEngBlock, kBalMinBlocks<T, R>) k_bal_xrupdate
         long plo, phi;
         if (pf_range(E, tab, plo, phi)) {
             pf_rows(E.e, plo, phi);
-            pf_rows(E.xi, plo, phi);
-            pf_rows(E.p, plo, phi);
             pf_rows(E.v, plo, phi);
             pf_rows(E.r0, plo, phi);
         }
@@ -1727,7 +1734,7 @@ __global__ void __launch_bounds__(kEngBlock, kBalMinBlocks<T, R>) k_bal_xrupdate
             for (int st = 0; st < kTreeSteps; st++) {
                 const int cb = c0 + nwarps * (s0 + st) + w;
                 if (s0 + st >= nsteps || cb >= c1) break;          // the same for the whole warp
-                T ev[R], xv[R], pv[R], vv[R], r0v[R];
+                T ev[R], vv[R], r0v[R];
                 bool ok[R];
                 long i[R];
 #pragma unroll
@@ -1736,8 +1743,6 @@ __global__ void __launch_bounds__(kEngBlock, kBalMinBlocks<T, R>) k_bal_xrupdate
                     ok[u] = r < n;
                     i[u] = off + (ok[u] ? r : 0);
                     ev[u] = ldg2(E.e + i[u]);
-                    xv[u] = ldg2(E.xi + i[u]);
-                    pv[u] = ldg2(E.p + i[u]);
                     vv[u] = ldg2(E.v + i[u]);
                     r0v[u] = ldg2(E.r0 + i[u]);
                 }
@@ -1745,7 +1750,6 @@ __global__ void __launch_bounds__(kEngBlock, kBalMinBlocks<T, R>) k_bal_xrupdate
 #pragma unroll
                 for (int u = 0; u < R; u++) {
                     if (!ok[u]) continue;
-                    E.xi[i[u]] = fma_rn(AMU, ev[u], fma_rn(ALP, pv[u], xv[u]));
                     const T rn = fnma(AMU, vv[u], ev[u]);
                     E.r[i[u]] = rn;
                     v0 = fma_rn(rn, rn, v0);
@@ -1767,7 +1771,7 @@ __global__ void __launch_bounds__(kEngBlock, kBalMinBlocks<T, R>) k_bal_xrupdate
 #pragma unroll
         for (int st = 0; st < SPB; st++) {
             const int cb = c0 + (nwarps * (s0 + st) + w) * CPS;
-            T ev[R], xv[R], pv[R], vv[R], r0v[R];
+            T ev[R], vv[R], r0v[R];
             bool ok[R];
 #pragma unroll
             for (int u = 0; u < R; u++) {
@@ -1776,8 +1780,6 @@ __global__ void __launch_bounds__(kEngBlock, kBalMinBlocks<T, R>) k_bal_xrupdate
                 ok[u] = cc < c1 && r < n;
                 const long i = off + (ok[u] ? r : 0);
                 ev[u] = ldg2(E.e + i);
-                xv[u] = ldg2(E.xi + i);
-                pv[u] = ldg2(E.p + i);
                 vv[u] = ldg2(E.v + i);
                 r0v[u] = ldg2(E.r0 + i);
             }
@@ -1785,7 +1787,6 @@ __global__ void __launch_bounds__(kEngBlock, kBalMinBlocks<T, R>) k_bal_xrupdate
             for (int u = 0; u < R; u++) {
                 if (!ok[u] || done) continue;
                 const long i = off + (long)(cb + u / kChunkRows) * kChunk + 32 * (u % kChunkRows) + lane;
-                E.xi[i] = fma_rn(AMU, ev[u], fma_rn(ALP, pv[u], xv[u]));
                 const T rn = fnma(AMU, vv[u], ev[u]);
                 E.r[i] = rn;
                 const int q = (st * CPS + u / kChunkRows) * 2;
@@ -1798,9 +1799,34 @@ __global__ void __launch_bounds__(kEngBlock, kBalMinBlocks<T, R>) k_bal_xrupdate
     }
     if (done) return;
     double tot[2];
-    if (!account_chunks(E, bb.m, c0, c1, tot) || lane != 0) return;
-    E.ticket[bb.m] = 0;
-    finish_xrupdate<true>(E.S + bb.m, tot, &s_pre);          // kernel completion publishes it
+    if (account_chunks(E, bb.m, c0, c1, tot) && lane == 0) {
+        E.ticket[bb.m] = 0;
+        finish_xrupdate<true>(E.S + bb.m, tot, &s_pre);      // kernel completion publishes it
+    }
+    __syncwarp();
+    // x is read and written once per iteration: evict-first, for the vectors gathered next
+    for (int sb = (c1 - c0 + nwarps * CPS - 1) / (nwarps * CPS) - 1; sb >= 0; sb--) {
+        const int cb = c0 + (sb * nwarps + w) * CPS;
+        if (cb >= c1) continue;
+        long i[R];
+        bool ok[R];
+        chunk_step<R>(off, n, cb, c1, i, ok);
+        T ev[R], xv[R], pv[R], qv[R];
+#pragma unroll
+        for (int u = 0; u < R; u++) {
+            ev[u] = ldg2(E.e + i[u]);
+            xv[u] = __ldcs(E.xi + i[u]);
+            pv[u] = ldg2(E.p + i[u]);
+            qv[u] = ldg2(E.q + i[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < R; u++) {
+            if (!ok[u]) continue;
+            __stcs(E.xi + i[u], fma_rn(AMU, ev[u], fma_rn(ALP, pv[u], xv[u])));
+            E.p[i[u]] = fnma(AMU, qv[u], pv[u]);
+        }
+        step_fence();
+    }
 }
 
 template <typename T, int R>
@@ -1810,30 +1836,28 @@ __global__ void __launch_bounds__(kEngBlock, kBalMinBlocks<T, R>) k_bal_pupdate(
     if (pf_range(E, tab, lo, hi)) {
         pf_rows(E.r, lo, hi);
         pf_rows(E.p, lo, hi);
-        pf_rows(E.q, lo, hi);
     }
     pdl_wait();
     BalBlock bb;
     long off;
     int n, c0, c1;
     if (!bal_block(E, tab, bb, off, n, c0, c1)) return;
-    const T BETA = T(sld(&E.S[bb.m].BETA)), AMU = T(sld(&E.S[bb.m].AMU));
+    const T BETA = T(sld(&E.S[bb.m].BETA));              // E.p holds p - AMU q (k_bal_xrupdate)
     constexpr int CPS = R / kChunkRows;
     const int nw = blockDim.x >> 5;
     for (int cb = c0 + bal_warp() * CPS; cb < c1; cb += nw * CPS) {
         long i[R];
         bool ok[R];
         chunk_step<R>(off, n, cb, c1, i, ok);
-        T rv[R], pv[R], qv[R];
+        T rv[R], pv[R];
 #pragma unroll
         for (int u = 0; u < R; u++) {
             rv[u] = ldg2(E.r + i[u]);
             pv[u] = ldg2(E.p + i[u]);
-            qv[u] = ldg2(E.q + i[u]);
         }
 #pragma unroll
         for (int u = 0; u < R; u++)
-            if (ok[u]) E.p[i[u]] = fma_rn(BETA, fnma(AMU, qv[u], pv[u]), rv[u]);
+            if (ok[u]) E.p[i[u]] = fma_rn(BETA, pv[u], rv[u]);
     }
 }
 

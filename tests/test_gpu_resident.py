@@ -66,6 +66,22 @@ def test_resident_equals_graph(gpu, monkeypatch, n, nl, kind):
         assert torch.equal(xr, xg), mixed
 
 
+@pytest.mark.parametrize("n", [1, 129, 257, 8193, 136193, 300000])
+def test_balanced_eight_rows_equals_resident(gpu, monkeypatch, n):
+    """The graph's balanced kernels at 8 rows per thread (two chunks per warp and step; the
+    r and the x / p parts of one kernel) at the edges of their chunk mapping."""
+    import torch
+    system = _system(n, 6, "band")
+    for mixed in (False, True):
+        _force(monkeypatch, "resident")
+        xr, ir = _solve(gpu, system, mixed, 1e-10)
+        _force(monkeypatch, "graph")
+        monkeypatch.setenv("CLOWNS_BALANCED_ROWS", "8")
+        xg, ig = _solve(gpu, system, mixed, 1e-10)
+        assert ir == ig, (mixed, ir, ig)
+        assert torch.equal(xr, xg), mixed
+
+
 def test_resident_ensemble_equals_graph(gpu, monkeypatch):
     """Members from one row to several blocks, four and six columns side by side, one
     with a NaN right-hand side: each ends as in the graph ensemble."""
