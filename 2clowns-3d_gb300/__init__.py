@@ -282,8 +282,9 @@ def set_nflag_dev(dc: DeviceCase):
     L = lib()
     case = dc.case
     ncell = case.inne2 + 2
-    fln = torch.zeros(ncell + 1, dtype=torch.int32, device="cuda")
-    sfn = torch.zeros(ncell + 1, dtype=torch.int32, device="cuda")
+    # the lists' entries in use are written by the call, and only those are returned
+    fln = torch.empty(ncell + 1, dtype=torch.int32, device="cuda")
+    sfn = torch.empty(ncell + 1, dtype=torch.int32, device="cuda")
     wbytes = L.clowns_set_nflag_workspace_bytes(dc.dims.numpy().ctypes.data, case.inne2)
     work = torch.empty(max(1, wbytes), dtype=torch.uint8, device="cuda")
     ifln, isfn, passes = C.c_int(0), C.c_int(0), C.c_int(0)
@@ -331,9 +332,10 @@ def rows_rhs_assemble_dev(dc: DeviceCase, fln, ifln: int, mp, alu_c, ll_c, de_c,
     is_, js, ks, ie, je, ke = (int(v) for v in case.dims)
     dims = dc.dims.numpy()
     mno = torch.empty((je, ke, ie), dtype=torch.int32, device="cuda")
-    mno2mn = torch.zeros(mm2, dtype=torch.int32, device="cuda")
+    mno2mn = torch.empty(mm2, dtype=torch.int32, device="cuda")
     b = torch.empty(mm2, dtype=torch.float64, device="cuda")
-    xe = torch.zeros(mm2 + 1, dtype=torch.float64, device="cuda")
+    xe = torch.empty(mm2 + 1, dtype=torch.float64, device="cuda")
+    xe[:1].zero_()                              # the rest is cleared by rows_rhs
     de = torch.empty(mm2, dtype=torch.float64, device="cuda")
     wbytes = L.clowns_rows_rhs_workspace_bytes(ifln)
     work = torch.empty(max(1, wbytes), dtype=torch.uint8, device="cuda")
@@ -346,10 +348,15 @@ def rows_rhs_assemble_dev(dc: DeviceCase, fln, ifln: int, mp, alu_c, ll_c, de_c,
                                _ptr(mno2mn), _ptr(b), _ptr(xe) + 8, _ptr(de), C.byref(mnoe), C.byref(dmax),
                                _ptr(work), wbytes, _stream())
     _check(rc, "rows_rhs")
-    nl = alu_c.shape[0]
-    alu = torch.zeros((nl, mm2), dtype=torch.float64, device="cuda")
-    llu = torch.zeros((nl, mm2), dtype=torch.int32, device="cuda")
-    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    # rows 1 .. mnoe are written whole; only the spare ones behind them need clearing (writing
+    # everything twice took 30 of 1105 us for a build of 2.8 M rows)
+    nl, n = alu_c.shape[0], mnoe.value
+    alu = torch.empty((nl, mm2), dtype=torch.float64, device="cuda")
+    llu = torch.empty((nl, mm2), dtype=torch.int32, device="cuda")
+    err = torch.empty(1, dtype=torch.int32, device="cuda")
+    alu[:, n:].zero_()
+    llu[:, n:].zero_()
+    mno2mn[n:].zero_()
     rc = L.clowns_assemble_dev(dims.ctypes.data, case.inne, case.inne2, case.mx2, _ptr(dc.in_), _ptr(dc.jn),
                                _ptr(dc.kn), _ptr(dc.nf), _ptr(dc.nfb), _ptr(dc.x), _ptr(dc.dx), _ptr(dc.sp),
                                ifln, flnp, _ptr(mno), _ptr(alu_c), _ptr(ll_c), _ptr(de_c), mm2, _ptr(alu),
@@ -379,12 +386,12 @@ PREC_MIXED = 1
 
 
 def tuned_shape(sizes, precision=0):
-    """Execution the autotuner chose for the iteration loop of this row space:
+    """Execution of the iteration loop of this row space (by size, or the autotuner's choice):
     {"mode": "graph", "block": .., "fused_sweeps": .., "reduce_block": ..,
     "balanced_rows": 0 | 4 | 8, "staged_axsub": ..} (balanced_rows > 0: one-wave
     kernels over even row ranges, that many rows per thread per step;
     staged_axsub: the FP32 AXSUB with its streams staged by bulk copies) or
-    {"mode": "persistent" | "wave", "block": .., "grid": .., "registers": ..},
+    {"mode": "resident" | "persistent" | "wave", "block": .., "grid": .., "registers": ..},
     or None before a solve of that size has run."""
     L = lib()
     arr = (C.c_int * len(sizes))(*[int(v) for v in sizes])
