@@ -337,6 +337,11 @@ def rows_rhs_assemble_dev(dc: DeviceCase, fln, ifln: int, mp, alu_c, ll_c, de_c,
     xe = torch.empty(mm2 + 1, dtype=torch.float64, device="cuda")
     xe[:1].zero_()                              # the rest is cleared by rows_rhs
     de = torch.empty(mm2, dtype=torch.float64, device="cuda")
+    # everything is allocated before the call that waits for the device, which has no work after it
+    nl = alu_c.shape[0]
+    alu = torch.empty((nl, mm2), dtype=torch.float64, device="cuda")
+    llu = torch.empty((nl, mm2), dtype=torch.int32, device="cuda")
+    err = torch.empty(1, dtype=torch.int32, device="cuda")
     wbytes = L.clowns_rows_rhs_workspace_bytes(ifln)
     work = torch.empty(max(1, wbytes), dtype=torch.uint8, device="cuda")
     mnoe = C.c_int(0)
@@ -348,20 +353,17 @@ def rows_rhs_assemble_dev(dc: DeviceCase, fln, ifln: int, mp, alu_c, ll_c, de_c,
                                _ptr(mno2mn), _ptr(b), _ptr(xe) + 8, _ptr(de), C.byref(mnoe), C.byref(dmax),
                                _ptr(work), wbytes, _stream())
     _check(rc, "rows_rhs")
-    # rows 1 .. mnoe are written whole; only the spare ones behind them need clearing (writing
-    # everything twice took 30 of 1105 us for a build of 2.8 M rows)
-    nl, n = alu_c.shape[0], mnoe.value
-    alu = torch.empty((nl, mm2), dtype=torch.float64, device="cuda")
-    llu = torch.empty((nl, mm2), dtype=torch.int32, device="cuda")
-    err = torch.empty(1, dtype=torch.int32, device="cuda")
-    alu[:, n:].zero_()
-    llu[:, n:].zero_()
-    mno2mn[n:].zero_()
     rc = L.clowns_assemble_dev(dims.ctypes.data, case.inne, case.inne2, case.mx2, _ptr(dc.in_), _ptr(dc.jn),
                                _ptr(dc.kn), _ptr(dc.nf), _ptr(dc.nfb), _ptr(dc.x), _ptr(dc.dx), _ptr(dc.sp),
                                ifln, flnp, _ptr(mno), _ptr(alu_c), _ptr(ll_c), _ptr(de_c), mm2, _ptr(alu),
                                _ptr(llu), _ptr(de), _ptr(err), _stream())
     _check(rc, "assemble")
+    # rows 1 .. mnoe are written whole; only the spare ones behind them need clearing (writing
+    # everything twice took 30 of 1105 us for a build of 2.8 M rows)
+    n = mnoe.value
+    alu[:, n:].zero_()
+    llu[:, n:].zero_()
+    mno2mn[n:].zero_()
     bad = int(err.item())
     if bad:
         raise ClownsError(f"cal_matrix_element: unexpected flag on row cell {bad}")
