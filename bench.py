@@ -56,8 +56,8 @@ def measured_peaks():
 # accumulation; 96 B for the FP64 -> FP32 conversion).
 # Measured DRAM bytes per row and iteration of the loop graph (ncu, the graph as
 # one unit, beach_256x256x96): profiles/pcgpme_loop_dram_beach_256x256x96.md.
-TRAFFIC_ROW_ITER_FP64 = 434.2
-TRAFFIC_ROW_ITER_MIXED = 224.6
+TRAFFIC_ROW_ITER_FP64 = 432.7
+TRAFFIC_ROW_ITER_MIXED = 224.2
 
 # What pins the CPU port: run on one thread it reproduces the reference's own
 # PCGPME, executed from its Fortran source, bit for bit.
@@ -736,6 +736,9 @@ def _report(pkg, args, world, rank, case, n, ms, infos, info, it, value, alg, ac
             err_mixed = float(np.linalg.norm(x_mixed - r.x) / nrm)
 
     if rank == 0:
+        shape = {"fp64": pkg.tuned_shape([n], 0), "mixed": pkg.tuned_shape([n], 1)}
+        resident = {k: (v or {}).get("mode") == "resident" for k, v in shape.items()}
+        solve_name = "pcgpme FP64 solve (one %s launch)" % ("resident-kernel" if resident["fp64"] else "graph")
         line = {
             "metric": "pressure solves/s", "value": value, "unit": "solves/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms / args.steps,
@@ -746,14 +749,16 @@ def _report(pkg, args, world, rank, case, n, ms, infos, info, it, value, alg, ac
                        "rel_l2_vs_oracle": err_plain, "true_rel_residual": args.res_plain,
                        "l2": "inputs larger than L2 (matrix %.0f MB)" % (n * 80 / 1e6),
                        "path": "plain FP64", "parallelism": f"replicas x{world}"},
-            "roofline": {"bound": "hbm", "kernel": "pcgpme FP64 solve (one graph launch)",
+            "roofline": {"bound": "hbm", "kernel": solve_name,
                          "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
-                         "frac": achieved / peak, "traffic": TRAFFIC_ROW_ITER_FP64 * n * it,
+                         "frac": achieved / peak,
+                         # a resident solve reads DRAM about once: profiles/pcgpme_resident_beach.md
+                         "traffic": None if resident["fp64"] else TRAFFIC_ROW_ITER_FP64 * n * it,
                          "traffic_source": "ncu DRAM bytes of the loop graph per row-iteration, "
                                            "profiles/pcgpme_loop_dram_beach_256x256x96.md",
                          "frac_with_index_streams": bytes_solve_fp64_with_indices(n, it) / alg * achieved / peak,
                          "algorithmic_bytes_per_solve": alg},
-            "roofline_fp64": {"bound": "fp64", "kernel": "pcgpme FP64 solve (one graph launch)",
+            "roofline_fp64": {"bound": "fp64", "kernel": solve_name,
                               "achieved": args.fma_achieved / 1e9, "peak": args.fma_peak / 1e9,
                               "peak_kind": "measured (clowns_fp64_fma_rate, this run)", "unit": "G FMA/s",
                               "frac": args.fma_achieved / args.fma_peak,
@@ -761,7 +766,7 @@ def _report(pkg, args, world, rank, case, n, ms, infos, info, it, value, alg, ac
             "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h},
             "gpu_launches": args.timed_launches,
-            "tuned_shape": {"fp64": pkg.tuned_shape([n], 0), "mixed": pkg.tuned_shape([n], 1)},
+            "tuned_shape": shape,
             "clocks": clk,
         }
         if minfo is not None:
@@ -770,7 +775,7 @@ def _report(pkg, args, world, rank, case, n, ms, infos, info, it, value, alg, ac
                              "rel_l2_vs_oracle": err_mixed, "true_rel_residual": args.res_mixed,
                              "ms_per_solve": ms_m / args.steps,
                              "achieved_gbs": m_alg / (ms_m / 1000.0 / args.steps) / 1e9,
-                             "traffic": TRAFFIC_ROW_ITER_MIXED * n * minfo.iter,
+                             "traffic": None if resident["mixed"] else TRAFFIC_ROW_ITER_MIXED * n * minfo.iter,
                              "algorithmic_bytes_per_solve": m_alg}
         if cpu:
             line["cpu_baseline"] = cpu
