@@ -229,10 +229,10 @@ static inline int member_groups(int n) {
 
 // Systems and ensembles of up to this many rows in all are solved resident, without
 // tuning.  Measured (ms per solve, the tuned graph / resident): single systems FP64
-// 2.7 / 0.8 at 4 k rows, 6.8 / 2.2 at 74 k, 10.5 / 5.2 at 239 k, 12.1 / 7.9 at 413 k,
-// 23.5 / 20.6 at 660 k (a block's vectors fill its shared memory at 720 k); mixed 3.7 /
-// 1.1, 5.8 / 1.9, 9.1 / 3.8, 10.9 / 6.0, 17.3 / 10.7, 19.7 / 15.1 at 960 k, 21.2 / 22.6
-// at 1.15 M (words and matrix no longer fit L2); ensembles FP64 5.5 / 2.5 at 16 members
+// 2.7 / 0.8 at 4 k rows, 6.8 / 2.2 at 74 k, 10.5 / 5.2 at 239 k, 12.0 / 7.4 at 413 k,
+// 23.2 / 19.1 at 660 k (a block's vectors fill its shared memory at 720 k); mixed 3.7 /
+// 1.1, 5.8 / 1.9, 9.1 / 3.8, 10.9 / 5.8, 17.0 / 10.7, 19.6 / 15.3 at 960 k, 20.6 / 18.6 at
+// 1.09 M, 21.2 / 22.6 at 1.15 M (words and matrix no longer fit L2); ensembles FP64 5.5 / 2.5 at 16 members
 // of 214 k rows, 9.2 / 5.0 at 12 of 407 k, 8.8 / 6.3 at 70 of 552 k; mixed 5.7 / 2.1, 7.0
 // / 3.5, 7.6 / 4.4, 10.8 / 7.5 at 40 of 1.01 M, 14.5 / 11.8 at 12 of 1.16 M.
 constexpr int kResMaxRowsFp64 = 700000;
