@@ -164,3 +164,38 @@ def test_resident_wait_runs_out_and_context_recovers(gpu, monkeypatch):
     assert "(-4)" in str(err.value), str(err.value)
     x, info = _solve(gpu, (al, ll, d, b), False, 1e-10)
     assert info == ok and torch.equal(x, x_ok)
+
+
+@pytest.mark.parametrize("sizes", [(8193, 8192), (300000, 19457), (300000, 300000)])
+def test_resident_solves_on_two_streams(gpu, monkeypatch, sizes):
+    """Two threads, a stream each, solve at the same time while ordinary kernels run on a
+    third stream: every solve gives the bits of the one that ran alone."""
+    import threading
+
+    import torch
+    _force(monkeypatch, "resident")
+    systems = [_system(n, 6, "band") for n in sizes]
+    alone = [[_solve(gpu, s, mixed, 1e-10) for mixed in (False, True)] for s in systems]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(8):
+                    for mixed in (False, True):
+                        x, info = _solve(gpu, systems[k], mixed, 1e-10)
+                        if info != alone[k][mixed][1] or not torch.equal(x, alone[k][mixed][0]):
+                            bad.append((k, mixed, info))
+        except Exception as e:
+            bad.append((k, e))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    a = torch.randn(2048, 2048, device="cuda")
+    for t in threads:
+        t.start()
+    while any(t.is_alive() for t in threads):
+        (a @ a).sum().item()
+    for t in threads:
+        t.join()
+    assert not bad
