@@ -298,7 +298,11 @@ struct ResShared {
     ResStop st;
     Recip rq, amu;       // reciprocals for BETA, formed while others compute
     int fail;            // a poll ran out
-    int stop;            // the scalar warp's verdict at the last reduction: leave the loop
+    // The scalar warp's verdicts (leave the loop), a word for each reduction: once a poll has
+    // given up, that warp no longer waits for the row warps' contributions and may reach the
+    // next verdict while a row warp still has to read this one.  With one word the row
+    // warps could part there, and those that went on wait for the others without a limit.
+    int stop[kResReds];
 };
 
 // The butterfly over lanes of which only the first cnt hold terms: the levels that
@@ -429,14 +433,13 @@ struct Resident {
     unsigned row0;
     TagWord<double>*part, *gpart;
 
-    // false: a stopped member, none of its blocks works
     __device__ __forceinline__ Resident(const Eng<T>& E_, const ResBufs<T>& R_, ResShared& sh_, double* vecs, long limit)
         : E(E_), R(R_), sh(sh_), wt{limit, E_.abort, &sh_.fail} {
         lane = threadIdx.x & 31;
         w = threadIdx.x >> 5;
         nw = ws = (blockDim.x >> 5) - 1;
         bal_block(E, R.tab, bb, off, n, c0, c1);
-        if (threadIdx.x == 0) sh.fail = sh.stop = 0;
+        if (threadIdx.x == 0) sh.fail = 0;
         copy_scalars(sh.s, E.S + bb.m);
         __syncthreads();
         nc = (n + kChunk - 1) / kChunk;
@@ -652,7 +655,8 @@ struct Resident {
         });
     }
     // The member's totals of reduction `red` and what follows from them: fin(totals) in
-    // one thread; every thread then knows whether to go on.
+    // one thread; every thread then knows whether to go on.  A reduction never follows
+    // itself, so a verdict is written over only after another reduction's barrier.
     template <int NVAL, typename F>
     __device__ __forceinline__ bool totals(int red, unsigned tag, F fin) const {
         if (w == ws) {
@@ -660,11 +664,11 @@ struct Resident {
             res_totals<NVAL>(part + red * pstride, gpart + red * gstride, nc, c0, c1, tag, wt, tot);
             if (lane == 0) {
                 fin(tot);
-                sh.stop = sh.s.done || *(volatile int*)&sh.fail;
+                sh.stop[red] = sh.s.done || *(volatile int*)&sh.fail;
             }
         }
         __syncthreads();
-        return sh.stop == 0;
+        return sh.stop[red] == 0;
     }
     // The iterations of one (inner) solve from r = p = r0, x, BN and C1; ep: epochs used so
     // far, each iteration takes two.
@@ -730,7 +734,7 @@ struct Resident {
                 if (sh.s.mode != 2) beta = div_by(beta, sh.rq);
                 sh.beta = beta;
             });
-            if (*(volatile int*)&sh.stop) break;            // a poll ran out
+            if (sh.stop[2]) break;                          // a poll ran out
             // the stop tests, while the row warps start the next iteration; the verdict counts
             // at its first reduction
             if (w == ws && lane == 0) res_stop_tests(&sh.s, sh.st, rn, c1n, beta);
