@@ -1577,6 +1577,8 @@ int engine_solve_mixed(int M, const MemberIn* ins, double eps, double parm, doub
                    s, &sh);
     if (rc) return rc;
     t_launches = 0;
+    // a solve that needs no inner loop reads the abort flag too, and only the loops clear it
+    CLOWNS_CUDA_TRY(cudaMemsetAsync(gb, 0, sizeof(GridBar), s));
     setup(s);
     t_launches += 7;
     CLOWNS_CUDA_TRY(cudaGetLastError());
