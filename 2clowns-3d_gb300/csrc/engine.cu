@@ -238,6 +238,9 @@ static inline int member_groups(int n) {
 constexpr int kResMaxRowsFp64 = 700000;
 constexpr int kResMaxRowsMixed = 1100000;
 constexpr int kResEnsRowsMixed = 1250000;
+static long res_max_rows(int M, int mixed) {
+    return !mixed ? kResMaxRowsFp64 : M == 1 ? kResMaxRowsMixed : kResEnsRowsMixed;
+}
 constexpr int kResMaxBlocks = kNumSMs;
 constexpr size_t kResMaxSmem = 224 * 1024;      // a block's rows of its vectors: 37 chunks in FP64, 74 in FP32
 
@@ -288,9 +291,7 @@ static size_t res_smem_bytes(int per, int tsize) { return (size_t)tsize * kResVe
 static bool res_serves(int M, const int* n, int mixed) {
     long rows = 0;
     for (int m = 0; m < M; m++) rows += n[m];
-    if (2 * M > std::min(device_sms(), kResMaxBlocks) ||
-        rows > (!mixed ? kResMaxRowsFp64 : M == 1 ? kResMaxRowsMixed : kResEnsRowsMixed))
-        return false;
+    if (2 * M > std::min(device_sms(), kResMaxBlocks) || rows > res_max_rows(M, mixed)) return false;
     std::vector<int> g;
     return res_smem_bytes(res_blocks(M, n, g), mixed ? 4 : 8) <= kResMaxSmem;
 }
@@ -309,20 +310,24 @@ struct EngLayout {
     size_t total = 0;
 };
 
-// wave: -1 = the wavefront loop's buffers for single systems (M == 1), 0 = none.
-static EngLayout eng_layout(int M, const int* n, int mixed, int wave = -1) {
+// Padded rows and reduction groups of all members.
+static void row_space(int M, const int* n, long* NV, int* ngrp) {
+    *NV = 0;
+    *ngrp = 0;
+    for (int m = 0; m < M; m++) {
+        *NV += (long)align_up((size_t)n[m] + 1, kTile);
+        *ngrp += member_groups(n[m]);
+    }
+}
+
+// wave: the wavefront loop's buffers; res: the resident solve's, behind all others, so
+// that the rest lies the same with and without them.
+static EngLayout eng_layout(int M, long NV, int ngrp, int mixed, bool wave, bool res) {
     EngLayout L;
     L.M = M;
     L.mixed = mixed;
-    L.wave = wave < 0 ? (M == 1) : wave;
-    L.n1 = M == 1 ? n[0] : 0;
+    L.wave = wave;
     L.tsize = mixed ? 4 : 8;
-    long NV = 0;
-    int ngrp = 0;
-    for (int m = 0; m < M; m++) {
-        NV += (long)align_up((size_t)n[m] + 1, kTile);
-        ngrp += member_groups(n[m]);
-    }
     L.NV = NV;
     L.nblk = (int)(NV / kTile);
     L.ngrp = ngrp;
@@ -367,7 +372,11 @@ static EngLayout eng_layout(int M, const int* n, int mixed, int wave = -1) {
         L.o_wave = 0;
         for (int k = 0; k < kWaveBufs; k++) L.o_wbuf[k] = 0;
     }
-    L.res = wave < 0 && res_serves(M, n, mixed);
+    if (M > 1) {
+        L.o_baltab = take(sizeof(BalBlock) * 16 * (size_t)kBalTabMax);
+        L.o_balg = take(sizeof(int) * 16);
+    }
+    L.res = res;
     if (L.res) {
         for (int k = 0; k < 1 + kResSteps; k++) L.o_rword[k] = take(2 * (size_t)L.tsize * NV);
         if (mixed)
@@ -377,12 +386,28 @@ static EngLayout eng_layout(int M, const int* n, int mixed, int wave = -1) {
         L.o_ra = take((size_t)L.tsize * kResCoef<6> * NV);
         L.o_rc = take(sizeof(int) * kResIdx<6> * (size_t)NV);
     }
-    if (M > 1) {
-        L.o_baltab = take(sizeof(BalBlock) * 16 * (size_t)kBalTabMax);
-        L.o_balg = take(sizeof(int) * 16);
-    }
     L.total = o;
     return L;
+}
+
+static EngLayout eng_layout(int M, const int* n, int mixed, bool res) {
+    long NV;
+    int ngrp;
+    row_space(M, n, &NV, &ngrp);
+    EngLayout L = eng_layout(M, NV, ngrp, mixed, M == 1, res);
+    L.n1 = M == 1 ? n[0] : 0;
+    return L;
+}
+
+// The layout of a solve in work_bytes: with the resident solve's buffers where it serves
+// the sizes and they fit.  A workspace that holds the rest only is not refused: the
+// solve then takes the general path, with the same bits.
+static EngLayout solve_layout(int M, const int* n, int mixed, size_t work_bytes) {
+    if (res_serves(M, n, mixed)) {
+        const EngLayout L = eng_layout(M, n, mixed, true);
+        if (L.total <= work_bytes) return L;
+    }
+    return eng_layout(M, n, mixed, false);
 }
 
 // Matrix columns the balanced kernels keep in L2 (the first ones of the sorted
@@ -1303,12 +1328,12 @@ int engine_tuned_shape(long nv, int prec, int single, int* mode, int* block, int
     return CLOWNS_OK;
 }
 
-long engine_row_space(int M, const int* n, int mixed) { return eng_layout(M, n, mixed).NV; }
+long engine_row_space(int M, const int* n, int mixed) { return eng_layout(M, n, mixed, false).NV; }
 
 long engine_last_launches() { return t_launches; }
 
 double* engine_residual_ptr(void* work, int n) {
-    return (double*)((char*)work + eng_layout(1, &n, 0).o_vec[0]);
+    return (double*)((char*)work + eng_layout(1, &n, 0, false).o_vec[0]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1348,11 +1373,28 @@ static int read_results(void* work, const EngLayout& L, cudaStream_t s, clowns_s
     return CLOWNS_OK;
 }
 
-size_t engine_workspace_bytes(int M, const int* n, int mixed) {
+size_t engine_least_bytes(int M, const int* n, int mixed) {
     if (M < 1) return 0;
     for (int m = 0; m < M; m++)
         if (n[m] < 1) return 0;
-    return eng_layout(M, n, mixed).total;
+    return eng_layout(M, n, mixed, false).total;
+}
+
+// Enough for the same number of members of any smaller sizes too: a caller sizes its
+// workspace for its largest row count and solves fewer rows in it.  Sizes past the
+// resident solve's rows therefore hold the buffers of the largest that it serves.
+size_t engine_workspace_bytes(int M, const int* n, int mixed) {
+    const size_t least = engine_least_bytes(M, n, mixed);
+    if (!least || 2 * M > kResMaxBlocks) return least;
+    long NV;
+    int ngrp;
+    row_space(M, n, &NV, &ngrp);
+    const long most = (long)align_up((size_t)res_max_rows(M, mixed) + M, kTile) + (long)(M - 1) * kTile;
+    if (NV > most) {
+        NV = most;
+        ngrp = std::min(ngrp, (int)(most / (kChunk * kGroupChunks)) + M);
+    }
+    return std::max(least, eng_layout(M, NV, ngrp, mixed, M == 1, true).total);
 }
 
 static int check_members(int M, const MemberIn* ins, std::vector<int>& n, int* nl_out) {
@@ -1446,7 +1488,7 @@ int engine_solve_plain(int M, const MemberIn* ins, double eps, double parm, int 
     int nl = 6;
     int rc = check_members(M, ins, n, &nl);
     if (rc) return rc;
-    EngLayout L = eng_layout(M, n.data(), 0);
+    const EngLayout L = solve_layout(M, n.data(), 0, work_bytes);
     if (!work || work_bytes < L.total) {
         set_last_error_msg("pcgpme: workspace too small");
         return CLOWNS_ERR_WORKSPACE;
@@ -1527,7 +1569,7 @@ int engine_solve_mixed(int M, const MemberIn* ins, double eps, double parm, doub
     int nl = 6;
     int rc = check_members(M, ins, n, &nl);
     if (rc) return rc;
-    EngLayout L = eng_layout(M, n.data(), 1);
+    const EngLayout L = solve_layout(M, n.data(), 1, work_bytes);
     if (!work || work_bytes < L.total) {
         set_last_error_msg("pcgpme_mixed: workspace too small");
         return CLOWNS_ERR_WORKSPACE;
@@ -1614,7 +1656,7 @@ int engine_setup_export(const MemberIn& in, double parm, double* al_s, int* ll_s
     int nl;
     int rc = check_members(1, &in, n, &nl);
     if (rc) return rc;
-    EngLayout L = eng_layout(1, n.data(), 0);
+    const EngLayout L = eng_layout(1, n.data(), 0, false);
     if (!work || work_bytes < L.total) {
         set_last_error_msg("setup: workspace too small");
         return CLOWNS_ERR_WORKSPACE;
@@ -1647,7 +1689,7 @@ int engine_apply_pm_a(const MemberIn& in, double parm, const double* x, double* 
     int nl;
     int rc = check_members(1, &in, n, &nl);
     if (rc) return rc;
-    EngLayout L = eng_layout(1, n.data(), 0);
+    const EngLayout L = eng_layout(1, n.data(), 0, false);
     if (!work || work_bytes < L.total) {
         set_last_error_msg("apply: workspace too small");
         return CLOWNS_ERR_WORKSPACE;
@@ -1771,7 +1813,11 @@ extern "C" int clowns_pcgpme_static_dev(const double* al, int nl, int na, const 
     void* work = nullptr;
     int rc = static_scratch(&work);
     if (rc) return rc;
-    EngLayout L = eng_layout(1, &n, 0, 0);
+    long NV;
+    int ngrp;
+    row_space(1, &n, &NV, &ngrp);
+    EngLayout L = eng_layout(1, NV, ngrp, 0, false, false);
+    L.n1 = n;
     if (L.total > kStaticBytes || L.nblk > kStaticMaxBlk) {
         set_last_error_msg("pcgpme_static: layout exceeds the static scratch");
         return CLOWNS_ERR_LIMIT;

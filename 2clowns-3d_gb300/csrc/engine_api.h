@@ -9,7 +9,10 @@ namespace clowns {
 
 struct MemberIn;
 
+// Workspace to ask for (also for smaller sizes of as many members), and the least that
+// a solve of these sizes accepts.
 size_t engine_workspace_bytes(int M, const int* n, int mixed);
+size_t engine_least_bytes(int M, const int* n, int mixed);
 // variant 0: PCGPME (pcgpme_para.F90); 2: PCGPME_WILL's iteration (pcgpme_2DH.f90:
 // BETA = C1 / (AMU RQ), eps and iter taken as given, iter >= 1).
 int engine_solve_plain(int M, const MemberIn* ins, double eps, double parm, int iter, void* work,

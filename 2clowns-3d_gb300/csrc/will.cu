@@ -84,8 +84,9 @@ static int will_postprocess(const double* x, const double* r, const int* ll, int
     return CLOWNS_ERR_NOCONV;
 }
 
+// The engine's part is last: it takes what the workspace has beyond the rest.
 struct WillLayout {
-    size_t o_x, o_post, o_eng, eng_bytes, total;
+    size_t o_x, o_post, o_eng, least, total;
 };
 
 static WillLayout will_layout(int n) {
@@ -94,9 +95,9 @@ static WillLayout will_layout(int n) {
     auto take = [&](size_t bytes) { size_t at = o; o = align_up(o + bytes, 256); return at; };
     L.o_x = take(sizeof(double) * (size_t)n);
     L.o_post = take(will_post_bytes(n));
-    L.eng_bytes = engine_workspace_bytes(1, &n, 0);
-    L.o_eng = take(L.eng_bytes);
-    L.total = o;
+    L.o_eng = o;
+    L.least = o + engine_least_bytes(1, &n, 0);
+    L.total = align_up(o + engine_workspace_bytes(1, &n, 0), 256);
     return L;
 }
 
@@ -118,7 +119,7 @@ extern "C" int clowns_pcgpme_will_dev(const double* al, int nl, int na, const in
         return CLOWNS_ERR_ARG;
     }
     const WillLayout L = will_layout(n);
-    if (work_bytes < L.total) {
+    if (work_bytes < L.least) {
         set_last_error_msg("pcgpme_will: workspace too small");
         return CLOWNS_ERR_WORKSPACE;
     }
@@ -131,7 +132,7 @@ extern "C" int clowns_pcgpme_will_dev(const double* al, int nl, int na, const in
     in.na = na; in.n = n; in.nl = nl; in.pad = 0;
     clowns_solve_info local;
     clowns_solve_info* inf = info ? info : &local;
-    int rc = engine_solve_plain(1, &in, eps, parm, iter, w + L.o_eng, L.eng_bytes, s, inf, 2);
+    int rc = engine_solve_plain(1, &in, eps, parm, iter, w + L.o_eng, work_bytes - L.o_eng, s, inf, 2);
     if (rc) return rc;
     if (inf->ier == CLOWNS_IER_ARG) {
         set_last_error_msg("pcgpme_will: a column index is outside 0..n");

@@ -29,7 +29,9 @@
  * Functions whose name ends in _dev take DEVICE pointers and a cudaStream_t
  * (as void*; NULL = legacy default stream) and allocate nothing: scratch space
  * is a caller-provided device workspace whose size a *_workspace_bytes query
- * returns.  Functions without the suffix take HOST pointers, manage device
+ * returns.  A solve's workspace serves all smaller systems too (ensembles: as many
+ * members, none larger), so one sized for the largest row count does for every step.
+ * Functions without the suffix take HOST pointers, manage device
  * memory inside the library and return when the results are back on the host.
  *
  * Return codes: 0 on success, a negative CLOWNS_ERR_* value on failure (the

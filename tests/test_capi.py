@@ -58,3 +58,25 @@ def test_will_dropin_rejects_bad_arguments_without_a_gpu(pkg):
     assert L.clowns_pcgpme_will_workspace_bytes(0, 4) == 0
     assert L.clowns_pcgpme_will_workspace_bytes(100, 5) == 0
     assert L.clowns_pcgpme_will_workspace_bytes(100, 4) > 0
+
+
+def test_solve_workspaces_serve_all_smaller_systems(pkg):
+    """Workspace sizes never shrink with the rows, across the limits up to which solves
+    run resident (and need more) as elsewhere: a host that sizes its workspace for the
+    largest row count solves fewer rows in it.  Ensembles: with each member's rows."""
+    import ctypes as C
+    L = pkg.lib()
+    rows = [1, 1023, 1024, 32768, 300000, 690000, 699999, 700000, 700001, 700415, 700416, 710000, 1000000, 1099999,
+            1100000, 1100001, 1200000, 1250000, 1250001, 1340000, 2000000, 2350000, 2400000, 8550000]
+    for f in (L.clowns_pcgpme_workspace_bytes, L.clowns_pcgpme_mixed_workspace_bytes,
+              L.clowns_pcgpme_will_workspace_bytes):
+        sizes = [f(n, 4) for n in rows]
+        assert sizes == sorted(sizes), (f.__name__, sizes)
+    for m in (2, 12, 76, 77):
+        for prec in (0, 1):
+            def size(ns):
+                return L.clowns_pcgpme_batched_workspace_bytes(m, (C.c_int * m)(*ns), prec)
+            even = [size([max(1, n // m)] * m) for n in rows]
+            assert even == sorted(even), (m, prec, even)
+            one = [size([n] + [1000] * (m - 1)) for n in rows]
+            assert one == sorted(one), (m, prec, one)
