@@ -10,6 +10,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <tuple>
 #include <type_traits>
@@ -680,6 +681,16 @@ static std::mutex g_loop_mu;
 // (row space, precision, wave loop available, forced execution or -1): a forced
 // execution is tuned among its own shapes and never served an automatic pick.
 static std::map<std::tuple<long, int, int, int>, LoopShape> g_loop_shapes;
+// Row spaces (padded rows, members, precision, forced execution or -1) whose last solve ran
+// resident; for clowns_tuned_shape only.  Kept apart from the tuner's table: a row space
+// may hold systems on both sides of the resident solve's limits.
+static std::set<std::tuple<long, int, int, int>> g_resident;
+static void note_route(const EngLayout& L, bool resident) {
+    const auto key = std::make_tuple(L.NV, L.M, L.mixed, forced_loop_mode());
+    std::lock_guard<std::mutex> lk(g_loop_mu);
+    if (resident) g_resident.insert(key);
+    else g_resident.erase(key);
+}
 
 template <typename T>
 static int loop_max_grid(int block, int minb, int* out, bool wave = false) {
@@ -1106,13 +1117,17 @@ static int run_loop(Eng<T> E, const void* work, GridBar* gb, int prec, const Loo
         t_launches += 1;
         return CLOWNS_OK;
     }
-    if (sh.graph) {
+    if (sh.graph == 1) {
         cudaGraphExec_t ex;
         int rc = loop_graph(E, work, prec, sh.fuse, sh.rblock, sh.bal, sh.stg, &ex);
         if (rc) return rc;
         CLOWNS_CUDA_TRY(cudaMemsetAsync(gb, 0, sizeof(GridBar), s));
         CLOWNS_CUDA_TRY(cudaGraphLaunch(ex, s));
         return CLOWNS_OK;     // bodies are counted from ctrl[0] + ctrl[2] after the solve
+    }
+    if (sh.graph != 0) {
+        set_last_error_msg("pcgpme: unknown execution of the iteration loop");
+        return CLOWNS_ERR_ARG;
     }
     int grid = std::max(1, std::min(sh.grid, E.nblk));
     CLOWNS_CUDA_TRY(cudaMemsetAsync(gb, 0, sizeof(GridBar), s));
@@ -1312,12 +1327,17 @@ static int tune_loop(Eng<T> E, const void* work, GridBar* gb, long key_nv, int k
 // mode: 0 persistent, 1 CUDA graph, 3 wavefront; fuse (graph): bit 0 fused sweep
 // pairs, bit 1 dot-product kernels at 64 threads per tile, bit 2 balanced
 // one-wave kernels (bit 3: 8 rows per thread per step, else 4), bit 4 the
-// staged FP32 AXSUB
-int engine_tuned_shape(long nv, int prec, int single, int* mode, int* block, int* grid, int* minb, int* fuse) {
+// staged FP32 AXSUB.  A resident solve's shape (mode 4) follows from the sizes.
+int engine_tuned_shape(int M, const int* n, int mixed, int* mode, int* block, int* grid, int* minb, int* fuse) {
+    for (int m = 0; m < M; m++)
+        if (n[m] < 1) return CLOWNS_ERR_ARG;
+    const long nv = eng_layout(M, n, mixed, false).NV;
+    std::vector<int> g;
     std::lock_guard<std::mutex> lk(g_loop_mu);
-    auto it = g_loop_shapes.find(std::make_tuple(nv, prec, single, forced_loop_mode()));
-    if (it == g_loop_shapes.end()) return CLOWNS_ERR_ARG;
-    const LoopShape& sh = it->second;
+    const bool resident = res_serves(M, n, mixed) && g_resident.count(std::make_tuple(nv, M, mixed, forced_loop_mode()));
+    auto it = g_loop_shapes.find(std::make_tuple(nv, mixed, (int)(M == 1), forced_loop_mode()));
+    if (!resident && it == g_loop_shapes.end()) return CLOWNS_ERR_ARG;
+    const LoopShape sh = resident ? res_shape(M, g, res_blocks(M, n, g), nullptr) : it->second;
     *mode = sh.graph;
     *block = sh.block;
     *grid = sh.graph == 1 ? 0 : sh.grid;
@@ -1327,8 +1347,6 @@ int engine_tuned_shape(long nv, int prec, int single, int* mode, int* block, int
                           : 0;
     return CLOWNS_OK;
 }
-
-long engine_row_space(int M, const int* n, int mixed) { return eng_layout(M, n, mixed, false).NV; }
 
 long engine_last_launches() { return t_launches; }
 
@@ -1473,10 +1491,7 @@ static int solve_resident(const EngLayout& L, const int* n, const MemberIn* ins,
         CLOWNS_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(sh.grid), dim3(sh.block), args, smem, s));
     }
     t_launches = 3;
-    {
-        std::lock_guard<std::mutex> lk(g_loop_mu);            // for clowns_tuned_shape
-        g_loop_shapes[std::make_tuple(L.NV, (int)mixed, (int)(L.M == 1), forced_loop_mode())] = sh;
-    }
+    note_route(L, true);
     return read_results(work, L, s, info, mixed, sh);
 }
 
@@ -1538,6 +1553,7 @@ int engine_solve_plain(int M, const MemberIn* ins, double eps, double parm, int 
     };
     LoopShape sh;
     // tuning runs: kTuneIters iterations from the real start (not counted as the solve's launches)
+    note_route(L, false);
     rc = tune_loop(E, work, gb, L.NV, 0, [&](cudaStream_t cs) { prime(cs, 1e-300, kTuneIters); start(cs); }, s, &sh);
     if (rc) return rc;
     t_launches = 0;
@@ -1615,6 +1631,7 @@ int engine_solve_mixed(int M, const MemberIn* ins, double eps, double parm, doub
         k_mx_normalize<float><<<kg, ksh.block, 0, cs>>>(E);
     };
     LoopShape sh;
+    note_route(L, false);
     rc = tune_loop(E, work, gb, L.NV, 1, [&](cudaStream_t cs) { setup(cs); sweep_head(cs, 1e-30, kTuneIters); },
                    s, &sh);
     if (rc) return rc;

@@ -109,7 +109,7 @@ extern "C" int clowns_tuned_shape(int m, const int* n, int precision, int* mode,
     }
     const int mixed = precision == CLOWNS_PREC_MIXED;
     int minb = 0;
-    int rc = engine_tuned_shape(engine_row_space(m, n, mixed), mixed, m == 1, mode, block, grid, &minb, fused);
+    int rc = engine_tuned_shape(m, n, mixed, mode, block, grid, &minb, fused);
     if (rc) {
         set_last_error_msg("tuned_shape: no solve of this size has run yet");
         return rc;
