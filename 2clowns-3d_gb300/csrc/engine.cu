@@ -1328,7 +1328,7 @@ static int tune_loop(Eng<T> E, const void* work, GridBar* gb, long key_nv, int k
 // pairs, bit 1 dot-product kernels at 64 threads per tile, bit 2 balanced
 // one-wave kernels (bit 3: 8 rows per thread per step, else 4), bit 4 the
 // staged FP32 AXSUB.  A resident solve's shape (mode 4) follows from the sizes.
-int engine_tuned_shape(int M, const int* n, int mixed, int* mode, int* block, int* grid, int* minb, int* fuse) {
+int engine_tuned_shape(int M, const int* n, int mixed, int* mode, int* block, int* grid, int* regs, int* fuse) {
     for (int m = 0; m < M; m++)
         if (n[m] < 1) return CLOWNS_ERR_ARG;
     const long nv = eng_layout(M, n, mixed, false).NV;
@@ -1341,7 +1341,7 @@ int engine_tuned_shape(int M, const int* n, int mixed, int* mode, int* block, in
     *mode = sh.graph;
     *block = sh.block;
     *grid = sh.graph == 1 ? 0 : sh.grid;
-    *minb = sh.graph == 1 ? 0 : sh.minb;
+    *regs = sh.graph == 1 ? 0 : sh.graph == 4 ? kResRegs : 65536 / (sh.minb * sh.block) & ~7;
     *fuse = sh.graph == 1 ? (sh.fuse | (sh.rblock != kStepBlock ? 2 : 0) | (sh.bal ? 4 : 0) | (sh.bal == 8 ? 8 : 0) |
                              (sh.stg ? 16 : 0))
                           : 0;

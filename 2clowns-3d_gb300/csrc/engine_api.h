@@ -27,7 +27,7 @@ int engine_setup_export(const MemberIn& in, double parm, double* al_s, int* ll_s
 int engine_apply_pm_a(const MemberIn& in, double parm, const double* x, double* y, void* work,
                       size_t work_bytes, cudaStream_t s);
 void release_all_graphs();
-int engine_tuned_shape(int M, const int* n, int mixed, int* mode, int* block, int* grid, int* minb, int* fuse);
+int engine_tuned_shape(int M, const int* n, int mixed, int* mode, int* block, int* grid, int* regs, int* fuse);
 long engine_last_launches();
 // Test hook: the next plain solve's cooperative loop kernel waits at most
 // `limit` polls per device-wide wait and its block `absent` leaves at once.

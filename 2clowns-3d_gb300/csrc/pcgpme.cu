@@ -108,14 +108,9 @@ extern "C" int clowns_tuned_shape(int m, const int* n, int precision, int* mode,
         return CLOWNS_ERR_ARG;
     }
     const int mixed = precision == CLOWNS_PREC_MIXED;
-    int minb = 0;
-    int rc = engine_tuned_shape(m, n, mixed, mode, block, grid, &minb, fused);
-    if (rc) {
-        set_last_error_msg("tuned_shape: no solve of this size has run yet");
-        return rc;
-    }
-    *regs = minb > 0 ? (65536 / (minb * *block)) & ~7 : 0;   // register budget of a co-resident kernel
-    return CLOWNS_OK;
+    int rc = engine_tuned_shape(m, n, mixed, mode, block, grid, regs, fused);
+    if (rc) set_last_error_msg("tuned_shape: no solve of this size has run yet");
+    return rc;
 }
 
 extern "C" long clowns_last_kernel_launches(void) { return engine_last_launches(); }

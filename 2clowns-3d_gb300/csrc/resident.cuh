@@ -52,7 +52,8 @@
 namespace clowns {
 
 constexpr int kResWarps = 28;                    // row warps of a block at most
-constexpr int kResThreads = 32 * kResWarps + 32; // and the scalar warp: 64 registers per thread
+constexpr int kResThreads = 32 * kResWarps + 32; // and the scalar warp
+constexpr int kResRegs = 65536 / kResThreads & ~7;  // 64 registers per thread, at any launch size
 constexpr int kResReds = 5;                      // RQ, AMU, RN, and two of the mixed path's refinement: a
                                                  // reduction's words are written again only after another one
 constexpr int kResVecs = 6;                      // vectors a block keeps in shared memory

@@ -70,3 +70,12 @@ def test_single_systems_of_one_row_space(gpu, monkeypatch, prec, limit):
     monkeypatch.delenv("CLOWNS_LOOP_MODE", raising=False)
     shapes = [_check(gpu, [n], prec, n <= limit)[1] for n in (limit, limit + 1, limit, limit + 1)]
     assert shapes[0] == shapes[2] and shapes[1] == shapes[3]
+
+
+@pytest.mark.parametrize("sizes", [[100], [5000], [300000], [900, 40, 7000]], ids=str)
+def test_resident_register_budget(gpu, monkeypatch, sizes):
+    """The resident kernel is built for 29 warps of 64 registers and launched with that
+    or fewer."""
+    monkeypatch.delenv("CLOWNS_LOOP_MODE", raising=False)
+    shape = _solve(gpu, sizes, 0)[2]
+    assert shape["mode"] == "resident" and shape["registers"] == 64, shape
