@@ -108,6 +108,7 @@ _SIGS = {
     "clowns_last_kernel_launches": (C.c_long, []),
     "clowns_fp64_fma_rate": (C.c_int, [C.c_void_p, C.c_void_p]),
     "clowns_test_arm_wait_timeout": (C.c_int, [C.c_long, C.c_int]),
+    "clowns_test_arm_launch_refusal": (C.c_int, []),
     "clowns_session_create": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int] + [C.c_void_p] * 7),
     "clowns_session_set_fields": (C.c_int, [C.c_void_p] * 9),
     "clowns_session_classify": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),

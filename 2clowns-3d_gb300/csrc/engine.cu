@@ -4,6 +4,7 @@
 // stop tests clear it), the plain FP64 path and the mixed-precision path
 // (FP32 storage, FP64 iterative refinement).
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <climits>
@@ -245,28 +246,15 @@ static long res_max_rows(int M, int mixed) {
 constexpr int kResMaxBlocks = kNumSMs;
 constexpr size_t kResMaxSmem = 224 * 1024;      // a block's rows of its vectors: 37 chunks in FP64, 74 in FP32
 
-static int device_sms() {
-    static const int sms = [] {
-        int dev = 0, v = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1) {
-            cudaGetLastError();
-            v = kNumSMs;
-        }
-        return v;
-    }();
-    return sms;
-}
-
 // Blocks of each member in the resident solve: at most one per SM, dealt in proportion
 // to the members' chunks (a block takes its member's next even share).  Returns the
-// largest number of chunks of a block.
-static int res_blocks(int M, const int* n, std::vector<int>& g) {
+// largest number of chunks of a block.  M <= sms.
+static int res_blocks(int M, const int* n, int sms, std::vector<int>& g) {
     std::vector<int> nc(M);
     g.assign(M, 0);
     long total = 0;
     for (int m = 0; m < M; m++) total += nc[m] = (n[m] + kChunk - 1) / kChunk;
-    const int G = (int)std::min<long>(total, std::min(device_sms(), kResMaxBlocks));
+    const int G = (int)std::min<long>(total, std::min(sms, kResMaxBlocks));
     int used = 0;
     for (int m = 0; m < M; m++) used += g[m] = (int)std::max<long>(1, std::min<long>(nc[m], (long)G * nc[m] / total));
     // the largest share per block gets the next block; a surplus comes from the smallest
@@ -289,12 +277,27 @@ static int res_blocks(int M, const int* n, std::vector<int>& g) {
 }
 static size_t res_smem_bytes(int per, int tsize) { return (size_t)tsize * kResVecs * kChunk * per; }
 
+// By the sizes and the whole GPU's SMs alone: workspace queries need no device.  A solve
+// that finds fewer SMs deals its blocks anew (res_deal).
 static bool res_serves(int M, const int* n, int mixed) {
     long rows = 0;
     for (int m = 0; m < M; m++) rows += n[m];
-    if (2 * M > std::min(device_sms(), kResMaxBlocks) || rows > res_max_rows(M, mixed)) return false;
+    if (2 * M > kResMaxBlocks || rows > res_max_rows(M, mixed)) return false;
     std::vector<int> g;
-    return res_smem_bytes(res_blocks(M, n, g), mixed ? 4 : 8) <= kResMaxSmem;
+    return res_smem_bytes(res_blocks(M, n, kResMaxBlocks, g), mixed ? 4 : 8) <= kResMaxSmem;
+}
+
+// Blocks of the members on the current device; false where it has too few SMs for them.
+static bool res_deal(int M, const int* n, int mixed, std::vector<int>& g, int& per) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (2 * M > sms) return false;
+    per = res_blocks(M, n, sms, g);
+    return res_smem_bytes(per, mixed ? 4 : 8) <= kResMaxSmem;
 }
 
 struct EngLayout {
@@ -1333,11 +1336,12 @@ int engine_tuned_shape(int M, const int* n, int mixed, int* mode, int* block, in
         if (n[m] < 1) return CLOWNS_ERR_ARG;
     const long nv = eng_layout(M, n, mixed, false).NV;
     std::vector<int> g;
+    int per = 0;
     std::lock_guard<std::mutex> lk(g_loop_mu);
-    const bool resident = res_serves(M, n, mixed) && g_resident.count(std::make_tuple(nv, M, mixed, forced_loop_mode()));
+    const bool resident = res_serves(M, n, mixed) && res_deal(M, n, mixed, g, per) && g_resident.count(std::make_tuple(nv, M, mixed, forced_loop_mode()));
     auto it = g_loop_shapes.find(std::make_tuple(nv, mixed, (int)(M == 1), forced_loop_mode()));
     if (!resident && it == g_loop_shapes.end()) return CLOWNS_ERR_ARG;
-    const LoopShape sh = resident ? res_shape(M, g, res_blocks(M, n, g), nullptr) : it->second;
+    const LoopShape sh = resident ? res_shape(M, g, per, nullptr) : it->second;
     *mode = sh.graph;
     *block = sh.block;
     *grid = sh.graph == 1 ? 0 : sh.grid;
@@ -1449,9 +1453,16 @@ static cudaError_t res_smem(const void* fn, size_t bytes) {
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResMaxSmem);
 }
 
+// Test hook (clowns_test_arm_launch_refusal): the next resident launch is refused.
+static std::atomic<bool> g_refuse{false};
+void engine_arm_launch_refusal() { g_refuse = true; }
+
 // A solve in three kernels -- setup, composed coefficients, and the whole of the rest
 // resident -- between one upload (tables, inputs, initial scalars, a cleared abort
-// flag) and one read-back (scalars and abort flag).
+// flag) and one read-back (scalars and abort flag).  kResRefused: this context does not
+// give the launch a block per SM (fewer SMs than the device's, shared memory); nothing
+// is in flight and the solve takes the general path.
+constexpr int kResRefused = 1;
 template <typename T>
 static int solve_resident(const EngLayout& L, const int* n, const MemberIn* ins, const MemberScalars& init, int nl,
                           double P1, double P2, double inner_tol, int inner_max, void* work, cudaStream_t s,
@@ -1460,7 +1471,8 @@ static int solve_resident(const EngLayout& L, const int* n, const MemberIn* ins,
     std::vector<char> t = eng_tables(L, n, ins);
     for (int m = 0; m < L.M; m++) ((MemberScalars*)(t.data() + L.o_S))[m] = init;
     std::vector<int> g;
-    const int per = res_blocks(L.M, n, g);
+    int per;
+    if (!res_deal(L.M, n, mixed, g, per)) return kResRefused;
     const size_t smem = res_smem_bytes(per, L.tsize);
     const LoopShape sh = res_shape(L.M, g, per, L.M > 1 ? (BalBlock*)(t.data() + L.o_restab) : nullptr);
     CLOWNS_CUDA_TRY(cudaMemcpyAsync(work, t.data(), L.o_tables, cudaMemcpyHostToDevice, s));
@@ -1476,19 +1488,29 @@ static int solve_resident(const EngLayout& L, const int* n, const MemberIn* ins,
         k_eng_setup<T, 4><<<gs, kEngBlock, 0, s>>>(E, P1, P2, mixed);
         k_res_compose<T, 4><<<gs, kEngBlock, 0, s>>>(E, R);
     }
+    CLOWNS_CUDA_TRY(cudaGetLastError());
     long lim;
     int absent;
     wait_params(!mixed, &lim, &absent);
+    auto launch = [&](const void* fn, void** args) -> cudaError_t {
+        if (g_refuse.exchange(false)) return cudaErrorCooperativeLaunchTooLarge;
+        const cudaError_t e = res_smem(fn, smem);
+        return e != cudaSuccess ? e : cudaLaunchCooperativeKernel(fn, dim3(sh.grid), dim3(sh.block), args, smem, s);
+    };
+    cudaError_t e;
     if constexpr (mixed) {
         void* args[] = {(void*)&E, (void*)&R, (void*)&inner_tol, (void*)&inner_max, (void*)&lim, (void*)&absent};
         const void* fn = nl == 4 ? (const void*)k_res_mixed<4> : (const void*)k_res_mixed<6>;
-        CLOWNS_CUDA_TRY(res_smem(fn, smem));
-        CLOWNS_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(sh.grid), dim3(sh.block), args, smem, s));
+        e = launch(fn, args);
     } else {
         void* args[] = {(void*)&E, (void*)&R, (void*)&lim, (void*)&absent};
         const void* fn = nl == 4 ? (const void*)k_res_plain<4> : (const void*)k_res_plain<6>;
-        CLOWNS_CUDA_TRY(res_smem(fn, smem));
-        CLOWNS_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(sh.grid), dim3(sh.block), args, smem, s));
+        e = launch(fn, args);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        CLOWNS_CUDA_TRY(cudaStreamSynchronize(s));               // an earlier fault shows here
+        return kResRefused;
     }
     t_launches = 3;
     note_route(L, true);
@@ -1526,7 +1548,8 @@ int engine_solve_plain(int M, const MemberIn* ins, double eps, double parm, int 
         init.EPS = eps_r;
         init.ITER = iter_r;
         init.mode = mode;
-        return solve_resident<double>(L, n.data(), ins, init, nl, P1, P2, 0.0, 0, work, s, info);
+        rc = solve_resident<double>(L, n.data(), ins, init, nl, P1, P2, 0.0, 0, work, s, info);
+        if (rc != kResRefused) return rc;
     }
     rc = eng_upload_tables(work, L, n.data(), ins, s);
     if (rc) return rc;
@@ -1602,7 +1625,8 @@ int engine_solve_mixed(int M, const MemberIn* ins, double eps, double parm, doub
         init.EPS64 = eps_r;
         init.OITER = max_outer;
         init.mode = 1;
-        return solve_resident<float>(L, n.data(), ins, init, nl, P1, P2, inner_tol, inner_max, work, s, info);
+        rc = solve_resident<float>(L, n.data(), ins, init, nl, P1, P2, inner_tol, inner_max, work, s, info);
+        if (rc != kResRefused) return rc;
     }
     rc = eng_upload_tables(work, L, n.data(), ins, s);
     if (rc) return rc;

@@ -32,5 +32,7 @@ long engine_last_launches();
 // Test hook: the next plain solve's cooperative loop kernel waits at most
 // `limit` polls per device-wide wait and its block `absent` leaves at once.
 void engine_arm_wait_fault(long limit, int absent);
+// Test hook: the next resident launch is refused.
+void engine_arm_launch_refusal();
 
 }  // namespace clowns

@@ -184,3 +184,8 @@ extern "C" int clowns_test_arm_wait_timeout(long polls, int absent_block) {
     engine_arm_wait_fault(polls, absent_block);
     return CLOWNS_OK;
 }
+
+extern "C" int clowns_test_arm_launch_refusal(void) {
+    engine_arm_launch_refusal();
+    return CLOWNS_OK;
+}

@@ -148,6 +148,11 @@ module clowns_gpu
             integer(c_int), value :: absent_block
         end function clowns_test_arm_wait_timeout
 
+        integer(c_int) function clowns_test_arm_launch_refusal() &
+                bind(C, name="clowns_test_arm_launch_refusal")
+            import :: c_int
+        end function clowns_test_arm_launch_refusal
+
         integer(c_long) function clowns_last_kernel_launches() bind(C, name="clowns_last_kernel_launches")
             import :: c_long
         end function clowns_last_kernel_launches

@@ -204,6 +204,11 @@ int clowns_tuned_shape(int m, const int* n, int precision, int* mode, int* block
  * one solve, then disarms; later solves on the same context run normally. */
 int clowns_test_arm_wait_timeout(long polls, int absent_block);
 
+/* Test hook: the launch of the next resident solve (CLOWNS_LOOP_RESIDENT) is refused
+ * as by a context that cannot hold its blocks at once; nothing is launched, and the
+ * solve takes the general path.  Applies to one solve. */
+int clowns_test_arm_launch_refusal(void);
+
 /* Kernels the calling thread's last solve (plain or mixed, single or batched)
  * launched: host launches plus the kernel nodes its loop graphs executed
  * (per iteration 16 with single LDUSUB sweeps, 12 with fused sweep pairs, the

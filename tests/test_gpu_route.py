@@ -79,3 +79,35 @@ def test_resident_register_budget(gpu, monkeypatch, sizes):
     monkeypatch.delenv("CLOWNS_LOOP_MODE", raising=False)
     shape = _solve(gpu, sizes, 0)[2]
     assert shape["mode"] == "resident" and shape["registers"] == 64, shape
+
+
+@pytest.mark.parametrize("sizes", [[5000], [129, 4097, 900]], ids=str)
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "mixed"])
+def test_refused_launch_takes_the_general_path(gpu, monkeypatch, prec, sizes):
+    """A context without room for one block per SM refuses the cooperative launch; the
+    solve then runs as systems past the limits do, with the same bits, and the next one
+    is resident again."""
+    import torch
+    monkeypatch.delenv("CLOWNS_LOOP_MODE", raising=False)
+    xs, infos, shape, _ = _solve(gpu, sizes, prec)
+    assert shape["mode"] == "resident"
+    assert gpu.lib().clowns_test_arm_launch_refusal() == 0
+    xr, infor, shaper, launches = _solve(gpu, sizes, prec)
+    assert shaper["mode"] != "resident" and launches > 3
+    assert [i.as_dict() for i in infor] == [i.as_dict() for i in infos]
+    assert all(torch.equal(a, b) for a, b in zip(xs, xr))
+    assert _solve(gpu, sizes, prec)[2] == shape
+
+
+def test_refused_launch_of_the_2dh_solve(gpu, monkeypatch):
+    import torch
+    monkeypatch.delenv("CLOWNS_LOOP_MODE", raising=False)
+    al, ll, d, b = _band(5000, 4)
+    got = []
+    for refuse in (False, True):
+        if refuse:
+            assert gpu.lib().clowns_test_arm_launch_refusal() == 0
+        rhs = b.clone()
+        info = gpu.WillSolver(5000).solve(al, ll, d, rhs, eps=1e-10)
+        got.append((info.as_dict(), rhs))
+    assert got[0][0] == got[1][0] and torch.equal(got[0][1], got[1][1])
