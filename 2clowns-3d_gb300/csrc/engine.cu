@@ -1034,8 +1034,8 @@ static long loop_launches(const LoopShape& sh, long bodies) {
 }
 
 // Test hook of the bounded device waits (clowns_test_arm_wait_timeout): the
-// next solve whose loop runs as one cooperative kernel gives every wait
-// `limit` polls and makes block `absent` leave without arriving.  One use.
+// next resident solve, or plain FP64 solve whose loop runs as one cooperative
+// kernel, gives every wait `limit` polls and makes block `absent` leave without arriving.  One use.
 struct WaitFault {
     long limit = kBarSpinLimit;
     int absent = -1;
@@ -1491,7 +1491,7 @@ static int solve_resident(const EngLayout& L, const int* n, const MemberIn* ins,
     CLOWNS_CUDA_TRY(cudaGetLastError());
     long lim;
     int absent;
-    wait_params(!mixed, &lim, &absent);
+    wait_params(true, &lim, &absent);
     auto launch = [&](const void* fn, void** args) -> cudaError_t {
         if (g_refuse.exchange(false)) return cudaErrorCooperativeLaunchTooLarge;
         const cudaError_t e = res_smem(fn, smem);

@@ -194,9 +194,10 @@ int clowns_tuned_shape(int m, const int* n, int precision, int* mode, int* block
                        int* fused);
 
 /* Test hook of failure detection (no counterpart in the reference): the next
+ * solve that runs resident (CLOWNS_LOOP_RESIDENT; any precision, ensembles too), or
  * plain FP64 solve whose iteration loop runs as one cooperative kernel
  * (CLOWNS_LOOP_PERSISTENT or CLOWNS_LOOP_WAVE, e.g. forced by
- * CLOWNS_LOOP_MODE=persistent|wave) gives every device-wide wait `polls` polls
+ * CLOWNS_LOOP_MODE=persistent|wave), gives every device-wide wait `polls` polls
  * instead of 2^24 and makes its block `absent_block` leave the kernel without
  * arriving anywhere.  The other blocks' waits then run out: they raise the
  * abort flag and return, nothing hangs or faults, and the solve reports
