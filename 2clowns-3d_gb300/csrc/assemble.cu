@@ -539,7 +539,7 @@ extern "C" int clowns_rows_rhs_dev(const int* dims, int inne2, int mx2, const in
         // take the count from the device, the host reads it with dmax at the end
         const int tiles = (int)rows_tiles(ifln);
         k_row_flags<<<tiles, kBitThreads, 0, s>>>(g, ifln, fln, mn, in_, jn, kn, nf, nfb, fb, mask, sums);
-        int rc = scan_tiles_dev(1, sums, ifln, nullptr, &out->mnoe, s);
+        int rc = scan_tiles_dev(1, sums, ifln, &out->mnoe, s);
         if (rc) return rc;
         k_row_scatter<<<tiles, kBitThreads, 0, s>>>(g, ifln, mm2, fln, in_, jn, kn, mask, sums, mno, mno2mn);
         // the reciprocals leave three blocks per SM their shared memory up to 3072 cells in i + j + k

@@ -81,8 +81,8 @@ __device__ __forceinline__ void bit_prefix(const unsigned* words, int* pre) {
     pre[lane] = x - c;
 }
 
-// Exclusive scan of the tiles' counts (`lists` of them, 1 or 2, interleaved) in place
-// and their totals; nt_p: the number of tiles on the device (nullptr: all of n).
-int scan_tiles_dev(int lists, int* sums, long n, const int* nt_p, int* totals, cudaStream_t s);
+// Exclusive scan of the counts of n positions' tiles (`lists` of them, 1 or 2,
+// interleaved) in place and their totals.
+int scan_tiles_dev(int lists, int* sums, long n, int* totals, cudaStream_t s);
 
 }  // namespace clowns

@@ -490,7 +490,7 @@ extern "C" int clowns_set_nflag_dev(const int* dims, int inne, int inne2, int mx
         // the lists, and the surface loops as far as they change nothing, with one read-back
         CLOWNS_CUDA_TRY(cudaMemsetAsync(W.ctr + kCtrUnsettled, 0, sizeof(int), s));
         k_surface_flags<<<tiles, kBitThreads, 0, s>>>(A, W.ctr, W.wet, W.surf, W.sums);
-        int rc = scan_tiles_dev(2, W.sums, (long)nf_box(dims), nullptr, W.ctr + kCtrWet, s);
+        int rc = scan_tiles_dev(2, W.sums, (long)nf_box(dims), W.ctr + kCtrWet, s);
         if (rc) return rc;
         k_surface_scatter<<<tiles, kBitThreads, 0, s>>>(A, W.ctr, W.wet, W.surf, W.sums, fln, sfn, W.spos_cell);
         k_surface_check<<<152 * 4, kNfBlock, 0, s>>>(A, f, sfn, W.spos_cell, W.bout, W.ctr);

@@ -6,12 +6,10 @@
 namespace clowns {
 
 // One block scans the tiles' counts in place, NV interleaved lists at once; totals[k]
-// is list k's sum.  nt: tiles, read from the device where the caller knows only a bound.
+// is list k's sum.
 template <int NV>
-__global__ void __launch_bounds__(1024) k_scan_tiles(int* __restrict__ sums, int nt, const int* __restrict__ nt_p,
-                                                     int* __restrict__ totals) {
+__global__ void __launch_bounds__(1024) k_scan_tiles(int* __restrict__ sums, int nt, int* __restrict__ totals) {
     __shared__ int sm[NV][32];
-    if (nt_p) nt = min(nt, *nt_p);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int per = (nt + 1023) / 1024, lo = threadIdx.x * per;
     int s[NV], x[NV];
@@ -46,10 +44,10 @@ __global__ void __launch_bounds__(1024) k_scan_tiles(int* __restrict__ sums, int
         }
 }
 
-int scan_tiles_dev(int lists, int* sums, long n, const int* nt_p, int* totals, cudaStream_t s) {
+int scan_tiles_dev(int lists, int* sums, long n, int* totals, cudaStream_t s) {
     const int nt = (int)((n + kBitTile - 1) / kBitTile);
-    if (lists == 1) k_scan_tiles<1><<<1, 1024, 0, s>>>(sums, nt, nt_p, totals);
-    else k_scan_tiles<2><<<1, 1024, 0, s>>>(sums, nt, nt_p, totals);
+    if (lists == 1) k_scan_tiles<1><<<1, 1024, 0, s>>>(sums, nt, totals);
+    else k_scan_tiles<2><<<1, 1024, 0, s>>>(sums, nt, totals);
     CLOWNS_CUDA_TRY(cudaGetLastError());
     return CLOWNS_OK;
 }
