@@ -230,13 +230,16 @@ static inline int member_groups(int n) {
 }
 
 // Systems and ensembles of up to this many rows in all are solved resident, without
-// tuning.  Measured (ms per solve, the tuned graph / resident): single systems FP64
+// tuning, unless a block gets more chunks than its limit (uneven ensembles: every member
+// takes at least one block).  Measured (ms per solve, the tuned graph / resident): single systems FP64
 // 2.7 / 0.8 at 4 k rows, 6.8 / 2.2 at 74 k, 10.5 / 5.2 at 239 k, 12.0 / 7.4 at 413 k,
-// 23.2 / 19.1 at 660 k (a block's vectors fill its shared memory at 720 k); mixed 3.7 /
-// 1.1, 5.8 / 1.9, 9.1 / 3.8, 10.9 / 5.8, 17.0 / 10.7, 19.6 / 15.3 at 960 k, 20.6 / 18.6 at
-// 1.09 M, 21.2 / 22.6 at 1.15 M (words and matrix no longer fit L2); ensembles FP64 5.5 / 2.5 at 16 members
-// of 214 k rows, 9.2 / 5.0 at 12 of 407 k, 8.8 / 6.3 at 70 of 552 k; mixed 5.7 / 2.1, 7.0
-// / 3.5, 7.6 / 4.4, 10.8 / 7.5 at 40 of 1.01 M, 14.5 / 11.8 at 12 of 1.16 M.
+// 23.2 / 19.1 at 660 k; mixed 3.7 / 1.1, 5.8 / 1.9, 9.1 / 3.8, 10.9 / 5.8, 17.0 / 10.7, 19.6 / 15.3 at 960 k,
+// 20.6 / 18.6 at 1.09 M, 21.2 / 22.6 at 1.15 M (words and matrix no longer fit L2).
+// Ensembles, us per iteration, graph / resident (rows of a uniform grid; in brackets with
+// coefficients drawn for each row by itself, whose gathers scatter most): FP64 119 / 46 at 76
+// members of 389 k rows, 116 / 59 at one of 408 k beside 69 of 10 rows, 123 / 91 (130 / 109) at
+// 12 of 664 k; mixed 107 / 55 at 76 of 817 k, 133 / 100 (142 / 120) at 76 of 1.245 M, 145 /
+// 109 (149 / 143) at 2 of 1.245 M.
 constexpr int kResMaxRowsFp64 = 700000;
 constexpr int kResMaxRowsMixed = 1100000;
 constexpr int kResEnsRowsMixed = 1250000;
@@ -244,7 +247,15 @@ static long res_max_rows(int M, int mixed) {
     return !mixed ? kResMaxRowsFp64 : M == 1 ? kResMaxRowsMixed : kResEnsRowsMixed;
 }
 constexpr int kResMaxBlocks = kNumSMs;
-constexpr size_t kResMaxSmem = 224 * 1024;      // a block's rows of its vectors: 37 chunks in FP64, 74 in FP32
+// Chunks of a block at most: graph / resident, us per iteration, rows as in the brackets
+// above, FP64 132 / 119 at 37 chunks (12 members); mixed 125 / 123 at 65, 127 / 125 at
+// 70 (ten rounds of the 28 warps), 131 / 141 at 74 (40 members).
+static int res_max_chunks(int mixed) { return mixed ? 70 : 37; }
+// Shared memory of a block that leaves its L1 cache 60 KB for the matrix.  A block whose six
+// vectors take more (33 chunks in FP64, 65 in FP32) leaves r0 in global memory: with
+// all six there, past 192 KB, 28 KB of L1 were left, and the same rows took 153 us (153 /
+// 111 at 642 k rows, the graph 114; uneven grids of 690 k rows with porosities 119 / 99, the graph 113).
+constexpr size_t kResL1Smem = 192 * 1024;
 
 // Blocks of each member in the resident solve: at most one per SM, dealt in proportion
 // to the members' chunks (a block takes its member's next even share).  Returns the
@@ -275,7 +286,10 @@ static int res_blocks(int M, const int* n, int sms, std::vector<int>& g) {
     for (int m = 0; m < M; m++) per = std::max(per, (nc[m] + g[m] - 1) / g[m]);
     return per;
 }
-static size_t res_smem_bytes(int per, int tsize) { return (size_t)tsize * kResVecs * kChunk * per; }
+static bool res_far_r0(int per, int tsize) { return (size_t)tsize * kResVecs * kChunk * per > kResL1Smem; }
+static size_t res_smem_bytes(int per, int tsize) {
+    return (size_t)tsize * (kResVecs - res_far_r0(per, tsize)) * kChunk * per;
+}
 
 // By the sizes and the whole GPU's SMs alone: workspace queries need no device.  A solve
 // that finds fewer SMs deals its blocks anew (res_deal).
@@ -284,7 +298,7 @@ static bool res_serves(int M, const int* n, int mixed) {
     for (int m = 0; m < M; m++) rows += n[m];
     if (2 * M > kResMaxBlocks || rows > res_max_rows(M, mixed)) return false;
     std::vector<int> g;
-    return res_smem_bytes(res_blocks(M, n, kResMaxBlocks, g), mixed ? 4 : 8) <= kResMaxSmem;
+    return res_blocks(M, n, kResMaxBlocks, g) <= res_max_chunks(mixed);
 }
 
 // Blocks of the members on the current device; false where it has too few SMs for them.
@@ -297,7 +311,7 @@ static bool res_deal(int M, const int* n, int mixed, std::vector<int>& g, int& p
     }
     if (2 * M > sms) return false;
     per = res_blocks(M, n, sms, g);
-    return res_smem_bytes(per, mixed ? 4 : 8) <= kResMaxSmem;
+    return per <= res_max_chunks(mixed);
 }
 
 struct EngLayout {
@@ -1450,7 +1464,7 @@ static bool res_chosen(const EngLayout& L) {
 // Shared memory (the static part included) beyond the 48 KB a kernel may have without asking.
 static cudaError_t res_smem(const void* fn, size_t bytes) {
     if (bytes + sizeof(ResShared) <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResMaxSmem);
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResL1Smem);
 }
 
 // Test hook (clowns_test_arm_launch_refusal): the next resident launch is refused.
@@ -1498,14 +1512,15 @@ static int solve_resident(const EngLayout& L, const int* n, const MemberIn* ins,
         return e != cudaSuccess ? e : cudaLaunchCooperativeKernel(fn, dim3(sh.grid), dim3(sh.block), args, smem, s);
     };
     cudaError_t e;
+    const bool far = res_far_r0(per, L.tsize);
     if constexpr (mixed) {
         void* args[] = {(void*)&E, (void*)&R, (void*)&inner_tol, (void*)&inner_max, (void*)&lim, (void*)&absent};
-        const void* fn = nl == 4 ? (const void*)k_res_mixed<4> : (const void*)k_res_mixed<6>;
-        e = launch(fn, args);
+        e = launch(nl == 4 ? (far ? (const void*)k_res_mixed<4, true> : (const void*)k_res_mixed<4, false>)
+                           : (far ? (const void*)k_res_mixed<6, true> : (const void*)k_res_mixed<6, false>), args);
     } else {
         void* args[] = {(void*)&E, (void*)&R, (void*)&lim, (void*)&absent};
-        const void* fn = nl == 4 ? (const void*)k_res_plain<4> : (const void*)k_res_plain<6>;
-        e = launch(fn, args);
+        e = launch(nl == 4 ? (far ? (const void*)k_res_plain<4, true> : (const void*)k_res_plain<4, false>)
+                           : (far ? (const void*)k_res_plain<6, true> : (const void*)k_res_plain<6, false>), args);
     }
     if (e != cudaSuccess) {
         cudaGetLastError();

@@ -39,7 +39,8 @@
 // the operator's intermediates (a vector of its own for each step) are rewritten
 // once per reduction RQ / AMU, the word of p and e likewise, and each of the three reductions has its own totals.
 // The vectors no other block reads (q, r / v, p, e, r0, x) live in shared memory, in 48
-// (FP64) or 24 bytes per row, which leaves L2 to the matrix and the words.
+// (FP64) or 24 bytes per row, which leaves L2 to the matrix and the words (r0 in global
+// memory where they would take the L1 cache's share).
 // Every poll is bounded: a warp that runs out raises the abort flag, polls of
 // the other warps and blocks then give up too, and the block leaves at the next
 // reduction; the host reports the failure.
@@ -56,7 +57,7 @@ constexpr int kResThreads = 32 * kResWarps + 32; // and the scalar warp
 constexpr int kResRegs = 65536 / kResThreads & ~7;  // 64 registers per thread, at any launch size
 constexpr int kResReds = 5;                      // RQ, AMU, RN, and two of the mixed path's refinement: a
                                                  // reduction's words are written again only after another one
-constexpr int kResVecs = 6;                      // vectors a block keeps in shared memory
+constexpr int kResVecs = 6;                      // vectors a block keeps in shared memory, five with FAR
 constexpr int kResSteps = 3;                     // vectors between the operator's steps (NL / 2 of them used)
 
 // Coefficients and indices of one 32-row group in the resident loop's layout:
@@ -416,8 +417,9 @@ struct ResRow {
     bool ok;
 };
 
-// One block's part of a member's solve.
-template <typename T, int NL>
+// One block's part of a member's solve.  FAR: r0, read twice an iteration, stays in
+// global memory (kResL1Smem).
+template <typename T, int NL, bool FAR>
 struct Resident {
     static constexpr int NI = kResIdx<NL>, NC = NI + 1;
     static constexpr bool kWide = sizeof(T) == 4;     // FP64 rows take twice the registers
@@ -450,8 +452,8 @@ struct Resident {
         rv = q + rows_b;
         p = rv + rows_b;
         e = p + rows_b;
-        r0 = e + rows_b;
-        x = r0 + rows_b;
+        r0 = FAR ? E.r0 + off + (long)c0 * kChunk : e + rows_b;
+        x = e + (FAR ? 1 : 2) * rows_b;
         nq = w == ws ? 0 : 4 * (c1 - c0);                   // the scalar warp has no rows
         row0 = (unsigned)(off + (long)c0 * kChunk) + lane;
         part = R.part + 2 * (off / kChunk);
@@ -759,13 +761,13 @@ struct Resident {
 
 // A whole FP64 solve after the setup kernels: b^ = PM W b and BN, r = b^ - PM A x0
 // and C1 (pcgpme_para.F90:113-145), the iterations, x to the caller.
-template <int NL>
+template <int NL, bool FAR>
 __global__ void __launch_bounds__(kResThreads, 1) k_res_plain(const Eng<double> E, const ResBufs<double> R, long limit,
                                                              int absent) {
     if ((int)blockIdx.x == absent) return;
     __shared__ ResShared sh;
     extern __shared__ double vecs[];
-    const Resident<double, NL> S(E, R, sh, vecs, limit);
+    const Resident<double, NL, FAR> S(E, R, sh, vecs, limit);
     S.rows([&](const ResRow& rw) {
         if (!rw.ok) return;
         const double x0 = E.xi[rw.i];
@@ -804,13 +806,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res_plain(const Eng<double> 
 // A whole mixed-precision solve after the setup kernels: ||PM W b|| on FP64 vectors,
 // then refinement sweeps (as k_mx_residual, k_mx_sweep56, k_mx_normalize, k_mx_update)
 // around the FP32 iterations until the member's outer stop test.
-template <int NL>
+template <int NL, bool FAR>
 __global__ void __launch_bounds__(kResThreads, 1) k_res_mixed(const Eng<float> E, const ResBufs<float> R,
                                                              double inner_tol, int inner_max, long limit, int absent) {
     if ((int)blockIdx.x == absent) return;
     __shared__ ResShared sh;
     extern __shared__ double vecs[];
-    const Resident<float, NL> S(E, R, sh, vecs, limit);
+    const Resident<float, NL, FAR> S(E, R, sh, vecs, limit);
     const MemberIn in = E.in[S.bb.m];
     double* y64 = vecs;                                     // FP64 operands lie over q and rv, dead between the sweeps
     S.rows([&](const ResRow& rw) {

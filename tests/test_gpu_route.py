@@ -111,3 +111,11 @@ def test_refused_launch_of_the_2dh_solve(gpu, monkeypatch):
         info = gpu.WillSolver(5000).solve(al, ll, d, rhs, eps=1e-10)
         got.append((info.as_dict(), rhs))
     assert got[0][0] == got[1][0] and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("chunks,resident", [(70, True), (71, False)])
+def test_uneven_ensembles_stay_below_a_blocks_limit(gpu, monkeypatch, chunks, resident):
+    """69 members of ten rows take a block each, so the 83 others share one large member:
+    past 70 chunks a block the graph is the faster."""
+    monkeypatch.delenv("CLOWNS_LOOP_MODE", raising=False)
+    _check(gpu, [83 * 128 * chunks - 1] + [10] * 69, 1, resident)
