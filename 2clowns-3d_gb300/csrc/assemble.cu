@@ -64,8 +64,12 @@ __device__ __forceinline__ double cal_alu(double fnn, double dx, double dxm) {
 // products with its area and porosity where these are not 1; the six quotients by one
 // porosity take its reciprocal (Markstein): 176 us, half of it FP64 and the rest the
 // dependent loads of six neighbours.
-// TAB = false: grids whose table exceeds shared memory form every factor.
+// TAB = false: grids whose table exceeds shared memory form every factor, in small blocks:
+// there is no table to share, and long grids of few cells (1024 / 128 threads: 45 / 29 us
+// at 1500 x 1 x 45 cells, 74 / 50 at 2000 x 1 x 80, 634 / 579 at 1600 x 40 x 30) leave SMs idle
+// otherwise.
 constexpr int kInitBlock = 1024;
+constexpr int kInitPlainBlock = 128;
 template <int NL, bool TAB>
 __global__ void __launch_bounds__(kInitBlock, 1) k_init_matrix(GridIdx g, int inne, int mx2, const int* __restrict__ mn,
                                                           const int* __restrict__ in_, const int* __restrict__ jn,
@@ -472,8 +476,9 @@ extern "C" int clowns_init_matrix_dev(const int* dims, int inne, int mx2, const 
     const int entries = (g.ie - g.is + 3) + (g.je - g.js + 3) + (g.ke - g.ks + 3);
     const size_t tab = sizeof(double) * 4 * (size_t)entries;
     auto launch = [&](auto kern, size_t smem) {
-        const int blocks = (int)std::min<long>((inne + kInitBlock - 1L) / kInitBlock, smem ? 152L : 152L * 16);
-        kern<<<blocks, kInitBlock, smem, s>>>(g, inne, mx2, mn, in_, jn, kn, nf, nfb, a, fb, dx, mp, alu_c, ll_c, de_c);
+        const int block = smem ? kInitBlock : kInitPlainBlock;
+        const int blocks = (int)std::min<long>((inne + block - 1L) / block, smem ? 152L : 152L * 16);
+        kern<<<blocks, block, smem, s>>>(g, inne, mx2, mn, in_, jn, kn, nf, nfb, a, fb, dx, mp, alu_c, ll_c, de_c);
     };
     // the table fits the shared memory every launch may have up to 1536 cells in i + j + k
     if (tab <= 48 * 1024) {
