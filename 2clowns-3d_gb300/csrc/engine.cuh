@@ -1697,9 +1697,10 @@ __global__ void __launch_bounds__(kEngBlock, kBalMinBlocks<T, R>) k_bal_eupdate(
 // do.  Here they stream x, p and q meanwhile, from the last chunk back, whose e is the
 // likeliest to be in L2 still; that costs 16 B more per row and saves 8 in the p update.
 // us per iteration before / now: FP64 125.2 / 119.0 at 826 k rows, 156.5 / 153.0 at 1.15 M,
-// 302.8 / 301.0 at 2.8 M (bound by HBM and the FP64 pipe); mixed 104.3 / 101.6 and 197.5 /
-// 192.1 (in another process, other buffers, 195.8 / 194.8).  (Only x in the second part: 121.4, 154.8, 303.5; mixed 104.3, 195.6.  Second
-// part upwards: 302.7 at 2.8 M.)
+// 302.8 / 301.0 at 2.8 M (bound by HBM and the FP64 pipe); mixed 104.3 / 101.6 at 1.15 M and
+// 195.8 / 194.8 at 2.8 M (197.5 / 192.1 in another process; whole solves there differ by
+// 0.2-0.8 %, no more than two runs of one build).  (Only x in the second part: 121.4,
+// 154.8, 303.5; mixed 104.3, 195.6.  Second part upwards: 302.7 at 2.8 M.)
 template <typename T, int R>
 __global__ void __launch_bounds__(kEngBlock, kBalMinBlocks<T, R>) k_bal_xrupdate(Eng<T> E, const BalBlock* __restrict__ tab) {
     pdl_trigger();

@@ -1,8 +1,8 @@
 // resident.cuh -- solves of small and medium systems and ensembles as ONE resident
 // kernel whose blocks exchange vectors through self-validating words.
 //
-// Below about half a million rows an iteration of the kernel-per-phase loop is
-// bound by its kernel boundaries, not by its work: 12 kernels of about 4 us each
+// Below some 0.7 M rows (FP64; 1.1 M in mixed precision) an iteration of the
+// kernel-per-phase loop is bound by its kernel boundaries, not by its work: 12 kernels of about 4 us each
 // at 4 k rows (0.3 us of FP64 arithmetic) and still 5-7 us each at 0.4 M rows.
 // Here one cooperative launch (at most one block per SM, member rows dealt to
 // the blocks in 128-row chunks) runs every iteration, and nothing in it is a
@@ -21,13 +21,16 @@
 //     pair's second sweep needs from coefficients composed once per solve
 //     (k_res_compose), with the same fused multiply-adds, so the bits are those of
 //     separate sweeps.  That costs 4 more operations per row and iteration and
-//     saves four trips.  (us per iteration with pairs / threes, 1-2-3 | 4-5-6, 12
-//     more operations and one trip less each way / single sweeps: FP64 16.6 / 16.7 /
-//     18.5 at 27 k rows, 39.8 / 43.5 / 40.7 at 239 k, 67.0 / 72.6 / 70.4 at 413 k.)
-// What bounds it: a trip takes 0.3-0.5 us; a warp's FP64 operation holds its SM
+//     saves four trips.  (us per iteration of the kernel's first form with pairs /
+//     threes, 1-2-3 | 4-5-6, 12 more operations and one trip less each way / single
+//     sweeps: FP64 16.6 / 16.7 / 18.5 at 27 k rows, 39.8 / 43.5 / 40.7 at 239 k, 67.0 /
+//     72.6 / 70.4 at 413 k; the present form takes 16.6, 32 and 49 with pairs.)
+// What bounds it: a trip takes 0.25 us inside a die and 0.45 us across (two words sent to
+// and fro: 515-550 and 910-920 clocks each way); a warp's FP64 operation holds its SM
 // sub-partition for 64 cycles whatever its active lanes (76 with all four busy),
 // so small systems are bound by the chain of dependent FP64 operations and large
-// ones by their number.  Hence: rows are dealt out in groups of 32, one row per
+// ones by their number and that chain (FP64 pipe 60 % busy at 413 k rows; L2, asked for
+// 1.1 KB per row and iteration, is at 31 % of its peak throughput).  Hence: rows are dealt out in groups of 32, one row per
 // lane, so that a chunk's four groups use four sub-partitions; the two totals of
 // a dot-product pair are folded by different warps; an extra warp per block
 // finalises the scalars, and takes the square root and the stop tests of an
@@ -37,7 +40,8 @@
 // A word is overwritten only after a reduction of the same iteration that every
 // reader's own contribution had to precede, so no reader can miss its epoch:
 // the operator's intermediates (a vector of its own for each step) are rewritten
-// once per reduction RQ / AMU, the word of p and e likewise, and each of the three reductions has its own totals.
+// once per reduction RQ / AMU, the word of p and e likewise, and each of the three
+// reductions has its own totals and its own verdict.
 // The vectors no other block reads (q, r / v, p, e, r0, x) live in shared memory, in 48
 // (FP64) or 24 bytes per row, which leaves L2 to the matrix and the words (r0 in global
 // memory where they would take the L1 cache's share).
