@@ -456,8 +456,12 @@ struct Resident {
         rv = q + rows_b;
         p = rv + rows_b;
         e = p + rows_b;
-        r0 = FAR ? E.r0 + off + (long)c0 * kChunk : e + rows_b;
-        x = e + (FAR ? 1 : 2) * rows_b;
+        r0 = e + rows_b;
+        x = r0 + rows_b;
+        if constexpr (FAR) {
+            x = r0;
+            r0 = E.r0 + off + (long)c0 * kChunk;
+        }
         nq = w == ws ? 0 : 4 * (c1 - c0);                   // the scalar warp has no rows
         row0 = (unsigned)(off + (long)c0 * kChunk) + lane;
         part = R.part + 2 * (off / kChunk);
