@@ -236,9 +236,9 @@ static inline int member_groups(int n) {
 // 23.2 / 19.1 at 660 k; mixed 3.7 / 1.1, 5.8 / 1.9, 9.1 / 3.8, 10.9 / 5.8, 17.0 / 10.7, 19.6 / 15.3 at 960 k,
 // 20.6 / 18.6 at 1.09 M, 21.2 / 22.6 at 1.15 M (words and matrix no longer fit L2).
 // Ensembles, us per iteration, graph / resident (rows of a uniform grid; in brackets with
-// coefficients drawn for each row by itself, whose gathers scatter most): FP64 119 / 46 at 76
-// members of 389 k rows, 116 / 59 at one of 408 k beside 69 of 10 rows, 123 / 91 (130 / 109) at
-// 12 of 664 k; mixed 107 / 55 at 76 of 817 k, 133 / 100 (142 / 120) at 76 of 1.245 M, 145 /
+// coefficients drawn for each row by itself, whose gathers scatter most): FP64 99 / 46 at 76
+// members of 389 k rows, 105 / 80 (108 / 97) at one of 383 k beside 69 of 10 rows, 123 / 91
+// (131 / 109) at 12 of 664 k; mixed 107 / 55 at 76 of 817 k, 133 / 100 (142 / 120) at 76 of 1.245 M, 145 /
 // 109 (149 / 143) at 2 of 1.245 M.
 constexpr int kResMaxRowsFp64 = 700000;
 constexpr int kResMaxRowsMixed = 1100000;
@@ -252,9 +252,10 @@ constexpr int kResMaxBlocks = kNumSMs;
 // 70 (ten rounds of the 28 warps), 131 / 141 at 74 (40 members).
 static int res_max_chunks(int mixed) { return mixed ? 70 : 37; }
 // Shared memory of a block that leaves its L1 cache 60 KB for the matrix.  A block whose six
-// vectors take more (33 chunks in FP64, 65 in FP32) leaves r0 in global memory: with
-// all six there, past 192 KB, 28 KB of L1 were left, and the same rows took 153 us (153 /
-// 111 at 642 k rows, the graph 114; uneven grids of 690 k rows with porosities 119 / 99, the graph 113).
+// vectors take more (33 chunks in FP64, 65 in FP32) leaves r0 in global memory.  us per
+// iteration, all six in shared memory (28 KB of L1 left) / r0 outside / the graph: 153 / 111 /
+// 114 at 642 k rows with coefficients drawn per row, 119 / 99 / 113 on an uneven grid of 690 k
+// rows with porosities, 86.3 / 89.5 / 109 on a uniform one of 642 k.
 constexpr size_t kResL1Smem = 192 * 1024;
 
 // Blocks of each member in the resident solve: at most one per SM, dealt in proportion
