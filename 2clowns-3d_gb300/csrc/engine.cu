@@ -1050,7 +1050,8 @@ static long loop_launches(const LoopShape& sh, long bodies) {
 
 // Test hook of the bounded device waits (clowns_test_arm_wait_timeout): the
 // next resident solve, or plain FP64 solve whose loop runs as one cooperative
-// kernel, gives every wait `limit` polls and makes block `absent` leave without arriving.  One use.
+// kernel, gives every wait `limit` polls and makes block `absent` leave without
+// arriving.  One use.
 struct WaitFault {
     long limit = kBarSpinLimit;
     int absent = -1;
@@ -1353,7 +1354,8 @@ int engine_tuned_shape(int M, const int* n, int mixed, int* mode, int* block, in
     std::vector<int> g;
     int per = 0;
     std::lock_guard<std::mutex> lk(g_loop_mu);
-    const bool resident = res_serves(M, n, mixed) && res_deal(M, n, mixed, g, per) && g_resident.count(std::make_tuple(nv, M, mixed, forced_loop_mode()));
+    const bool resident = g_resident.count(std::make_tuple(nv, M, mixed, forced_loop_mode())) &&
+                          res_serves(M, n, mixed) && res_deal(M, n, mixed, g, per);
     auto it = g_loop_shapes.find(std::make_tuple(nv, mixed, (int)(M == 1), forced_loop_mode()));
     if (!resident && it == g_loop_shapes.end()) return CLOWNS_ERR_ARG;
     const LoopShape sh = resident ? res_shape(M, g, per, nullptr) : it->second;
